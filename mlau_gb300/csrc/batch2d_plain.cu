@@ -55,22 +55,22 @@ __device__ void pp_prep(const BArgs &A, int nt, const BTile *tl, int rk)
             wx = wy = I.base + sy * bwrap(j, I.ny, I.off) + bwrap(i, I.nx, I.off);
         }
         const double *bx = a.s[5], *by = a.s[6];
-        const double cx = gx * face2cen(A.odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
-        const double cy = gy * face2cen(A.odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
-        const double ro = a.s[0][c];
-        const double iro = 1.0 / ro;
-        const double vx = a.s[1][c] * iro, vy = a.s[2][c] * iro, vz = a.s[3][c] * iro;
-        const double bz = a.s[7][c];
-        const double v2 = (vx * vx + vy * vy + vz * vz);
-        const double b2 = (cx * cx + cy * cy + bz * bz);
-        const double pr = (I.gamma - 1) * (a.s[4][c] - 0.5 * (ro * v2 + b2));
-        a.vx[c] = vx;
-        a.vy[c] = vy;
-        a.vz[c] = vz;
-        a.pr[c] = pr;
-        a.m2[c] = v2 / (I.gamma * pr * iro);
-        a.cx[c] = cx;
-        a.cy[c] = cy;
+        const ed cx = ed(gx) * face2cen<ed>(A.odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
+        const ed cy = ed(gy) * face2cen<ed>(A.odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
+        const ed ro = a.s[0][c];
+        const ed iro = trcp(ro);
+        const ed vx = a.s[1][c] * iro, vy = a.s[2][c] * iro, vz = a.s[3][c] * iro;
+        const ed bz = a.s[7][c];
+        const ed v2 = (vx * vx + vy * vy + vz * vz);
+        const ed b2 = (cx * cx + cy * cy + bz * bz);
+        const ed pr = ed(I.gamma - 1) * (a.s[4][c] - ed(0.5) * (ro * v2 + b2));
+        a.vx[c] = vx.v;
+        a.vy[c] = vy.v;
+        a.vz[c] = vz.v;
+        a.pr[c] = pr.v;
+        a.m2[c] = (v2 / (I.gamma * pr * iro)).v;
+        a.cx[c] = cx.v;
+        a.cy[c] = cy.v;
         if (rk == 0)
             for (int v = 0; v < 8; v++) a.u0[v][c] = a.s[v][c];
     });
@@ -111,7 +111,7 @@ __device__ void pp_rec(const BArgs &A, int nt, const BTile *tl, int D)
         const double *cn = D == 0 ? a.cx : a.cy, *ct = D == 0 ? a.cy : a.s[7],
                      *cu = D == 0 ? a.s[7] : a.cx;
         const double *bface = D == 0 ? a.s[5] : a.s[6];
-        double q[7][5];
+        ed q[7][5];
 #pragma unroll
         for (int m = 0; m < 5; m++) {
             const long long s = c + st * (m - 2);
@@ -123,28 +123,28 @@ __device__ void pp_rec(const BArgs &A, int nt, const BTile *tl, int D)
             q[5][m] = cu[s];
             q[6][m] = a.pr[s];
         }
-        double ul[7], ur[7];
+        ed ul[7], ur[7];
         if (vmax(a.m2[c - st], vmax(a.m2[c], a.m2[c + st])) >= 1.0)
-            reconst_full(A.odr, q, cn[c], I.gamma, ul, ur);
+            reconst_full<ed>(A.odr, q, cn[c], I.gamma, ul, ur);
         else
-            reconst_alfven(A.odr, q, cn[c], I.gamma, ul, ur);
+            reconst_alfven<ed>(A.odr, q, cn[c], I.gamma, ul, ur);
 #pragma unroll
         for (int n = 0; n < 7; n++) {
-            a.ul[n][c + st] = ul[n];
-            a.ur[n][c] = ur[n];
+            a.ul[n][c + st] = ul[n].v;
+            a.ur[n][c] = ur[n].v;
         }
         const double *bt = D == 1 ? cu : ct, *vv = D == 1 ? vu : vt;
-        double a5[5], t5[5];
+        ed a5[5], t5[5];
 #pragma unroll
         for (int m = 0; m < 5; m++) {
             const long long s = c + st * (m - 2);
-            a5[m] = bt[s] * vn[s];
+            a5[m] = ed(bt[s]) * vn[s];
             t5[m] = vv[s];
         }
-        a.ul[7][c + st] = lin_l(A.odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                          - bface[c + st] * lin_l(A.odr, t5[0], t5[1], t5[2], t5[3], t5[4]);
-        a.ur[7][c] = lin_r(A.odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                     - bface[c] * lin_r(A.odr, t5[0], t5[1], t5[2], t5[3], t5[4]);
+        a.ul[7][c + st] = (lin_l(A.odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                          - ed(bface[c + st]) * lin_l(A.odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+        a.ur[7][c] = (lin_r(A.odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                     - ed(bface[c]) * lin_r(A.odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
     });
 }
 
@@ -157,19 +157,20 @@ __device__ void pp_flux(const BArgs &A, int nt, const BTile *tl, int D)
         const long long st = D == 0 ? 1 : I.nx;
         const double *vn = D == 0 ? a.vx : a.vy, *dvt = D == 0 ? a.dv[1] : a.dv[0];
         const double *bface = D == 0 ? a.s[5] : a.s[6];
-        double L[7], R[7], F[7];
+        ed L[7], R[7], F[7];
 #pragma unroll
         for (int n = 0; n < 7; n++) {
             L[n] = a.ul[n][c];
             R[n] = a.ur[n][c];
         }
-        const double bn = 0.5 * (bface[c] + bface[c]);
-        riemann(I.flux, L, R, bn, I.gamma, (vn[c] - vn[c - st]), vmin(dvt[c - st], dvt[c]), F);
-        const double fc = 0.5 * (a.ul[7][c] + a.ur[7][c]);
+        const ed bn = ed(0.5) * (ed(bface[c]) + bface[c]);
+        riemann<ed>(I.flux, L, R, bn, I.gamma, (ed(vn[c]) - vn[c - st]),
+                    vmin(dvt[c - st], dvt[c]), F);
+        const ed fc = ed(0.5) * (ed(a.ul[7][c]) + a.ur[7][c]);
         F[4 + D] -= fc;
 #pragma unroll
-        for (int n = 0; n < 7; n++) a.F[D][n][c] = F[n];
-        a.FC[D][c] = fc;
+        for (int n = 0; n < 7; n++) a.F[D][n][c] = F[n].v;
+        a.FC[D][c] = fc.v;
     });
 }
 
@@ -177,13 +178,13 @@ __device__ void pp_emf(const BArgs &A, int nt, const BTile *tl)
 {
     const BArrays &a = A.a;
     for_cells(A, nt, tl, [&](const BInst &I, int i, int j, long long c) {
-        double ez = 0.0;
+        ed ez = 0.0;
         if (i >= 3 && i < I.nx - 2 && j >= 3 && j < I.ny - 2) {
-            const double w = a.ct[c];
-            ez = (0.0 + emf_part(a.F[0][4], a.FC[0], (1.0 - w), -1.0, c, I.nx, A.odr))
+            const ed w = a.ct[c];
+            ez = (ed(0.0) + emf_part(a.F[0][4], a.FC[0], (ed(1.0) - w), -1.0, c, I.nx, A.odr))
                  + emf_part(a.F[1][5], a.FC[1], w, +1.0, c, 1, A.odr);
         }
-        a.ez[c] = ez;
+        a.ez[c] = ez.v;
     });
 }
 
@@ -193,29 +194,29 @@ __device__ void pp_update(const BArgs &A, int nt, const BTile *tl, int rk)
     // rk_fac of the reference for R_K=3 (mhd_fd_ct_2d.c:110)
     const double rkf[3][2] = {{0.0, 1.0}, {0.5 + (3 - 2) * 0.25, 0.5 - (3 - 2) * 0.25},
                               {1. / 3., 2. / 3.}};
-    const double ra = rkf[rk][0], rb = rkf[rk][1];
+    const ed ra = rkf[rk][0], rb = rkf[rk][1];
     for_cells(A, nt, tl, [&](const BInst &I, int i, int j, long long c) {
         if (i < I.off || i >= I.nx - I.off || j < I.off || j >= I.ny - I.off) return;
         const long long sy = I.nx;
-        const double dtdx = I.dt / I.dx, dtdy = I.dt / I.dy;
+        const ed dtdx = ed(I.dt) / I.dx, dtdy = ed(I.dt) / I.dy;
         const int sv[6] = {0, 1, 2, 3, 7, 4};
         const int cX[6] = {0, 1, 2, 3, 5, 6}, cY[6] = {0, 3, 1, 2, 4, 6};
         double out[8];
 #pragma unroll
         for (int v = 0; v < 6; v++) {
             const double *fx = a.F[0][cX[v]], *fy = a.F[1][cY[v]];
-            const double d0 = fdiff(A.odr, fx[c - 1], fx[c], fx[c + 1], fx[c + 2]);
-            const double d1 = fdiff(A.odr, fy[c - sy], fy[c], fy[c + sy], fy[c + 2 * sy]);
-            out[sv[v]] = ra * a.u0[sv[v]][c] + rb * (a.s[sv[v]][c] - dtdx * d0 - dtdy * d1);
+            const ed d0 = fdiff<ed>(A.odr, fx[c - 1], fx[c], fx[c + 1], fx[c + 2]);
+            const ed d1 = fdiff<ed>(A.odr, fy[c - sy], fy[c], fy[c + sy], fy[c + 2 * sy]);
+            out[sv[v]] = (ra * a.u0[sv[v]][c] + rb * (ed(a.s[sv[v]][c]) - dtdx * d0 - dtdy * d1)).v;
         }
         const double *ez = a.ez;
         {
-            const double dd = fdiff(A.odr, ez[c - sy], ez[c], ez[c + sy], ez[c + 2 * sy]);
-            out[5] = ra * a.u0[5][c] + rb * (a.s[5][c] - dtdy * dd);
+            const ed dd = fdiff<ed>(A.odr, ez[c - sy], ez[c], ez[c + sy], ez[c + 2 * sy]);
+            out[5] = (ra * a.u0[5][c] + rb * (ed(a.s[5][c]) - dtdy * dd)).v;
         }
         {
-            const double dd = fdiff(A.odr, ez[c - 1], ez[c], ez[c + 1], ez[c + 2]);
-            out[6] = ra * a.u0[6][c] + rb * (a.s[6][c] + dtdx * dd);
+            const ed dd = fdiff<ed>(A.odr, ez[c - 1], ez[c], ez[c + 1], ez[c + 2]);
+            out[6] = (ra * a.u0[6][c] + rb * (ed(a.s[6][c]) + dtdx * dd)).v;
         }
         if (I.walls) {  // the boundary phases fill the ghosts
 #pragma unroll
@@ -245,18 +246,18 @@ __device__ void pp_face(const BArgs &A, int nt, const BTile *tl, int rk)
     const BArrays &a = A.a;
     const double rkf[3][2] = {{0.0, 1.0}, {0.5 + (3 - 2) * 0.25, 0.5 - (3 - 2) * 0.25},
                               {1. / 3., 2. / 3.}};
-    const double ra = rkf[rk][0], rb = rkf[rk][1];
+    const ed ra = rkf[rk][0], rb = rkf[rk][1];
     for_cells(A, nt, tl, [&](const BInst &I, int i, int j, long long c) {
         if (!I.walls) return;
         const long long sy = I.nx;
         const double *ez = a.ez;
         if (I.bcx[5] != 0 && i == I.nx - I.off && j >= I.off && j < I.ny - I.off) {
-            const double dd = fdiff(A.odr, ez[c - sy], ez[c], ez[c + sy], ez[c + 2 * sy]);
-            a.s[5][c] = ra * a.u0[5][c] + rb * (a.s[5][c] - (I.dt / I.dy) * dd);
+            const ed dd = fdiff<ed>(A.odr, ez[c - sy], ez[c], ez[c + sy], ez[c + 2 * sy]);
+            a.s[5][c] = (ra * a.u0[5][c] + rb * (ed(a.s[5][c]) - (ed(I.dt) / I.dy) * dd)).v;
         }
         if (I.bcy[6] != 0 && j == I.ny - I.off && i >= I.off && i < I.nx - I.off) {
-            const double dd = fdiff(A.odr, ez[c - 1], ez[c], ez[c + 1], ez[c + 2]);
-            a.s[6][c] = ra * a.u0[6][c] + rb * (a.s[6][c] + (I.dt / I.dx) * dd);
+            const ed dd = fdiff<ed>(A.odr, ez[c - 1], ez[c], ez[c + 1], ez[c + 2]);
+            a.s[6][c] = (ra * a.u0[6][c] + rb * (ed(a.s[6][c]) + (ed(I.dt) / I.dx) * dd)).v;
         }
     });
 }

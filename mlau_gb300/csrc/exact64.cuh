@@ -1,0 +1,296 @@
+// Reciprocal, division and square root of doubles, correctly rounded (round to
+// nearest even), computed on the integer and FP32 pipes.
+//
+// Why: this part's FP64 pipe takes 64 cycles per warp instruction in each SM
+// sub-partition (2 lanes per cycle per SM), and CUDA's own FP64 division,
+// reciprocal and square root run on it: measured 577 / 362 / 602 cycles per
+// warp, while the integer and FP32 pipes beside it are idle.  The functions
+// here take 132 / 79 / 121 cycles of issue slots (latency 257 / 203 / 237
+// against 607 / 388 / 645), leave the FP64 pipe to the additions and products,
+// and return the same bits, so the plain FP64 kernels keep the reference's
+// values.
+//
+// Method: significands as 53-bit integers.  An FP32 reciprocal (square root)
+// seed, one Newton step whose residual is formed exactly modulo 2^64, and a
+// correction from the next exact residual give the quotient to well below a
+// unit; the correctly rounded result follows unless that lies within the
+// correction's error of a midpoint between two doubles (about one operand in
+// 2^15), where the pipe's own operation decides.  Division instead makes two
+// quotient digits (32 and 29 bits) and settles the last unit by its exact
+// remainder.  Operands whose magnitude is outside 2^-255 .. 2^256, zeros,
+// infinities and NaN also take the pipe's operation.  The seeds may be off by
+// 2 units in the last place (CUDA states at most 1 for rcp.approx, 2^-22.9 for
+// rsqrt.approx); tests/test_exact64.py tries them perturbed.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#include <cuda_runtime.h>
+#define X64 __host__ __device__ __forceinline__
+// the rarely run pipe operations stay out of line
+#define X64_SLOW __host__ __device__ __noinline__
+#else
+#define X64 inline
+#define X64_SLOW inline
+#endif
+
+namespace mlau {
+namespace x64 {
+
+X64 uint32_t hi32(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__double2hiint(x);
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return (uint32_t)(u >> 32);
+#endif
+}
+X64 uint32_t lo32(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__double2loint(x);
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return (uint32_t)u;
+#endif
+}
+X64 double make(uint32_t h, uint32_t l)
+{
+#ifdef __CUDA_ARCH__
+    return __hiloint2double((int)h, (int)l);
+#else
+    const uint64_t u = ((uint64_t)h << 32) | l;
+    double x;
+    memcpy(&x, &u, 8);
+    return x;
+#endif
+}
+X64 float as_f(uint32_t u)
+{
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float f;
+    memcpy(&f, &u, 4);
+    return f;
+#endif
+}
+X64 uint32_t as_u(float f)
+{
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(f);
+#else
+    uint32_t u;
+    memcpy(&u, &f, 4);
+    return u;
+#endif
+}
+// (hi:lo) << s, upper word; s in [0, 31]
+X64 uint32_t shfl_(uint32_t lo, uint32_t hi, int s)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, s);
+#else
+    return s ? (hi << s) | (lo >> (32 - s)) : hi;
+#endif
+}
+// (hi:lo) >> s, lower word; s in [0, 31]
+X64 uint32_t shfr_(uint32_t lo, uint32_t hi, int s)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, s);
+#else
+    return s ? (lo >> s) | (hi << (32 - s)) : lo;
+#endif
+}
+X64 uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+// The host's seeds are exact to half a unit; MLAU_X64_SEED_ULPS (a function
+// call in a test) moves them.
+#ifndef MLAU_X64_SEED_ULPS
+#define MLAU_X64_SEED_ULPS 0
+#endif
+X64 float seed_rcp(float x)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return as_f(as_u((float)(1.0 / (double)x)) + MLAU_X64_SEED_ULPS);
+#endif
+}
+X64 float seed_rsqrt(float x)
+{
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return as_f(as_u((float)(1.0 / std::sqrt((double)x))) + MLAU_X64_SEED_ULPS);
+#endif
+}
+
+// Zero exactly for exponent fields 768..1279 (magnitudes 2^-255 to 2^256, any
+// sign): the integer path's operands, whose products and quotients are normal.
+X64 uint32_t off_range(uint32_t h) { return (h + 0x50000000u) & 0x60000000u; }
+X64 uint32_t off_range(uint32_t h, uint32_t g)
+{
+    return ((h + 0x50000000u) | (g + 0x50000000u)) & 0x60000000u;
+}
+
+// Reciprocal seed of the 53-bit significand (mh:ml) in [2^52, 2^53): Y0 in
+// [2^23, 2^24) with Y0 ~ 2^76 / B, and e1 = (B Y0 - 2^76) >> 24.
+X64 void rcp_seed(uint32_t mh, uint32_t ml, uint32_t &Y0, int32_t &e1)
+{
+    const float x = as_f(0x3f800000u | (shfl_(ml, mh, 3) & 0x7fffffu));
+    // y in (0.49, 1.01): its distance to 1 - 2^-22, added to a power of two's
+    // significand, reads as an integer without a test of y's own exponent
+    const float y = seed_rcp(x) + (1.0f - 0x1p-22f);
+    Y0 = 2u * as_u(y) - (2u * 0x3f800000u - 4u);
+    const uint64_t p = wide(ml, Y0);
+    const uint32_t eh = mh * Y0 + (uint32_t)(p >> 32);
+    e1 = (int32_t)shfr_((uint32_t)p, eh, 24);
+}
+
+// The FP64 pipe's own results, for the few lanes the integer path leaves.
+static X64_SLOW double rcp_hw(double x) { return 1.0 / x; }
+static X64_SLOW double div_hw(double a, double b) { return a / b; }
+static X64_SLOW double sqrt_hw(double x) { return ::sqrt(x); }
+
+X64 double rcp(double x)
+{
+    const uint32_t ah = hi32(x), ml = lo32(x);
+    const uint32_t mh = (ah & 0xfffffu) | 0x100000u;
+    uint32_t Y0;
+    int32_t e1;
+    rcp_seed(mh, ml, Y0, e1);
+    // Q1 ~ 2^105 / B to 2^-44: Y0 2^29 - (Y0 e1 >> 23)
+    const uint64_t Q1 = ((uint64_t)Y0 << 29) - (uint64_t)(((int64_t)(int32_t)Y0 * e1) >> 23);
+    const uint32_t qh = (uint32_t)(Q1 >> 32), ql = (uint32_t)Q1;
+    // R = 2^105 - B Q1 (|R| < 2^61, exact modulo 2^64); r ~ R / 2^32
+    const uint64_t p = wide(ml, ql);
+    const uint32_t rh = (uint32_t)(p >> 32) + ml * qh + mh * ql;
+    const int32_t r = (int32_t)~rh;
+    // correction R Q1 / 2^105, 18 fraction bits
+    const int32_t P = (int32_t)(((int64_t)r * (int32_t)shfr_(ql, qh, 23)) >> 32);
+    const int32_t T = P + (1 << 17);
+    const uint64_t Q = Q1 + (uint64_t)(int64_t)(T >> 18);
+    const bool ok = off_range(ah) == 0 && (((uint32_t)T + 4u) & 0x3ffffu) > 8u;
+    const uint32_t e = (2044u << 20) - (ah & 0x7ff00000u) + (ah & 0x80000000u);
+    double q = make((uint32_t)(Q >> 32) + e, (uint32_t)Q);
+    if (!ok) q = rcp_hw(x);
+    return q;
+}
+
+// 0.5 / x
+X64 double half_over(double x)
+{
+    const double r = rcp(x);
+    // 1 / x a normal number above 2^-1021: the halving is exact
+    const uint32_t h = hi32(r), e = (h >> 20) & 0x7ffu;
+    return e - 2u < 2044u ? make(h - 0x100000u, lo32(r)) : div_hw(0.5, x);
+}
+
+// x / 24: the significand's quotient by 3 (no ties: the remainder is a third
+// of a unit or two), then the exponent.
+X64 double div24(double x)
+{
+    const uint32_t ah = hi32(x), al = lo32(x);
+    const uint32_t mh = (ah & 0xfffffu) | 0x100000u;
+    // N = B 2^s with N / 3 in [2^52, 2^53): s = 1 from 1.5 on, else 2
+    const uint32_t s = mh >= 0x180000u ? 1u : 2u;
+    const uint32_t nh = shfl_(al, mh, (int)s), nl = (al << s) + 1u;  // N + 1: round to nearest
+    const uint32_t qh = nh / 3u, ql = nl / 3u;
+    const uint32_t t = (nh - 3u * qh) + (nl - 3u * ql);
+    const uint64_t Q = (((uint64_t)qh << 32) | ql) + (uint64_t)(nh - 3u * qh) * 0x55555555u + (t >= 3u ? 1u : 0u);
+    // x / 24 = Q 2^-s 2^-3 in units of x's significand
+    const uint32_t e = (ah & 0xfff00000u) - ((4u + s) << 20);
+    double q = make((uint32_t)(Q >> 32) + e, (uint32_t)Q);
+    if (off_range(ah)) q = div_hw(x, 24.0);
+    return q;
+}
+
+X64 double div(double a, double b)
+{
+    const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), ml = lo32(b);
+    const uint32_t na = (ah & 0xfffffu) | 0x100000u, mh = (bh & 0xfffffu) | 0x100000u;
+    uint32_t Y0;
+    int32_t e1;
+    rcp_seed(mh, ml, Y0, e1);
+    // Y1 ~ 2^84 / B, 2 to 5 units low
+    const uint32_t Y1 = (Y0 << 8) - (uint32_t)(int32_t)(((int64_t)(int32_t)Y0 * e1) >> 44) - 3u;
+    // first digit, low: (A / B) 2^31 - d1 in (0, 12)
+    const uint32_t d1 = (uint32_t)(wide(shfl_(al, na, 11), Y1) >> 32) - 3u;
+    // R1 = A 2^31 - B d1
+    const uint64_t pb = wide(ml, d1);
+    const uint32_t ph = (uint32_t)(pb >> 32) + mh * d1;
+    const uint64_t R1 = (((uint64_t)shfr_(al, na, 1) << 32) | (al << 31)) -
+                        (((uint64_t)ph << 32) | (uint32_t)pb);
+    // second digit: (A / B) 2^31 = d1 + P / 2^58
+    const uint32_t r = shfr_((uint32_t)R1, (uint32_t)(R1 >> 32), 25);
+    const uint64_t P = wide(r, Y1 >> 1);
+    // quotient significand: (A / B) 2^52, or 2^53 where A < B
+    const bool lt = na < mh || (na == mh && al < ml);
+    const int sh = lt ? 22 : 21;
+    const uint32_t d2 = ((uint32_t)(P >> 32) + (1u << (25 - sh))) >> (26 - sh);
+    const uint64_t Q = ((uint64_t)d1 << sh) + d2;
+    // remainder A 2^(31+sh) - B Q = R1 2^sh - B d2, exact modulo 2^64
+    const uint64_t pd = wide(ml, d2);
+    const uint64_t R2 = (R1 << sh) - (((uint64_t)((uint32_t)(pd >> 32) + mh * d2) << 32) | (uint32_t)pd);
+    const int64_t B = (int64_t)(((uint64_t)mh << 32) | ml), t = 2 * (int64_t)R2;
+    const uint64_t Qr = Q + (t > B ? 1u : 0u) - (t < -B ? 1u : 0u);
+    const uint32_t e = (ah & 0x7ff00000u) - (bh & 0x7ff00000u) + ((lt ? 1021u : 1022u) << 20) +
+                       ((ah ^ bh) & 0x80000000u);
+    const bool ok = off_range(ah, bh) == 0;
+    double q = make((uint32_t)(Qr >> 32) + e, (uint32_t)Qr);
+    if (!ok) q = div_hw(a, b);
+    return q;
+}
+
+X64 double sqrt(double x)
+{
+    const uint32_t ah = hi32(x), al = lo32(x);
+    // x = X 2^(2k - 52), X = B or 2 B in [2^52, 2^54)
+    const uint32_t odd = (~ah >> 20) & 1u, o23 = odd << 23;
+    // xh + xl = X / 2^52 in [1, 4): the top 24 bits, the rest (23 bits of it)
+    const float xh = as_f((o23 + 0x3f800000u) | (shfl_(al, ah, 3) & 0x7fffffu));
+    const float xl = as_f((o23 + 0x34000000u) | ((al & 0x1fffffffu) >> 6)) - as_f(o23 + 0x34000000u);
+    float y = seed_rsqrt(xh);
+    y = fmaf(0.5f * y, fmaf(-xh * y, y, 1.0f), y);
+    const float s1 = fminf(fmaxf(xh * y, 1.0f), 0x1.fffffep0f);
+    // sqrt = s1 + c, |c| < 2^-21: C = c 2^52
+    const float r1 = fmaf(-s1, s1, xh) + xl;
+#ifdef __CUDA_ARCH__
+    const int32_t C = __float2int_rn(r1 * (y * 0x1p51f));
+#else
+    const int32_t C = (int32_t)std::lrintf(r1 * (y * 0x1p51f));
+#endif
+    const uint64_t S2 = ((uint64_t)((as_u(s1) & 0x7fffffu) | 0x800000u) << 29) + (uint64_t)(int64_t)C;
+    const uint32_t sh = (uint32_t)(S2 >> 32), sl = (uint32_t)S2;
+    // R = X 2^52 - S2^2 (|R| < 2^63, exact modulo 2^64); r = floor(R / 2^32)
+    const uint64_t p = wide(sl, sl);
+    const uint32_t ph = (uint32_t)(p >> 32) + 2u * sh * sl;
+    const int32_t r = (int32_t)((al << (20 + odd)) - ph - ((uint32_t)p != 0 ? 1u : 0u));
+    // correction R / (2 S2) = r Y / 2^52 with Y = y 2^31, 20 fraction bits
+    const uint32_t yb = as_u(y) < 0x3f7fffffu ? as_u(y) : 0x3f7fffffu;
+    const int32_t P = (int32_t)(((int64_t)r * (int32_t)(((yb & 0x7fffffu) | 0x800000u) << 7)) >> 32);
+    const int32_t T = P + (1 << 19);
+    const uint64_t S = S2 + (uint64_t)(int64_t)(T >> 20);
+    const uint32_t e = (((ah + 0x100000u) >> 1) & 0x7ff00000u) + (510u << 20);
+    // positive, mid-range and not near a midpoint
+    const bool ok = (ah + 0x50000000u) >> 29 == 4u && (((uint32_t)T + 64u) & 0xfffffu) > 128u;
+    double q = make((uint32_t)(S >> 32) + e, (uint32_t)S);
+    if (!ok) q = sqrt_hw(x);
+    return q;
+}
+
+}  // namespace x64
+
+}  // namespace mlau

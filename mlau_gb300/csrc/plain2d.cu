@@ -26,23 +26,23 @@ k_prim2(PlainFields f, Dims d, Box b, int odr, double gamma, Bc2 bc)
     const int iy = bc_src(i, d.nx, d.ox, 0, bc.x[6], &gy), jy = bc_src(j, d.ny, d.oy, 0, bc.y[6], &gy);
     const long long wx = d.at(ix, jx, 0), wy = d.at(iy, jy, 0);
     const double *bx = f.s[5], *by = f.s[6];
-    const double cx = gx * face2cen(odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
-    const double cy = gy * face2cen(odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
+    const ed cx = ed(gx) * face2cen<ed>(odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
+    const ed cy = ed(gy) * face2cen<ed>(odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
     const long long s = d.at(i, j, 0);
-    const double ro = f.s[0][s];
-    const double iro = 1.0 / ro;
-    const double vx = f.s[1][s] * iro, vy = f.s[2][s] * iro, vz = f.s[3][s] * iro;
-    const double bz = f.s[7][s];
-    const double v2 = (vx * vx + vy * vy + vz * vz);
-    const double b2 = (cx * cx + cy * cy + bz * bz);
-    const double pr = (gamma - 1) * (f.s[4][s] - 0.5 * (ro * v2 + b2));
-    f.vx[s] = vx;
-    f.vy[s] = vy;
-    f.vz[s] = vz;
-    f.pr[s] = pr;
-    f.m2[s] = v2 / (gamma * pr * iro);
-    f.cx[s] = cx;
-    f.cy[s] = cy;
+    const ed ro = f.s[0][s];
+    const ed iro = trcp(ro);
+    const ed vx = f.s[1][s] * iro, vy = f.s[2][s] * iro, vz = f.s[3][s] * iro;
+    const ed bz = f.s[7][s];
+    const ed v2 = (vx * vx + vy * vy + vz * vz);
+    const ed b2 = (cx * cx + cy * cy + bz * bz);
+    const ed pr = ed(gamma - 1) * (f.s[4][s] - ed(0.5) * (ro * v2 + b2));
+    f.vx[s] = vx.v;
+    f.vy[s] = vy.v;
+    f.vz[s] = vz.v;
+    f.pr[s] = pr.v;
+    f.m2[s] = (v2 / (gamma * pr * iro)).v;
+    f.cx[s] = cx.v;
+    f.cy[s] = cy.v;
 }
 
 // Shock sensors, with the sign rules of their ghost fill (:262-271): dvx
@@ -82,7 +82,7 @@ k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, do
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
-    double q[7][5];
+    ed q[7][5];
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
@@ -94,26 +94,26 @@ k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, do
         q[5][m] = v.cu[s];
         q[6][m] = f.pr[s];
     }
-    double ul[7], ur[7];
-    reconst_face(odr, eig, vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])), q, v.cn[c], gamma,
-                 ul, ur);
+    ed ul[7], ur[7];
+    reconst_face<ed>(odr, eig, vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])), q, v.cn[c], gamma,
+                     ul, ur);
 #pragma unroll
     for (int n = 0; n < 7; n++) {
-        f.ul[n][c + st] = ul[n];
-        f.ur[n][c] = ur[n];
+        f.ul[n][c + st] = ul[n].v;
+        f.ur[n][c] = ur[n].v;
     }
     const double *bt = v.split_u ? v.cu : v.ct, *vt = v.split_u ? v.vu : v.vt;
-    double a5[5], t5[5];
+    ed a5[5], t5[5];
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
-        a5[m] = bt[s] * v.vn[s];
+        a5[m] = ed(bt[s]) * v.vn[s];
         t5[m] = vt[s];
     }
-    f.ql[0][c + st] = lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - v.bface[c + st] * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4]);
-    f.qr[0][c] = lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - v.bface[c] * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4]);
+    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                      - ed(v.bface[c + st]) * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                 - ed(v.bface[c]) * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
 }
 
 __global__ void __launch_bounds__(TPB)
@@ -122,19 +122,20 @@ k_flux2(PlainFields f, View2 v, Dims d, Box b, long long st, int D, int which, d
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
-    double L[7], R[7], F[7];
+    ed L[7], R[7], F[7];
 #pragma unroll
     for (int n = 0; n < 7; n++) {
         L[n] = f.ul[n][c];
         R[n] = f.ur[n][c];
     }
-    const double bn = 0.5 * (v.bface[c] + v.bface[c]);
-    riemann(which, L, R, bn, gamma, (v.vn[c] - v.vn[c - st]), vmin(v.dvt[c - st], v.dvt[c]), F);
-    const double fc = 0.5 * (f.ql[0][c] + f.qr[0][c]);
+    const ed bn = ed(0.5) * (ed(v.bface[c]) + v.bface[c]);
+    riemann<ed>(which, L, R, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]),
+                vmin(v.dvt[c - st], v.dvt[c]), F);
+    const ed fc = ed(0.5) * (ed(f.ql[0][c]) + f.qr[0][c]);
     F[4 + v.split_u] -= fc;
 #pragma unroll
-    for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n];
-    f.FC[D][0][c] = fc;
+    for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n].v;
+    f.FC[D][0][c] = fc.v;
 }
 
 __global__ void __launch_bounds__(TPB) k_emf2(PlainFields f, Dims d, Box b, int odr)
@@ -142,21 +143,22 @@ __global__ void __launch_bounds__(TPB) k_emf2(PlainFields f, Dims d, Box b, int 
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
-    double ez = 0.0;
+    ed ez = 0.0;
     if (i >= 3 && i < d.nx - 2 && j >= 3 && j < d.ny - 2) {
-        const double w = f.ct[0][c];
-        ez = (0.0 + emf_part(f.F[0][4], f.FC[0][0], (1.0 - w), -1.0, c, d.nx, odr))
+        const ed w = f.ct[0][c];
+        ez = (ed(0.0) + emf_part(f.F[0][4], f.FC[0][0], (ed(1.0) - w), -1.0, c, d.nx, odr))
              + emf_part(f.F[1][5], f.FC[1][0], w, +1.0, c, 1, odr);
     }
-    f.e[2][c] = ez;
+    f.e[2][c] = ez.v;
 }
 
 // RK combine + CT curl of the interior.  With periodic tables each cell also
 // writes its periodic images; otherwise k_face2 and k_bc2 follow.
 __global__ void __launch_bounds__(TPB)
-k_update2(PlainFields f, Dims d, Box b, int odr, double ra, double rb, double dtdx, double dtdy,
-          int images)
+k_update2(PlainFields f, Dims d, Box b, int odr, double ra_, double rb_, double dtdx_,
+          double dtdy_, int images)
 {
+    const ed ra = ra_, rb = rb_, dtdx = dtdx_, dtdy = dtdy_;
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long sy = d.nx;
@@ -168,18 +170,18 @@ k_update2(PlainFields f, Dims d, Box b, int odr, double ra, double rb, double dt
 #pragma unroll
     for (int v = 0; v < 6; v++) {
         const double *fx = f.F[0][cX[v]], *fy = f.F[1][cY[v]];
-        const double d0 = fdiff(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
-        const double d1 = fdiff(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
-        out[sv[v]] = ra * f.u0[sv[v]][s] + rb * (f.s[sv[v]][s] - dtdx * d0 - dtdy * d1);
+        const ed d0 = fdiff<ed>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
+        const ed d1 = fdiff<ed>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
+        out[sv[v]] = (ra * f.u0[sv[v]][s] + rb * (ed(f.s[sv[v]][s]) - dtdx * d0 - dtdy * d1)).v;
     }
     const double *ez = f.e[2];
     {
-        const double dd = fdiff(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
-        out[5] = ra * f.u0[5][s] + rb * (f.s[5][s] - dtdy * dd);
+        const ed dd = fdiff<ed>(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
+        out[5] = (ra * f.u0[5][s] + rb * (ed(f.s[5][s]) - dtdy * dd)).v;
     }
     {
-        const double dd = fdiff(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
-        out[6] = ra * f.u0[6][s] + rb * (f.s[6][s] + dtdx * dd);
+        const ed dd = fdiff<ed>(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
+        out[6] = (ra * f.u0[6][s] + rb * (ed(f.s[6][s]) + dtdx * dd)).v;
     }
     if (!images) {
 #pragma unroll
@@ -204,22 +206,23 @@ k_update2(PlainFields f, Dims d, Box b, int odr, double ra, double rb, double dt
 // further, i < nx-xoff+1 for Bx and j < ny-yoff+1 for By); they survive the
 // boundary fill only where that axis mirrors the face array.
 __global__ void __launch_bounds__(TPB)
-k_face2(PlainFields f, Dims d, int odr, double ra, double rb, double dtdx, double dtdy, int do_x,
-        int do_y)
+k_face2(PlainFields f, Dims d, int odr, double ra_, double rb_, double dtdx_, double dtdy_,
+        int do_x, int do_y)
 {
+    const ed ra = ra_, rb = rb_, dtdx = dtdx_, dtdy = dtdy_;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const long long sy = d.nx;
     const double *ez = f.e[2];
     const int ny_in = d.ny - 2 * d.oy, nx_in = d.nx - 2 * d.ox;
     if (do_x && t < ny_in) {  // Bx at i = nx - xoff
         const long long s = d.at(d.nx - d.ox, d.oy + t, 0);
-        const double dd = fdiff(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
-        f.s[5][s] = ra * f.u0[5][s] + rb * (f.s[5][s] - dtdy * dd);
+        const ed dd = fdiff<ed>(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
+        f.s[5][s] = (ra * f.u0[5][s] + rb * (ed(f.s[5][s]) - dtdy * dd)).v;
     }
     if (do_y && t < nx_in) {  // By at j = ny - yoff
         const long long s = d.at(d.ox + t, d.ny - d.oy, 0);
-        const double dd = fdiff(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
-        f.s[6][s] = ra * f.u0[6][s] + rb * (f.s[6][s] + dtdx * dd);
+        const ed dd = fdiff<ed>(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
+        f.s[6][s] = (ra * f.u0[6][s] + rb * (ed(f.s[6][s]) + dtdx * dd)).v;
     }
 }
 

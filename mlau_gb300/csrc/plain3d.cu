@@ -51,24 +51,24 @@ k_prim3(PlainFields f, Dims d, Box b, int odr, double gamma, Bc3 bc)
     const long long wy = src3(d, i, j, k, bc.x[6], bc.y[6], bc.z[6], &gy);
     const long long wz = src3(d, i, j, k, bc.x[7], bc.y[7], bc.z[7], &gz);
     const double *bx = f.s[5], *by = f.s[6], *bz = f.s[7];
-    const double cx = gx * face2cen(odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
-    const double cy = gy * face2cen(odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
-    const double cz = gz * face2cen(odr, bz[wz - sz], bz[wz], bz[wz + sz], bz[wz + 2 * sz]);
+    const ed cx = ed(gx) * face2cen<ed>(odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
+    const ed cy = ed(gy) * face2cen<ed>(odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
+    const ed cz = ed(gz) * face2cen<ed>(odr, bz[wz - sz], bz[wz], bz[wz + sz], bz[wz + 2 * sz]);
     const long long s = d.at(i, j, k);
-    const double ro = f.s[0][s];
-    const double iro = 1.0 / ro;
-    const double vx = f.s[1][s] * iro, vy = f.s[2][s] * iro, vz = f.s[3][s] * iro;
-    const double v2 = (vx * vx + vy * vy + vz * vz);
-    const double b2 = (cx * cx + cy * cy + cz * cz);
-    const double pr = (gamma - 1) * (f.s[4][s] - 0.5 * (ro * v2 + b2));
-    f.vx[s] = vx;
-    f.vy[s] = vy;
-    f.vz[s] = vz;
-    f.pr[s] = pr;
-    f.m2[s] = v2 / (gamma * pr * iro);
-    f.cx[s] = cx;
-    f.cy[s] = cy;
-    f.cz[s] = cz;
+    const ed ro = f.s[0][s];
+    const ed iro = trcp(ro);
+    const ed vx = f.s[1][s] * iro, vy = f.s[2][s] * iro, vz = f.s[3][s] * iro;
+    const ed v2 = (vx * vx + vy * vy + vz * vz);
+    const ed b2 = (cx * cx + cy * cy + cz * cz);
+    const ed pr = ed(gamma - 1) * (f.s[4][s] - ed(0.5) * (ro * v2 + b2));
+    f.vx[s] = vx.v;
+    f.vy[s] = vy.v;
+    f.vz[s] = vz.v;
+    f.pr[s] = pr.v;
+    f.m2[s] = (v2 / (gamma * pr * iro)).v;
+    f.cx[s] = cx.v;
+    f.cy[s] = cy.v;
+    f.cz[s] = cz.v;
 }
 
 // CT weights, and the shock sensors with the sign rules of their ghost fill
@@ -115,7 +115,7 @@ k_rec3(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, int eig
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, k);
-    double q[7][5];
+    ed q[7][5];
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
@@ -127,38 +127,38 @@ k_rec3(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, int eig
         q[5][m] = v.cu[s];
         q[6][m] = f.pr[s];
     }
-    double ul[7], ur[7];
-    reconst_face(odr, eig, vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])), q, v.cn[c], gamma,
-                 ul, ur);
+    ed ul[7], ur[7];
+    reconst_face<ed>(odr, eig, vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])), q, v.cn[c], gamma,
+                     ul, ur);
 #pragma unroll
     for (int n = 0; n < 7; n++) {
-        f.ul[n][c + st] = ul[n];
-        f.ur[n][c] = ur[n];
+        f.ul[n][c + st] = ul[n].v;
+        f.ur[n][c] = ur[n].v;
     }
     // Linear interpolation of the central (B_t v_n - B_n v_t) part of the two
     // tangential B fluxes (:441-453).
-    const double bl = v.bface[c + st], br = v.bface[c];
-    double a5[5], t5[5], u5[5];
+    const ed bl = v.bface[c + st], br = v.bface[c];
+    ed a5[5], t5[5], u5[5];
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
-        a5[m] = v.ct[s] * v.vn[s];
+        a5[m] = ed(v.ct[s]) * v.vn[s];
         t5[m] = v.vt[s];
     }
-    f.ql[0][c + st] = lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - bl * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4]);
-    f.qr[0][c] = lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - br * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4]);
+    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                      - bl * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                 - br * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
-        a5[m] = v.cu[s] * v.vn[s];
+        a5[m] = ed(v.cu[s]) * v.vn[s];
         u5[m] = v.vu[s];
     }
-    f.ql[1][c + st] = lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - bl * lin_l(odr, u5[0], u5[1], u5[2], u5[3], u5[4]);
-    f.qr[1][c] = lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - br * lin_r(odr, u5[0], u5[1], u5[2], u5[3], u5[4]);
+    f.ql[1][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                      - bl * lin_l(odr, u5[0], u5[1], u5[2], u5[3], u5[4])).v;
+    f.qr[1][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                 - br * lin_r(odr, u5[0], u5[1], u5[2], u5[3], u5[4])).v;
 }
 
 __global__ void __launch_bounds__(TPB)
@@ -167,23 +167,23 @@ k_flux3(PlainFields f, SweepView v, Dims d, Box b, long long st, int D, int whic
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, k);
-    double L[7], R[7], F[7];
+    ed L[7], R[7], F[7];
 #pragma unroll
     for (int n = 0; n < 7; n++) {
         L[n] = f.ul[n][c];
         R[n] = f.ur[n][c];
     }
-    const double bn = 0.5 * (v.bface[c] + v.bface[c]);
+    const ed bn = ed(0.5) * (ed(v.bface[c]) + v.bface[c]);
     const double dvtm = vmin(vmin(v.dvt[c - st], v.dvt[c]), vmin(v.dvu[c - st], v.dvu[c]));
-    riemann(which, L, R, bn, gamma, (v.vn[c] - v.vn[c - st]), dvtm, F);
-    const double fct = 0.5 * (f.ql[0][c] + f.qr[0][c]);
-    const double fcu = 0.5 * (f.ql[1][c] + f.qr[1][c]);
+    riemann<ed>(which, L, R, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]), dvtm, F);
+    const ed fct = ed(0.5) * (ed(f.ql[0][c]) + f.qr[0][c]);
+    const ed fcu = ed(0.5) * (ed(f.ql[1][c]) + f.qr[1][c]);
     F[4] -= fct;
     F[5] -= fcu;
 #pragma unroll
-    for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n];
-    f.FC[D][0][c] = fct;
-    f.FC[D][1][c] = fcu;
+    for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n].v;
+    f.FC[D][0][c] = fct.v;
+    f.FC[D][1][c] = fcu.v;
 }
 
 __global__ void __launch_bounds__(TPB) k_emf3(PlainFields f, Dims d, Box b, int odr)
@@ -196,31 +196,32 @@ __global__ void __launch_bounds__(TPB) k_emf3(PlainFields f, Dims d, Box b, int 
                zk = (k >= 3 && k < d.nz - 2);
     // F[d][4]/F[d][5] are the fluxes of the first/second tangential B:
     //   X: (By, Bz), Y: (Bz, Bx), Z: (Bx, By).
-    double ez = 0.0, ex = 0.0, ey = 0.0;
+    ed ez = 0.0, ex = 0.0, ey = 0.0;
     if (xi && yj) {
-        const double w = f.ct[0][c];
-        ez = (0.0 + emf_part(f.F[0][4], f.FC[0][0], (1.0 - w), -1.0, c, sy, odr))
+        const ed w = f.ct[0][c];
+        ez = (ed(0.0) + emf_part(f.F[0][4], f.FC[0][0], (ed(1.0) - w), -1.0, c, sy, odr))
              + emf_part(f.F[1][5], f.FC[1][1], w, +1.0, c, 1, odr);
     }
     if (yj && zk) {
-        const double w = f.ct[1][c];
-        ex = (0.0 + emf_part(f.F[1][4], f.FC[1][0], (1.0 - w), -1.0, c, sz, odr))
+        const ed w = f.ct[1][c];
+        ex = (ed(0.0) + emf_part(f.F[1][4], f.FC[1][0], (ed(1.0) - w), -1.0, c, sz, odr))
              + emf_part(f.F[2][5], f.FC[2][1], w, +1.0, c, sy, odr);
     }
     if (zk && xi) {
-        const double w = f.ct[2][c];
-        ey = (0.0 + emf_part(f.F[0][5], f.FC[0][1], w, +1.0, c, sz, odr))
-             + emf_part(f.F[2][4], f.FC[2][0], (1.0 - w), -1.0, c, 1, odr);
+        const ed w = f.ct[2][c];
+        ey = (ed(0.0) + emf_part(f.F[0][5], f.FC[0][1], w, +1.0, c, sz, odr))
+             + emf_part(f.F[2][4], f.FC[2][0], (ed(1.0) - w), -1.0, c, 1, odr);
     }
-    f.e[0][c] = ex;
-    f.e[1][c] = ey;
-    f.e[2][c] = ez;
+    f.e[0][c] = ex.v;
+    f.e[1][c] = ey.v;
+    f.e[2][c] = ez.v;
 }
 
 __global__ void __launch_bounds__(TPB)
-k_update3(PlainFields f, Dims d, Box b, int odr, double ra, double rb, double dtdx, double dtdy,
-          double dtdz, int images)
+k_update3(PlainFields f, Dims d, Box b, int odr, double ra_, double rb_, double dtdx_,
+          double dtdy_, double dtdz_, int images)
 {
+    const ed ra = ra_, rb = rb_, dtdx = dtdx_, dtdy = dtdy_, dtdz = dtdz_;
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long sy = d.nx, sz = (long long)d.nx * d.ny;
@@ -231,26 +232,26 @@ k_update3(PlainFields f, Dims d, Box b, int odr, double ra, double rb, double dt
 #pragma unroll
     for (int v = 0; v < 5; v++) {
         const double *fx = f.F[0][cX[v]], *fy = f.F[1][cY[v]], *fz = f.F[2][cZ[v]];
-        const double d0 = fdiff(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
-        const double d1 = fdiff(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
-        const double d2 = fdiff(odr, fz[s - sz], fz[s], fz[s + sz], fz[s + 2 * sz]);
-        out[v] = ra * f.u0[v][s] + rb * (f.s[v][s] - dtdx * d0 - dtdy * d1 - dtdz * d2);
+        const ed d0 = fdiff<ed>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
+        const ed d1 = fdiff<ed>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
+        const ed d2 = fdiff<ed>(odr, fz[s - sz], fz[s], fz[s + sz], fz[s + 2 * sz]);
+        out[v] = (ra * f.u0[v][s] + rb * (ed(f.s[v][s]) - dtdx * d0 - dtdy * d1 - dtdz * d2)).v;
     }
     const double *ex = f.e[0], *ey = f.e[1], *ez = f.e[2];
     {
-        const double d0 = fdiff(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
-        const double d1 = fdiff(odr, ey[s - sz], ey[s], ey[s + sz], ey[s + 2 * sz]);
-        out[5] = ra * f.u0[5][s] + rb * (f.s[5][s] - dtdy * d0 + dtdz * d1);
+        const ed d0 = fdiff<ed>(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
+        const ed d1 = fdiff<ed>(odr, ey[s - sz], ey[s], ey[s + sz], ey[s + 2 * sz]);
+        out[5] = (ra * f.u0[5][s] + rb * (ed(f.s[5][s]) - dtdy * d0 + dtdz * d1)).v;
     }
     {
-        const double d0 = fdiff(odr, ex[s - sz], ex[s], ex[s + sz], ex[s + 2 * sz]);
-        const double d1 = fdiff(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
-        out[6] = ra * f.u0[6][s] + rb * (f.s[6][s] - dtdz * d0 + dtdx * d1);
+        const ed d0 = fdiff<ed>(odr, ex[s - sz], ex[s], ex[s + sz], ex[s + 2 * sz]);
+        const ed d1 = fdiff<ed>(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
+        out[6] = (ra * f.u0[6][s] + rb * (ed(f.s[6][s]) - dtdz * d0 + dtdx * d1)).v;
     }
     {
-        const double d0 = fdiff(odr, ey[s - 1], ey[s], ey[s + 1], ey[s + 2]);
-        const double d1 = fdiff(odr, ex[s - sy], ex[s], ex[s + sy], ex[s + 2 * sy]);
-        out[7] = ra * f.u0[7][s] + rb * (f.s[7][s] - dtdx * d0 + dtdy * d1);
+        const ed d0 = fdiff<ed>(odr, ey[s - 1], ey[s], ey[s + 1], ey[s + 2]);
+        const ed d1 = fdiff<ed>(odr, ex[s - sy], ex[s], ex[s + sy], ex[s + 2 * sy]);
+        out[7] = (ra * f.u0[7][s] + rb * (ed(f.s[7][s]) - dtdx * d0 + dtdy * d1)).v;
     }
     if (!images) {
 #pragma unroll
@@ -281,30 +282,31 @@ k_update3(PlainFields f, Dims d, Box b, int odr, double ra, double rb, double dt
 // survive the ghost fill only where that axis mirrors the face array.  One
 // thread per face of the three planes.
 __global__ void __launch_bounds__(TPB)
-k_face3(PlainFields f, Dims d, int odr, double ra, double rb, double dtdx, double dtdy,
-        double dtdz, int do_x, int do_y, int do_z)
+k_face3(PlainFields f, Dims d, int odr, double ra_, double rb_, double dtdx_, double dtdy_,
+        double dtdz_, int do_x, int do_y, int do_z)
 {
+    const ed ra = ra_, rb = rb_, dtdx = dtdx_, dtdy = dtdy_, dtdz = dtdz_;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long sy = d.nx, sz = (long long)d.nx * d.ny;
     const int Nx = d.nx - 2 * d.ox, Ny = d.ny - 2 * d.oy, Nz = d.nz - 2 * d.oz;
     const double *ex = f.e[0], *ey = f.e[1], *ez = f.e[2];
     if (do_x && t < (long long)Ny * Nz) {  // Bx at i = nx - xoff
         const long long s = d.at(d.nx - d.ox, d.oy + (int)(t % Ny), d.oz + (int)(t / Ny));
-        const double d0 = fdiff(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
-        const double d1 = fdiff(odr, ey[s - sz], ey[s], ey[s + sz], ey[s + 2 * sz]);
-        f.s[5][s] = ra * f.u0[5][s] + rb * (f.s[5][s] - dtdy * d0 + dtdz * d1);
+        const ed d0 = fdiff<ed>(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
+        const ed d1 = fdiff<ed>(odr, ey[s - sz], ey[s], ey[s + sz], ey[s + 2 * sz]);
+        f.s[5][s] = (ra * f.u0[5][s] + rb * (ed(f.s[5][s]) - dtdy * d0 + dtdz * d1)).v;
     }
     if (do_y && t < (long long)Nx * Nz) {  // By at j = ny - yoff
         const long long s = d.at(d.ox + (int)(t % Nx), d.ny - d.oy, d.oz + (int)(t / Nx));
-        const double d0 = fdiff(odr, ex[s - sz], ex[s], ex[s + sz], ex[s + 2 * sz]);
-        const double d1 = fdiff(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
-        f.s[6][s] = ra * f.u0[6][s] + rb * (f.s[6][s] - dtdz * d0 + dtdx * d1);
+        const ed d0 = fdiff<ed>(odr, ex[s - sz], ex[s], ex[s + sz], ex[s + 2 * sz]);
+        const ed d1 = fdiff<ed>(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
+        f.s[6][s] = (ra * f.u0[6][s] + rb * (ed(f.s[6][s]) - dtdz * d0 + dtdx * d1)).v;
     }
     if (do_z && t < (long long)Nx * Ny) {  // Bz at k = nz - zoff
         const long long s = d.at(d.ox + (int)(t % Nx), d.oy + (int)(t / Nx), d.nz - d.oz);
-        const double d0 = fdiff(odr, ey[s - 1], ey[s], ey[s + 1], ey[s + 2]);
-        const double d1 = fdiff(odr, ex[s - sy], ex[s], ex[s + sy], ex[s + 2 * sy]);
-        f.s[7][s] = ra * f.u0[7][s] + rb * (f.s[7][s] - dtdx * d0 + dtdy * d1);
+        const ed d0 = fdiff<ed>(odr, ey[s - 1], ey[s], ey[s + 1], ey[s + 2]);
+        const ed d1 = fdiff<ed>(odr, ex[s - sy], ex[s], ex[s + sy], ex[s + 2 * sy]);
+        f.s[7][s] = (ra * f.u0[7][s] + rb * (ed(f.s[7][s]) - dtdx * d0 + dtdy * d1)).v;
     }
 }
 

@@ -35,6 +35,13 @@ template <> MLAU_HD float tsqrt<float>(float x) { return sqrtf(x); }
 template <class T> MLAU_HD T tabs(T x) { return fabs(x); }
 template <> MLAU_HD float tabs<float>(float x) { return fabsf(x); }
 
+// 1 / x, c / x and x / 24 (the exact-double type has its own forms).
+template <class T> MLAU_HD T trcp(T x) { return T(1.0) / x; }
+template <class T> MLAU_HD T thalf_over(T x) { return T(0.5) / x; }
+template <class T> MLAU_HD T tdiv24(T x) { return x / T(24.0); }
+template <class T> MLAU_HD T tsqrt_two() { return tsqrt(T(2.0)); }
+template <class T> MLAU_HD T tsqrt_half() { return tsqrt(T(0.5)); }
+
 // Epsilon of the WCNS nonlinear weights (interp.h:154,194).  In FP32 the
 // reference's 1e-40 is a denormal that flush-to-zero removes, so FP32 uses a
 // normal number far below any weight that matters.
@@ -128,15 +135,15 @@ template <class T> MLAU_HD void wcns4_lr(T f0, T f1, T f2, T f3, T f4, T &fl, T 
     p = f4 - T(4.0) * f3 + T(3.0) * f2;
     q = f4 - T(2.0) * f3 + f2;
     s2 = T(13. / 12.) * q * q + T(0.25) * p * p;
-    s0 = T(1.0) / (s0 * s0 + eps);
-    s1 = T(1.0) / (s1 * s1 + eps);
-    s2 = T(1.0) / (s2 * s2 + eps);
+    s0 = trcp(s0 * s0 + eps);
+    s1 = trcp(s1 * s1 + eps);
+    s2 = trcp(s2 * s2 + eps);
     // The three candidate stencils are shared by both sides.
     const T pa = T(3.0) * f0 - T(10.0) * f1 + T(15.0) * f2;
     const T pb = -f1 + T(6.0) * f2 + T(3.0) * f3;
     const T pc = +T(3.0) * f2 + T(6.0) * f3 - f4;
     T w0 = T(0.075) * s0, w1 = T(0.650) * s1, w2 = T(0.275) * s2;
-    T r = T(1.0) / (w0 + w1 + w2);
+    T r = trcp(w0 + w1 + w2);
     w0 *= r;
     w1 *= r;
     w2 = T(1.0) - w0 - w1;
@@ -147,7 +154,7 @@ template <class T> MLAU_HD void wcns4_lr(T f0, T f1, T f2, T f3, T f4, T &fl, T 
     w0 = T(0.275) * s0;
     w1 = T(0.650) * s1;
     w2 = T(0.075) * s2;
-    r = T(1.0) / (w0 + w1 + w2);
+    r = trcp(w0 + w1 + w2);
     w0 *= r;
     w1 *= r;
     w2 = T(1.0) - w0 - w1;
@@ -201,7 +208,7 @@ template <class T> MLAU_HD T wcns4_f(T fuu, T fup, T f, T fdn, T fdd)
     T w0 = T(0.075) / (s0 * s0 + eps);
     T w1 = T(0.650) / (s1 * s1 + eps);
     T w2 = T(0.275) / (s2 * s2 + eps);
-    const T den = T(1.0) / (w0 + w1 + w2);
+    const T den = trcp(w0 + w1 + w2);
     w0 *= den;
     w1 *= den;
     w2 = T(1.0) - w0 - w1;
@@ -255,7 +262,7 @@ template <class T> MLAU_HD T face2cen(int odr, T f0, T f1, T f2, T f3)
 template <class T> MLAU_HD T fdiff(int odr, T f0, T f1, T f2, T f3)
 {
     if (lin_odr(odr) <= 2) return f2 - f1;
-    return (T(27.0) * (f2 - f1) - (f3 - f0)) / T(24.0);
+    return tdiv24(T(27.0) * (f2 - f1) - (f3 - f0));
 }
 
 // ---------------------------------------------------------------------------
@@ -283,15 +290,15 @@ MLAU_HD void reconst_alfven_core(int odr, const T q[7][5], const T qc[7], T bn, 
                                  T ur[7])
 {
     const T ro = qc[0], by = qc[4], bz = qc[5], pr = qc[6];
-    T iro = T(1.0) / ro;
+    T iro = trcp(ro);
     T cs2 = gamma * pr * iro;
     T ca2 = bn * bn * iro;
     T ct2 = (by * by + bz * bz) * iro;
     T cb2 = cs2 + ca2 + ct2;
     T cf2 = T(0.5) * (cb2 + tsqrt(tabs(cb2 * cb2 - T(4.0) * cs2 * ca2)));
     T sro = tsqrt(ro);
-    T isroh = T(0.5) / sro;
-    T icf2 = T(1.0) / cf2;
+    T isroh = thalf_over(sro);
+    T icf2 = trcp(cf2);
     T byh = T(0.5) * by, bzh = T(0.5) * bz;
 
     T w[7][5];
@@ -350,10 +357,10 @@ template <class T>
 MLAU_HD void eigen_full(T ro, T vx, T bx, T by, T bz, T pr, T gamma, Eigen7<T> &E)
 {
     const T eps = T(1e-12);
-    T sqrt2 = tsqrt(T(2.0));
-    T iro = T(1.0) / ro;
+    T sqrt2 = tsqrt_two<T>();
+    T iro = trcp(ro);
     T sro = tsqrt(ro);
-    T isro = T(1.0) / sro;
+    T isro = trcp(sro);
     T bxsr = bx * isro, bysr = by * isro, bzsr = bz * isro;
     T bx2 = bxsr * bxsr;
     T bt2 = bysr * bysr + bzsr * bzsr;
@@ -370,17 +377,17 @@ MLAU_HD void eigen_full(T ro, T vx, T bx, T by, T bz, T pr, T gamma, Eigen7<T> &
     bx2 = bx * bx;
     bt2 = by * by + bz * bz;
     b2 = bx2 + bt2;
-    T den = T(1.0) / tsqrt(bt2);
+    T den = trcp(tsqrt(bt2));
     bool flag = (bt2 > eps * b2);
     T bey = flag ? (by * den) : (T(0.5) * sqrt2);
     T bez = flag ? (bz * den) : (T(0.5) * sqrt2);
-    den = T(1.0) / tsqrt(tabs(cf2 - cs2));
+    den = trcp(tsqrt(tabs(cf2 - cs2)));
     flag = ((bt2 > eps * b2) || (tabs(gamma * pr - bx2) > eps * gamma * pr));
     T af = flag ? (tsqrt(tabs(a2 - cs2)) * den) : T(1.0);
     T as = flag ? (tsqrt(tabs(cf2 - a2)) * den) : T(0.0);
     T sg = (bx > T(0)) ? T(1.0) : T(-1.0);
     T cfaf = cf * af, csas = cs * as, aaaf = aa * af, aaas = aa * as;
-    den = T(0.5) / a2;
+    den = thalf_over(a2);
     E.lam[0] = vx - cf; E.lam[1] = vx - ca; E.lam[2] = vx - cs; E.lam[3] = vx;
     E.lam[4] = vx + cs; E.lam[5] = vx + ca; E.lam[6] = vx + cf;
     E.a[1] = -cfaf * den;
@@ -536,7 +543,7 @@ MLAU_HD void eigen_st_dense(T ro, T vx, T vy, T vz, T bx, T by, T bz, T pr, T ga
 // (mhd_eigen.h:206-212, :337-343).
 template <class T> MLAU_HD T fast_speed2(T ro, T bx, T by, T bz, T pr, T gamma)
 {
-    const T iro = T(1.0) / ro;
+    const T iro = trcp(ro);
     const T cs2 = gamma * pr * iro;
     const T ca2 = bx * bx * iro;
     const T ct2 = (by * by + bz * bz) * iro;
@@ -552,8 +559,8 @@ MLAU_HD void eigen_ae_dense(T ro, T vx, T vy, T vz, T bx, T by, T bz, T pr, T ga
     (void)vx; (void)vy; (void)vz; (void)al;
     const T cf2 = fast_speed2(ro, bx, by, bz, pr, gamma);
     const T sro = tsqrt(ro);
-    const T isroh = T(0.5) / sro;
-    const T icf2 = T(1.0) / cf2;
+    const T isroh = thalf_over(sro);
+    const T icf2 = trcp(cf2);
     const T byh = T(0.5) * by, bzh = T(0.5) * bz;
     const T z = T(0), one = T(1.0), h = T(0.5);
     const T l[7][7] = {{z, +one, z, z, z, z, z},
@@ -587,10 +594,10 @@ MLAU_HD void eigen_mi_dense(T ro, T vx, T vy, T vz, T bx, T by, T bz, T pr, T ga
     const T cf = tsqrt(cf2);
     const T rcf = ro * cf;
     const T sro = tsqrt(ro);
-    const T isroh = T(0.5) / sro;
-    const T icf2 = T(1.0) / cf2;
+    const T isroh = thalf_over(sro);
+    const T icf2 = trcp(cf2);
     const T icf2h = T(0.5) * icf2;
-    const T ircfh = T(0.5) / rcf;
+    const T ircfh = thalf_over(rcf);
     const T byh = T(0.5) * by, bzh = T(0.5) * bz;
     const T z = T(0), one = T(1.0);
     const T l[7][7] = {{z, -rcf, z, z, +by, +bz, +one},
@@ -739,17 +746,17 @@ MLAU_HD void flux_mlau(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     const T EPS = T(1e-8);
     const T rol = L[0], vnl = L[1], vtl = L[2], vul = L[3], btl = L[4], bul = L[5], prl = L[6];
     const T ror = R[0], vnr = R[1], vtr = R[2], vur = R[3], btr = R[4], bur = R[5], prr = R[6];
-    T gm1i = T(1.0) / (gamma - T(1.0));
+    T gm1i = trcp(gamma - T(1.0));
     T bnc2 = bnc * bnc;
     T sgn = (bnc > T(0)) ? T(1.0) : T(-1.0);
     T bnca = sgn * bnc;
-    T roli = T(1.0) / rol;
+    T roli = trcp(rol);
     T vl2 = vnl * vnl + vtl * vtl + vul * vul;
     T pml = T(0.5) * (btl * btl + bul * bul);
     T ptl = prl + pml;
     T enl = gm1i * prl + pml + T(0.5) * rol * vl2;
     T hnl = (enl + ptl) * roli;
-    T rori = T(1.0) / ror;
+    T rori = trcp(ror);
     T vr2 = vnr * vnr + vtr * vtr + vur * vur;
     T pmr = T(0.5) * (btr * btr + bur * bur);
     T ptr = prr + pmr;
@@ -767,7 +774,7 @@ MLAU_HD void flux_mlau(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     T ccr2 = T(0.5) * (cbr2 + tsqrt(tabs(cbr2 * cbr2 - T(4.0) * vr2 * car2)));
     T cmax = tsqrt(vmax(cfl2, cfr2));
     T cfn = cmax;
-    T cfni = T(1.0) / cfn;
+    T cfni = trcp(cfn);
     T sl = vmin(T(0.0), vmin(vnl, vnr) - cmax);
     T sr = vmax(T(0.0), vmax(vnl, vnr) + cmax);
     T mal = vnl * cfni, mar = vnr * cfni;
@@ -815,7 +822,7 @@ MLAU_HD void flux_mlau(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     T vnc = ((tabs(vndnm) > EPS) && (snc != T(0))) ? (mflux * snc / vndnm)
                                                     : (dirl * vnl + dirr * vnr);
     T slvc = sl - vnc, srvc = sr - vnc;
-    T slvci = T(1.0) / slvc, srvci = T(1.0) / srvc;
+    T slvci = trcp(slvc), srvci = trcp(srvc);
     T rhdl = rol * slvl * slvc - bnc2;
     T rhdr = ror * srvr * srvc - bnc2;
     T dvtl = T(0.0), dvul = T(0.0), dbtl = T(0.0), dbul = T(0.0);
@@ -843,7 +850,7 @@ MLAU_HD void flux_mlau(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     T sror = tsqrt(ro2r);
     T vt2r = dvtr + vtr, vu2r = dvur + vur;
     T bt2r = dbtr + btr * cmpr, bu2r = dbur + bur * cmpr;
-    T sroi = T(1.0) / (srol + sror);
+    T sroi = trcp(srol + sror);
     T srollri = srol * sroi, srorlri = sror * sroi;
     T bnflb = sgn * vmin(vmax(T(0.0), srollri * (bnca + sror * vnc)), bnca);
     T bnfrb = sgn * vmin(vmax(T(0.0), srorlri * (bnca - srol * vnc)), bnca);
@@ -889,16 +896,16 @@ MLAU_HD void flux_hlld(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     const T EPS = T(1e-8);
     const T rol = L[0], vnl = L[1], vtl = L[2], vul = L[3], btl = L[4], bul = L[5], prl = L[6];
     const T ror = R[0], vnr = R[1], vtr = R[2], vur = R[3], btr = R[4], bur = R[5], prr = R[6];
-    T gm1i = T(1.0) / (gamma - T(1.0));
+    T gm1i = trcp(gamma - T(1.0));
     T bnc2 = bnc * bnc;
     T sgn = (bnc > T(0)) ? T(1.0) : T(-1.0);
-    T roli = T(1.0) / rol;
+    T roli = trcp(rol);
     T pml = T(0.5) * (btl * btl + bul * bul);
     T ptl = prl + pml;
     T vl2 = vnl * vnl + vtl * vtl + vul * vul;
     T enl = gm1i * prl + pml + T(0.5) * rol * vl2;
     T vbl = vtl * btl + vul * bul;
-    T rori = T(1.0) / ror;
+    T rori = trcp(ror);
     T pmr = T(0.5) * (btr * btr + bur * bur);
     T ptr = prr + pmr;
     T vr2 = vnr * vnr + vtr * vtr + vur * vur;
@@ -919,7 +926,7 @@ MLAU_HD void flux_hlld(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
         srvr = sr - vnr;
         rslvl = rol * slvl;
         rsrvr = ror * srvr;
-        drsvi = T(1.0) / (rsrvr - rslvl);
+        drsvi = trcp(rsrvr - rslvl);
         if (JUMPS) {
             vnc = (rsrvr * vnr - rslvl * vnl - jp) * drsvi;
             ptc = (rsrvr * ptl - rslvl * ptr + rsrvr * rslvl * jv) * drsvi;
@@ -939,7 +946,7 @@ MLAU_HD void flux_hlld(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
         srvr = sr - vnr;
         rslvl = rol * slvl;
         rsrvr = ror * srvr;
-        drsvi = T(1.0) / (rsrvr - rslvl);
+        drsvi = trcp(rsrvr - rslvl);
         T theta = vmin(T(1.0), (cmax - vmin(dv0, T(0.0))) / (cmax - vmin(dv1, T(0.0))));
         theta *= theta;
         theta *= theta;
@@ -954,7 +961,7 @@ MLAU_HD void flux_hlld(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     T rhdl = rslvl * slvc - bnc2, rhdr = rsrvr * srvc - bnc2;
     T vt2l, vu2l, bt2l, bu2l, vt2r, vu2r, bt2r, bu2r;
     if (tabs(rhdl) > EPS) {
-        T rhdli = T(1.0) / rhdl;
+        T rhdli = trcp(rhdl);
         T rhnvl = (vnl - vnc) * bnc;
         T rhnbl = rslvl * slvl - bnc2;
         vt2l = vtl + rhnvl * rhdli * btl;
@@ -965,7 +972,7 @@ MLAU_HD void flux_hlld(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
         vt2l = vtl; vu2l = vul; bt2l = btl; bu2l = bul;
     }
     if (tabs(rhdr) > EPS) {
-        T rhdri = T(1.0) / rhdr;
+        T rhdri = trcp(rhdr);
         T rhnvr = (vnr - vnc) * bnc;
         T rhnbr = rsrvr * srvr - bnc2;
         vt2r = vtr + rhnvr * rhdri * btr;
@@ -980,7 +987,7 @@ MLAU_HD void flux_hlld(const T *L, const T *R, T bnc, T gamma, T dv0, T dv1, T *
     T en2l = (slvl * enl - ptl * vnl + ptc * vnc + bnc * (vbl - vb2l)) / slvc;
     T en2r = (srvr * enr - ptr * vnr + ptc * vnc + bnc * (vbr - vb2r)) / srvc;
     T rro2l = tsqrt(ro2l), rro2r = tsqrt(ro2r);
-    T rro2i = T(1.0) / (rro2r + rro2l);
+    T rro2i = trcp(rro2r + rro2l);
     T vt3m = (rro2r * vt2r + rro2l * vt2l + (bt2r - bt2l) * sgn) * rro2i;
     T vu3m = (rro2r * vu2r + rro2l * vu2l + (bu2r - bu2l) * sgn) * rro2i;
     T bt3m = (rro2l * bt2r + rro2r * bt2l + rro2r * rro2l * (vt2r - vt2l) * sgn) * rro2i;
@@ -1016,12 +1023,12 @@ MLAU_HD void flux_roe(const T *L, const T *R, T bnc, T gamma, T *f)
     const T EPS = T(1e-8);
     const T rol = L[0], vnl = L[1], vtl = L[2], vul = L[3], btl = L[4], bul = L[5], prl = L[6];
     const T ror = R[0], vnr = R[1], vtr = R[2], vur = R[3], btr = R[4], bur = R[5], prr = R[6];
-    T gm1 = gamma - T(1.0), gm2 = gamma - T(2.0), gm1i = T(1.0) / gm1;
-    T roli = T(1.0) / rol, rori = T(1.0) / ror;
+    T gm1 = gamma - T(1.0), gm2 = gamma - T(2.0), gm1i = trcp(gm1);
+    T roli = trcp(rol), rori = trcp(ror);
     T rrol = tsqrt(rol), rror = tsqrt(ror);
-    T rroi = T(1.0) / (rrol + rror);
+    T rroi = trcp(rrol + rror);
     T robar = rrol * rror;
-    T robari = T(1.0) / robar;
+    T robari = trcp(robar);
     T rrobar = tsqrt(robar);
     T rrobai = tsqrt(robari);
     T vnbar = (rrol * vnl + rror * vnr) * rroi;
@@ -1048,20 +1055,20 @@ MLAU_HD void flux_roe(const T *L, const T *R, T bnc, T gamma, T *f)
     T cf2 = T(0.5) * (a2 + tsqrt(cb2 * (a2 + c2 + ca2) + (c2 - ca2) * (c2 - ca2)));
     T cs2 = c2 * ca2 / cf2;
     T cf = tsqrt(cf2), cs = tsqrt(cs2), ca = tsqrt(ca2), c = tsqrt(c2);
-    T cfi = T(1.0) / cf;
+    T cfi = trcp(cf);
     T sgr1 = btbar * btbar + bubar * bubar - EPS;
     T sf11 = (sgr1 > T(0)) ? T(1.0) : T(0.0);
     T sf21 = T(1.0) - sf11;
-    T beti = T(1.0) / tsqrt(btbar * btbar + bubar * bubar + sf21);
-    T bett = sf11 * btbar * beti + sf21 * tsqrt(T(0.5));
-    T betu = sf11 * bubar * beti + sf21 * tsqrt(T(0.5));
+    T beti = trcp(tsqrt(btbar * btbar + bubar * bubar + sf21));
+    T bett = sf11 * btbar * beti + sf21 * tsqrt_half<T>();
+    T betu = sf11 * bubar * beti + sf21 * tsqrt_half<T>();
     T sgr2 = (btbar * btbar + bubar * bubar) * robari + tabs(ca2 - c2) - EPS;
     T sf12 = (sgr2 > T(0)) ? T(1.0) : T(0.0);
     T sf22 = T(1.0) - sf12;
     T cfca = vmax(T(0.0), cf2 - ca2);
     T cfcs = vmax(T(0.0), cf2 - cs2);
     T cfa = vmax(T(0.0), cf2 - c2);
-    T alpi = T(1.0) / tsqrt(cfcs + sf22);
+    T alpi = trcp(tsqrt(cfcs + sf22));
     T alpf = sf12 * tsqrt(cfca) * alpi + sf22;
     T alps = sf12 * tsqrt(cfa) * alpi;
     const T eeps = T(0.0);
@@ -1089,8 +1096,8 @@ MLAU_HD void flux_roe(const T *L, const T *R, T bnc, T gamma, T *f)
     T p22 = alps * (cs2 - c2 * gm2 * gm1i);
     T q11 = alpf * cf, q12 = alps * cs;
     T q21 = -alps * ca * sgn, q22 = alpf * c * sgn;
-    T detpi = T(1.0) / (p11 * p22 - p12 * p21);
-    T detqi = T(1.0) / (q11 * q22 - q12 * q21);
+    T detpi = trcp(p11 * p22 - p12 * p21);
+    T detqi = trcp(q11 * q22 - q12 * q21);
     T wv[7];
     T pa = (p22 * t1 - p12 * t2) * detpi, qa = (q22 * s1 - q12 * s2) * detqi;
     T pb = (-p21 * t1 + p11 * t2) * detpi, qb = (-q21 * s1 + q11 * s2) * detqi;

@@ -3,6 +3,7 @@
 
 #include "sim.cuh"
 #include "point.cuh"
+#include "ed.cuh"
 
 namespace mlau {
 namespace {
@@ -43,28 +44,31 @@ __device__ __forceinline__ double ct_weight(const double *va, const double *vb, 
                                             const double *ba, const double *bbf, long long s,
                                             long long P, long long Q, long long oa, long long ob)
 {
-    const double eps = 1e-6;
-    double a = 0.25 * (va[s - P - Q] + va[s - P] + va[s - Q] + va[s]);
-    double c = 0.25 * (vb[s - P - Q] + vb[s - P] + vb[s - Q] + vb[s]);
-    double rc = 0.25 * (ro[s - P - Q] + ro[s - P] + ro[s - Q] + ro[s]);
-    rc = 1.0 / sqrt(rc);
-    double fa = 0.5 * (ba[s - oa] + ba[s]);
-    double fb = 0.5 * (bbf[s - ob] + bbf[s]);
-    a = fabs(a) + fabs(fa * rc);
-    c = fabs(c) + fabs(fb * rc);
-    return (a + 0.5 * eps) / (a + c + eps);
+    const ed eps = 1e-6, h = 0.5, q = 0.25;
+    auto sum4 = [&](const double *f) { return ed(f[s - P - Q]) + f[s - P] + f[s - Q] + f[s]; };
+    ed a = q * sum4(va);
+    ed c = q * sum4(vb);
+    ed rc = q * sum4(ro);
+    rc = trcp(tsqrt(rc));
+    const ed fa = h * (ed(ba[s - oa]) + ba[s]);
+    const ed fb = h * (ed(bbf[s - ob]) + bbf[s]);
+    a = tabs(a) + tabs(fa * rc);
+    c = tabs(c) + tabs(fb * rc);
+    return ((a + ed(0.5 * 1e-6)) / (a + c + eps)).v;
 }
 
 // One edge contribution: sgn*0.5*((ul0+ur0) + w*(ul1+ur1)) with ul from the
 // linear interpolation centred one edge below and ur centred on the edge.
-__device__ __forceinline__ double emf_part(const double *fu, const double *fc, double w,
-                                           double sgn, long long c, long long st, int odr)
+__device__ __forceinline__ ed emf_part(const double *fu, const double *fc, ed w, double sgn,
+                                       long long c, long long st, int odr)
 {
-    const double ul0 = lin_l(odr, fu[c - 3 * st], fu[c - 2 * st], fu[c - st], fu[c], fu[c + st]);
-    const double ul1 = lin_l(odr, fc[c - 3 * st], fc[c - 2 * st], fc[c - st], fc[c], fc[c + st]);
-    const double ur0 = lin_r(odr, fu[c - 2 * st], fu[c - st], fu[c], fu[c + st], fu[c + 2 * st]);
-    const double ur1 = lin_r(odr, fc[c - 2 * st], fc[c - st], fc[c], fc[c + st], fc[c + 2 * st]);
-    return sgn * 0.5 * ((ul0 + ur0) + w * (ul1 + ur1));
+    auto l = [&](const double *f) {
+        return lin_l<ed>(odr, f[c - 3 * st], f[c - 2 * st], f[c - st], f[c], f[c + st]);
+    };
+    auto r = [&](const double *f) {
+        return lin_r<ed>(odr, f[c - 2 * st], f[c - st], f[c], f[c + st], f[c + 2 * st]);
+    };
+    return ed(sgn * 0.5) * ((l(fu) + r(fu)) + w * (l(fc) + r(fc)));
 }
 
 inline void rk_coef(int nrk, int stage, double &a, double &b)
