@@ -88,4 +88,5 @@ template <> MLAU_HD ed tsqrt_two<ed>() { return 0x1.6a09e667f3bcdp+0; }
 template <> MLAU_HD ed tsqrt_half<ed>() { return 0x1.6a09e667f3bcdp-1; }
 template <> MLAU_HD ed tdiv24<ed>(ed x) { return x64::div24(x.v); }
 
+
 }  // namespace mlau

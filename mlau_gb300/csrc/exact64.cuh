@@ -1,5 +1,5 @@
-// Reciprocal, division and square root of doubles, correctly rounded (round to
-// nearest even), computed on the integer and FP32 pipes.
+// Reciprocal, division, square root and product of doubles, correctly rounded
+// (round to nearest even), computed on the integer and FP32 pipes.
 //
 // Why: this part's FP64 pipe takes 64 cycles per warp instruction in each SM
 // sub-partition (2 lanes per cycle per SM), and CUDA's own FP64 division,
@@ -145,6 +145,78 @@ X64 uint32_t off_range(uint32_t h, uint32_t g)
     return ((h + 0x50000000u) | (g + 0x50000000u)) & 0x60000000u;
 }
 
+// Round (h:l | m as a fraction of 2^32 below l) to nearest even and add the
+// exponent and sign word e: the packed double.
+X64 double round_pack(uint32_t h, uint32_t l, uint32_t m, uint32_t e)
+{
+#ifdef __CUDA_ARCH__
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %0, 0;\n\t"
+        "addc.u32 %1, %1, %4;\n\t}"
+        : "+r"(l), "+r"(h)
+        : "r"(m), "r"(0x7fffffffu + (l & 1u)), "r"(e));
+    return make(h, l);
+#else
+    const uint64_t c = ((uint64_t)m + 0x7fffffffu + (l & 1u)) >> 32;
+    const uint64_t v = (((uint64_t)h << 32) | l) + c;
+    return make((uint32_t)(v >> 32) + e, (uint32_t)v);
+#endif
+}
+
+// 106-bit product w3:w2:w1:w0 of two 53-bit significands -> rounded double.
+// sg: sign and exponent word of the product before normalisation.
+X64 double norm_product(uint64_t p11, uint32_t w1, uint32_t w0, uint32_t sg)
+{
+    const uint32_t w3 = (uint32_t)(p11 >> 32), w2 = (uint32_t)p11;
+    const uint32_t s = 12u - (w3 >> 9);
+    const uint32_t h = shfl_(w2, w3, (int)s), l = shfl_(w1, w2, (int)s);
+    const uint32_t m = shfl_(w0, w1, (int)s) | (w0 < 1u ? w0 : 1u);
+    return round_pack(h, l, m, sg - (s << 20));
+}
+
+// Product, square and small odd multiple of doubles in range (see off_range;
+// the caller checks).
+X64 double mul_fast(double a, double b)
+{
+    const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
+    const uint32_t ma = (ah & 0xfffffu) | 0x100000u, mb = (bh & 0xfffffu) | 0x100000u;
+    const uint64_t p00 = wide(al, bl);
+    const uint64_t p01 = wide(al, mb) + (p00 >> 32);
+    const uint64_t p10 = wide(ma, bl) + (uint32_t)p01;
+    const uint64_t p11 = wide(ma, mb) + (p01 >> 32) + (p10 >> 32);
+    const uint32_t sg = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) + ((ah ^ bh) & 0x80000000u) -
+                        (1012u << 20);
+    return norm_product(p11, (uint32_t)p10, (uint32_t)p00, sg);
+}
+
+X64 double sqr_fast(double a)
+{
+    const uint32_t ah = hi32(a), al = lo32(a);
+    const uint32_t ma = (ah & 0xfffffu) | 0x100000u;
+    const uint64_t p00 = wide(al, al);
+    const uint64_t p01 = wide(al, 2u * ma) + (p00 >> 32);
+    const uint64_t p11 = wide(ma, ma) + (p01 >> 32);
+    const uint32_t sg = ((ah & 0x7ff00000u) << 1) - (1012u << 20);
+    return norm_product(p11, (uint32_t)p01, (uint32_t)p00, sg);
+}
+
+// k * a for an odd integer k in [3, 255]
+template <int K> X64 double mulk_fast(double a)
+{
+    constexpr int B = K < 4 ? 2 : K < 8 ? 3 : K < 16 ? 4 : K < 32 ? 5 : K < 64 ? 6 : K < 128 ? 7 : 8;
+    // K << (11 - B) brings the 53-bit significand's product to bit 63 or 62
+    constexpr uint32_t KS = (uint32_t)K << (11 - B);
+    const uint32_t ah = hi32(a), al = lo32(a);
+    const uint32_t ma = (ah & 0xfffffu) | 0x100000u;
+    const uint64_t p0 = wide(al, KS);
+    const uint32_t xl = (uint32_t)p0, xh = ma * KS + (uint32_t)(p0 >> 32);
+    // significand = X >> (11 - s), s = 1 where bit 63 is clear
+    const uint32_t t = 10u + (xh >> 31);
+    const uint32_t h = xh >> t, l = shfr_(xl, xh, (int)t), f = xl << (32u - t);
+    const uint32_t e = (ah & 0xfff00000u) + (t << 20) + ((uint32_t)(B - 12) << 20);
+    return round_pack(h, l, f, e);
+}
+
+
 // Reciprocal seed of the 53-bit significand (mh:ml) in [2^52, 2^53): Y0 in
 // [2^23, 2^24) with Y0 ~ 2^76 / B, and e1 = (B Y0 - 2^76) >> 24.
 X64 void rcp_seed(uint32_t mh, uint32_t ml, uint32_t &Y0, int32_t &e1)
@@ -164,7 +236,8 @@ static X64_SLOW double rcp_hw(double x) { return 1.0 / x; }
 static X64_SLOW double div_hw(double a, double b) { return a / b; }
 static X64_SLOW double sqrt_hw(double x) { return ::sqrt(x); }
 
-X64 double rcp(double x)
+// bad: nonzero where the pipe's operation has to decide
+X64 double rcp_fast(double x, uint32_t &bad)
 {
     const uint32_t ah = hi32(x), ml = lo32(x);
     const uint32_t mh = (ah & 0xfffffu) | 0x100000u;
@@ -182,12 +255,19 @@ X64 double rcp(double x)
     const int32_t P = (int32_t)(((int64_t)r * (int32_t)shfr_(ql, qh, 23)) >> 32);
     const int32_t T = P + (1 << 17);
     const uint64_t Q = Q1 + (uint64_t)(int64_t)(T >> 18);
-    const bool ok = off_range(ah) == 0 && (((uint32_t)T + 4u) & 0x3ffffu) > 8u;
+    bad |= off_range(ah) | ((((uint32_t)T + 4u) & 0x3ffffu) <= 8u ? 1u : 0u);
     const uint32_t e = (2044u << 20) - (ah & 0x7ff00000u) + (ah & 0x80000000u);
-    double q = make((uint32_t)(Q >> 32) + e, (uint32_t)Q);
-    if (!ok) q = rcp_hw(x);
+    return make((uint32_t)(Q >> 32) + e, (uint32_t)Q);
+}
+
+X64 double rcp(double x)
+{
+    uint32_t bad = 0;
+    double q = rcp_fast(x, bad);
+    if (bad) q = rcp_hw(x);
     return q;
 }
+
 
 // 0.5 / x
 X64 double half_over(double x)

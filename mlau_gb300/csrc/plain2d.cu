@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "stencil.cuh"
+#include "rec_exact.cuh"
 
 namespace mlau {
 namespace {
@@ -76,6 +77,24 @@ View2 make_view2(const PlainFields &f, int D)
     return {f.vy, f.vz, f.vx, f.cy, f.s[7], f.cx, f.s[6], f.dv[0], 1};
 }
 
+// The linear interpolation of the central part of the split tangential B flux.
+__device__ __forceinline__ void rec_central2(const PlainFields &f, const View2 &v, long long c,
+                                             long long st, int odr)
+{
+    const double *bt = v.split_u ? v.cu : v.ct, *vt = v.split_u ? v.vu : v.vt;
+    ed a5[5], t5[5];
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        const long long s = c + st * (m - 2);
+        a5[m] = ed(bt[s]) * v.vn[s];
+        t5[m] = vt[s];
+    }
+    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                      - ed(v.bface[c + st]) * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                 - ed(v.bface[c]) * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+}
+
 __global__ void __launch_bounds__(TPB)
 k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, double gamma)
 {
@@ -102,18 +121,28 @@ k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, do
         f.ul[n][c + st] = ul[n].v;
         f.ur[n][c] = ur[n].v;
     }
-    const double *bt = v.split_u ? v.cu : v.ct, *vt = v.split_u ? v.vu : v.vt;
-    ed a5[5], t5[5];
+    rec_central2(f, v, c, st, odr);
+}
+
+// WCNS4 with the drivers' eigen-systems.
+__global__ void __launch_bounds__(TPB, 4)
+k_rec2_wcns4(PlainFields f, View2 v, Dims d, Box b, long long st, double gamma)
+{
+    __shared__ double w[35][TPB];
+    int i, j, k;
+    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    const long long c = d.at(i, j, 0);
+    const double *src[7] = {f.s[0], v.vn, v.vt, v.vu, v.ct, v.cu, f.pr};
+    auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
+    const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
+    ed ul[7], ur[7];
+    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, ul, ur);
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const long long s = c + st * (m - 2);
-        a5[m] = ed(bt[s]) * v.vn[s];
-        t5[m] = vt[s];
+    for (int n = 0; n < 7; n++) {
+        f.ul[n][c + st] = ul[n].v;
+        f.ur[n][c] = ur[n].v;
     }
-    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - ed(v.bface[c + st]) * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
-    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - ed(v.bface[c]) * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    rec_central2(f, v, c, st, 4);
 }
 
 __global__ void __launch_bounds__(TPB)
@@ -299,8 +328,11 @@ int plain2d_step(Sim *s, double dt)
             else { rb_.lo1 = 2; rb_.e1 = g.ny - 4; fb.lo1 = 3; fb.e1 = g.ny - 5; }
             {
                 TimedLaunch tl(&s->timer, KK_REC);
-                k_rec2<<<blocks_for(rb_.count(), TPB), TPB, 0, st>>>(f, v, d, rb_, stride, s->odr,
-                                                                     s->eig, s->gamma);
+                const unsigned nb = blocks_for(rb_.count(), TPB);
+                if (s->odr == 4 && s->eig == EIG_FULL)
+                    k_rec2_wcns4<<<nb, TPB, 0, st>>>(f, v, d, rb_, stride, s->gamma);
+                else
+                    k_rec2<<<nb, TPB, 0, st>>>(f, v, d, rb_, stride, s->odr, s->eig, s->gamma);
             }
             {
                 TimedLaunch tl(&s->timer, KK_FLUX);

@@ -27,6 +27,7 @@
 #include "sim.cuh"
 #include "point.cuh"
 #include "stencil.cuh"
+#include "rec_exact.cuh"
 
 namespace mlau {
 namespace {
@@ -109,6 +110,35 @@ __host__ SweepView make_view(const PlainFields &f, int D)
     return {f.vz, f.vx, f.vy, f.cz, f.cx, f.cy, f.s[7], f.dv[0], f.dv[1]};
 }
 
+// The linear interpolation of the central (B_t v_n - B_n v_t) parts of the two
+// tangential B fluxes (:441-453).
+__device__ __forceinline__ void rec_central(const PlainFields &f, const SweepView &v, long long c,
+                                            long long st, int odr)
+{
+    const ed bl = v.bface[c + st], br = v.bface[c];
+    ed a5[5], t5[5], u5[5];
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        const long long s = c + st * (m - 2);
+        a5[m] = ed(v.ct[s]) * v.vn[s];
+        t5[m] = v.vt[s];
+    }
+    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                      - bl * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                 - br * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+#pragma unroll
+    for (int m = 0; m < 5; m++) {
+        const long long s = c + st * (m - 2);
+        a5[m] = ed(v.cu[s]) * v.vn[s];
+        u5[m] = v.vu[s];
+    }
+    f.ql[1][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                      - bl * lin_l(odr, u5[0], u5[1], u5[2], u5[3], u5[4])).v;
+    f.qr[1][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                 - br * lin_r(odr, u5[0], u5[1], u5[2], u5[3], u5[4])).v;
+}
+
 __global__ void __launch_bounds__(TPB)
 k_rec3(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, int eig, double gamma)
 {
@@ -135,30 +165,28 @@ k_rec3(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, int eig
         f.ul[n][c + st] = ul[n].v;
         f.ur[n][c] = ur[n].v;
     }
-    // Linear interpolation of the central (B_t v_n - B_n v_t) part of the two
-    // tangential B fluxes (:441-453).
-    const ed bl = v.bface[c + st], br = v.bface[c];
-    ed a5[5], t5[5], u5[5];
+    rec_central(f, v, c, st, odr);
+}
+
+// WCNS4 with the drivers' eigen-systems.
+__global__ void __launch_bounds__(TPB, 4)
+k_rec3_wcns4(PlainFields f, SweepView v, Dims d, Box b, long long st, double gamma)
+{
+    __shared__ double w[35][TPB];
+    int i, j, k;
+    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    const long long c = d.at(i, j, k);
+    const double *src[7] = {f.s[0], v.vn, v.vt, v.vu, v.ct, v.cu, f.pr};
+    auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
+    const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
+    ed ul[7], ur[7];
+    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, ul, ur);
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const long long s = c + st * (m - 2);
-        a5[m] = ed(v.ct[s]) * v.vn[s];
-        t5[m] = v.vt[s];
+    for (int n = 0; n < 7; n++) {
+        f.ul[n][c + st] = ul[n].v;
+        f.ur[n][c] = ur[n].v;
     }
-    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - bl * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
-    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - br * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const long long s = c + st * (m - 2);
-        a5[m] = ed(v.cu[s]) * v.vn[s];
-        u5[m] = v.vu[s];
-    }
-    f.ql[1][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - bl * lin_l(odr, u5[0], u5[1], u5[2], u5[3], u5[4])).v;
-    f.qr[1][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - br * lin_r(odr, u5[0], u5[1], u5[2], u5[3], u5[4])).v;
+    rec_central(f, v, c, st, 4);
 }
 
 __global__ void __launch_bounds__(TPB)
@@ -404,8 +432,11 @@ int plain3d_step(Sim *s, double dt)
             *e_f[D] = len - 5;  // faces [3, len-2)
             {
                 TimedLaunch tl(&s->timer, KK_REC);
-                k_rec3<<<blocks_for(rb_.count(), TPB), TPB, 0, st>>>(f, v, d, rb_, strides[D],
-                                                                     s->odr, s->eig, s->gamma);
+                const unsigned nb = blocks_for(rb_.count(), TPB);
+                if (s->odr == 4 && s->eig == EIG_FULL)
+                    k_rec3_wcns4<<<nb, TPB, 0, st>>>(f, v, d, rb_, strides[D], s->gamma);
+                else
+                    k_rec3<<<nb, TPB, 0, st>>>(f, v, d, rb_, strides[D], s->odr, s->eig, s->gamma);
             }
             {
                 TimedLaunch tl(&s->timer, KK_FLUX);

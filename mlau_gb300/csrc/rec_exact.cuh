@@ -1,0 +1,214 @@
+// Characteristic WCNS4 reconstruction of one cell for the plain FP64 kernels:
+// the values of reconst_full / reconst_alfven with wcns4_lr (point.cuh), bit
+// for bit, with the work split between the FP64 pipe and the integer pipes.
+//
+// What bounds it: the FP64 pipe, 64 cycles per warp instruction and
+// sub-partition.  Of the 92 products and 41 sums of one field's wcns4_lr, the
+// sums stay on that pipe, those by 2 and 4 fused into them (exact scalings);
+// the other products and the five reciprocals run as integer instructions
+// (exact64.cuh: 51 / 45 / 24 / 75 cycles for a b, a a, k a, 1 / x), in the
+// issue slots the FP64 pipe leaves idle.  The seven fields go through one loop
+// over a shared-memory scratch, since unrolled the code would overflow the
+// instruction cache.  One flag collects the operands outside the integer path's
+// range and the undecided reciprocals; such a lane evaluates the field on the
+// FP64 pipe alone.  Five equal values (a uniform region) take constants.
+//
+// Reconstruction of a 3D 128^3 MLAU step: 34.0 -> 20.5 ms (FP64 pipe 91 %
+// busy, issue slots 31 %); 2D 512^2 pass 4.31 -> 2.87 ms.
+#pragma once
+
+#include "ed.cuh"
+
+namespace mlau {
+
+// wcns4_lr on the FP64 pipe.
+static __device__ __noinline__ double2 wcns4_pipe(double f0, double f1, double f2, double f3, double f4)
+{
+    double2 r;
+    wcns4_lr<double>(f0, f1, f2, f3, f4, r.x, r.y);
+    return r;
+}
+
+// Constants that stay in registers (a constant operand slows the FP64 pipe).
+struct ConstReg {
+    uint32_t z;
+    __device__ __forceinline__ ConstReg() : z(opaque_zero()) {}
+    __device__ __forceinline__ double operator()(double c) const
+    {
+        return __hiloint2double((int)((uint32_t)__double2hiint(c) + z), (int)((uint32_t)__double2loint(c) + z));
+    }
+};
+
+// A stencil of five equal values c != 0: the weights are constants.
+static __device__ __noinline__ double2 wcns4_const(double c)
+{
+    constexpr double S = 1.0 / 1e-40, A = 0.075 * S, M = 0.65 * S, C = 0.275 * S;
+    constexpr double rl = 1.0 / (A + M + C), rr = 1.0 / (C + M + A);
+    constexpr double l0 = A * rl, l1 = M * rl, l2 = 1.0 - l0 - l1;
+    constexpr double r0 = C * rr, r1 = M * rr, r2 = 1.0 - r0 - r1;
+    const double c3 = 3.0 * c, c6 = 6.0 * c;
+    const double pa = c3 - 10.0 * c + 15.0 * c, pb = -c + c6 + c3, pc = c3 + c6 - c;
+    return make_double2(0.125 * (l0 * pa + l1 * pb + l2 * pc), 0.125 * (r2 * pa + r1 * pb + r0 * pc));
+}
+
+// (value at i+1/2 from the left, at i-1/2 from the right) of one field.  A
+// product by a power of two is exact, so 3 f2 serves 6 f2, and 0.25 p p is a
+// quarter of the rounded p p; the operands' range excludes the underflow that
+// would tell them apart.
+__device__ __forceinline__ double2 wcns4_ed(double f0, double f1, double f2, double f3, double f4)
+{
+    using namespace x64;
+    const uint32_t h2 = hi32(f2), l2 = lo32(f2);
+    if ((((hi32(f0) ^ h2) | (hi32(f1) ^ h2)) | ((hi32(f3) ^ h2) | (hi32(f4) ^ h2)) |
+         ((lo32(f0) ^ l2) | (lo32(f1) ^ l2)) | ((lo32(f3) ^ l2) | (lo32(f4) ^ l2))) == 0)
+        return (h2 << 1 | l2) == 0 ? make_double2(0.0, 0.0) : wcns4_const(f2);
+    const ConstReg K;
+    uint32_t bad = off_range(hi32(f0), hi32(f1)) | off_range(h2, hi32(f3)) | off_range(hi32(f4));
+    const double one = K(1.0), m4 = K(-4.0), m2 = K(-2.0), p2 = K(2.0), q4 = K(0.25), eps = K(1e-40);
+    auto add = [&](double a, double b) { return __fma_rn(a, one, b); };
+    auto sub = [&](double a, double b) { return __fma_rn(-b, one, a); };
+    auto mul = [&](double a, double b) {
+        bad |= off_range(hi32(a), hi32(b));
+        return mul_fast(a, b);
+    };
+    auto mulc = [&](double c, double b) {
+        bad |= off_range(hi32(b));
+        return mul_fast(c, b);
+    };
+    auto sqr = [&](double a) {
+        bad |= off_range(hi32(a));
+        return sqr_fast(a);
+    };
+    auto eighth = [&](double v) {
+        bad |= off_range(hi32(v));
+        return make(hi32(v) - (3u << 20), lo32(v));
+    };
+    const double t2 = mulk_fast<3>(f2);
+    auto ind = [&](double p, double q) {
+        const double s = __fma_rn(q4, sqr(p), mul(mulc(13. / 12., q), q));
+        return rcp_fast(add(sqr(s), eps), bad);
+    };
+    const double s0 = ind(add(__fma_rn(m4, f1, f0), t2), add(__fma_rn(m2, f1, f0), f2));
+    const double s1 = ind(sub(f1, f3), add(__fma_rn(m2, f2, f1), f3));
+    const double s2 = ind(add(__fma_rn(m4, f3, f4), t2), add(__fma_rn(m2, f3, f4), f2));
+    const double t1 = mulk_fast<3>(f1), t3 = mulk_fast<3>(f3), f15 = mulk_fast<15>(f2);
+    const double m1 = mulc(0.65, s1);
+    double2 r;
+    {
+        const double pa = add(__fma_rn(m2, mulk_fast<5>(f1), mulk_fast<3>(f0)), f15);
+        const double pb = add(__fma_rn(p2, t2, -f1), t3), pc = sub(__fma_rn(p2, t3, t2), f4);
+        const double w0 = mulc(0.075, s0);
+        const double d = rcp_fast(add(add(w0, m1), mulc(0.275, s2)), bad);
+        const double a = mul(w0, d), b = mul(m1, d), c = sub(sub(one, a), b);
+        r.x = eighth(add(add(mul(a, pa), mul(b, pb)), mul(c, pc)));
+    }
+    {
+        const double qa = add(__fma_rn(m2, mulk_fast<5>(f3), mulk_fast<3>(f4)), f15);
+        const double qb = add(__fma_rn(p2, t2, -f3), t1), qc = sub(__fma_rn(p2, t1, t2), f0);
+        const double w0 = mulc(0.275, s0);
+        const double d = rcp_fast(add(add(w0, m1), mulc(0.075, s2)), bad);
+        const double a = mul(w0, d), b = mul(m1, d), c = sub(sub(one, a), b);
+        r.y = eighth(add(add(mul(c, qa), mul(b, qb)), mul(a, qc)));
+    }
+    if (bad) r = wcns4_pipe(f0, f1, f2, f3, f4);
+    return r;
+}
+
+
+// One thread's part of a block's shared scratch: 35 rows of NT doubles.
+template <int NT> struct RecScratch {
+    double (*w)[NT];
+    int t;
+    __device__ __forceinline__ double &operator()(int n, int m) const { return w[5 * n + m][t]; }
+};
+
+// reconst_full / reconst_alfven (point.cuh) with WCNS4.  Q(k, m): variable k
+// at stencil point m; full: the full system.
+template <int NT, class LOAD>
+__device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed gamma,
+                                                 const RecScratch<NT> &W, ed ul[7], ed ur[7])
+{
+    unsigned nz[7] = {0, 0, 0, 0, 0, 0, 0};
+    auto column = [&](int m, ed c[7]) {
+#pragma unroll
+        for (int k = 0; k < 7; k++) {
+            const double x = Q(k, m);
+            c[k] = x;
+            nz[k] |= (x64::hi32(x) << 1) | x64::lo32(x);
+        }
+    };
+    ed by, bz, icf2, isroh;
+    if (full) {
+        ed c[7];
+        column(2, c);
+        Eigen7<ed> E;
+        eigen_full<ed>(c[0], c[1], bn, c[4], c[5], c[6], gamma, E);
+#pragma unroll
+        for (int m = 0; m < 5; m++) {
+            ed wm[7];
+            column(m, c);
+            proj_full<ed>(E, c[0], c[1], c[2], c[3], c[4], c[5], c[6], wm);
+#pragma unroll
+            for (int n = 0; n < 7; n++) W(n, m) = wm[n].v;
+        }
+    } else {
+        ed c[7];
+        column(2, c);
+        by = c[4];
+        bz = c[5];
+        const ed ro = c[0], iro = trcp(ro);
+        const ed cs2 = gamma * c[6] * iro;
+        const ed ca2 = bn * bn * iro;
+        const ed ct2 = (by * by + bz * bz) * iro;
+        const ed cb2 = cs2 + ca2 + ct2;
+        const ed cf2 = ed(0.5) * (cb2 + tsqrt(tabs(cb2 * cb2 - ed(4.0) * cs2 * ca2)));
+        const ed sro = tsqrt(ro);
+        isroh = thalf_over(sro);
+        icf2 = trcp(cf2);
+#pragma unroll
+        for (int m = 0; m < 5; m++) {
+            column(m, c);
+            const ed r = c[0], b1 = c[4], b2 = c[5], p = c[6];
+            const ed y1 = by * b1, z2 = bz * b2;
+            W(0, m) = c[1].v;
+            W(1, m) = (cf2 * r - y1 - z2 - p).v;
+            W(2, m) = (y1 + z2 + p).v;
+            const ed sy = sro * c[2], sz = sro * c[3];
+            W(3, m) = (sy + b1).v;
+            W(4, m) = (sy - b1).v;
+            W(5, m) = (sz + b2).v;
+            W(6, m) = (sz - b2).v;
+        }
+    }
+#pragma unroll 1
+    for (int n = 0; n < 7; n++) {
+        const double2 v = wcns4_ed(W(n, 0), W(n, 1), W(n, 2), W(n, 3), W(n, 4));
+        W(n, 0) = v.x;
+        W(n, 1) = v.y;
+    }
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        ed w[7], *u = s ? ur : ul;
+#pragma unroll
+        for (int n = 0; n < 7; n++) w[n] = W(n, s);
+        if (full) {
+            Eigen7<ed> E;
+            eigen_full<ed>(Q(0, 2), Q(1, 2), bn, Q(4, 2), Q(5, 2), Q(6, 2), gamma, E);
+            back_full<ed>(E, w, u);
+        } else {
+            const ed h = 0.5, byh = h * by, bzh = h * bz;
+            u[0] = icf2 * w[1] + icf2 * w[2];
+            u[1] = w[0];
+            u[2] = isroh * w[3] + isroh * w[4];
+            u[3] = isroh * w[5] + isroh * w[6];
+            u[4] = h * w[3] - h * w[4];
+            u[5] = h * w[5] - h * w[6];
+            u[6] = w[2] - byh * w[3] + byh * w[4] - bzh * w[5] + bzh * w[6];
+        }
+#pragma unroll
+        for (int k = 1; k <= 5; k++)
+            if (nz[k] == 0) u[k] = 0.0;
+    }
+}
+
+}  // namespace mlau

@@ -48,6 +48,12 @@ extern "C" long exact64_check(int kind, int ulps, long n, long seed)
         bad += !same(x64::div(a, b), a / b);
         bad += !same(x64::div24(a), a / 24.0);
         bad += !same(x64::sqrt(a), std::sqrt(a));
+        if (!x64::off_range(x64::hi32(a))) {
+            bad += !same(x64::sqr_fast(a), a * a);
+            bad += !same(x64::mulk_fast<3>(a), 3.0 * a) + !same(x64::mulk_fast<5>(a), 5.0 * a) +
+                   !same(x64::mulk_fast<15>(a), 15.0 * a);
+            if (!x64::off_range(x64::hi32(b))) bad += !same(x64::mul_fast(a, b), a * b);
+        }
         bad += !same(x64::sqrt(std::fabs(a)), std::sqrt(std::fabs(a)));
     }
     return bad;
