@@ -89,4 +89,107 @@ template <> MLAU_HD ed tsqrt_half<ed>() { return 0x1.6a09e667f3bcdp-1; }
 template <> MLAU_HD ed tdiv24<ed>(ed x) { return x64::div24(x.v); }
 
 
+// a * b on the integer pipe.
+static __device__ __noinline__ double mul_pipe(double a, double b) { return a * b; }
+__device__ __forceinline__ ed imul(ed a, ed b)
+{
+    uint32_t bad = x64::off_wide(a.v) | x64::off_wide(b.v);
+    double r = x64::mul(a.v, b.v, bad);
+    if (bad) r = mul_pipe(a.v, b.v);
+    return r;
+}
+// a / 2: exact for normal results
+__device__ __forceinline__ ed ihalf(ed a)
+{
+    double r = x64::scale<-1>(a.v);
+    if (x64::off_wide(a.v)) r = mul_pipe(a.v, 0.5);
+    return r;
+}
+
+template <> MLAU_HD ed thalf<ed>(ed x)
+{
+#ifdef __CUDA_ARCH__
+    return ihalf(x);
+#else
+    return x.v * 0.5;
+#endif
+}
+template <> MLAU_HD bool tzero<ed>(ed x) { return ((x64::hi32(x.v) << 1) | x64::lo32(x.v)) == 0; }
+
+// Comparisons (81 cycles each on the FP64 pipe) on the values' bits.  An
+// infinity or NaN among the operands takes the pipe's.
+MLAU_HD bool ed_special(uint32_t h, uint32_t g)
+{
+    const uint32_t a = h << 1, b = g << 1;
+    return (a > b ? a : b) >= 0xffe00000u;
+}
+static X64_SLOW bool ge_pipe(double a, double b) { return a >= b; }
+MLAU_HD bool ed_ge(ed a, ed b)
+{
+    const uint32_t ha = x64::hi32(a.v), hb = x64::hi32(b.v);
+    const int32_t sa = (int32_t)ha >> 31, sb = (int32_t)hb >> 31;
+    const int32_t ka = (int32_t)ha ^ (sa & 0x7fffffff), kb = (int32_t)hb ^ (sb & 0x7fffffff);
+    bool r = ka > kb || (ka == kb && (x64::lo32(a.v) ^ (uint32_t)sa) >= (x64::lo32(b.v) ^ (uint32_t)sb));
+    if (ed_special(ha, hb)) r = ge_pipe(a.v, b.v);
+    return r;
+}
+template <> MLAU_HD ed vmax<ed>(ed a, ed b) { return ed_ge(a, b) ? a : b; }
+template <> MLAU_HD ed vmin<ed>(ed a, ed b) { return ed_ge(a, b) ? b : a; }
+
+static X64_SLOW double minmod_pipe(double a, double b) { return minmod<double>(a, b); }
+static X64_SLOW double minmod3_pipe(double a, double b, double c) { return minmod3<double>(a, b, c); }
+// the operand of smaller magnitude where the signs agree, else 0
+template <> MLAU_HD ed minmod<ed>(ed a, ed b)
+{
+    const uint32_t ha = x64::hi32(a.v), hb = x64::hi32(b.v);
+    const uint32_t ma = ha & 0x7fffffffu, mb = hb & 0x7fffffffu;
+    double r = (ma < mb || (ma == mb && x64::lo32(a.v) < x64::lo32(b.v))) ? a.v : b.v;
+    if ((ha ^ hb) >> 31) r = 0.0;
+    if (ed_special(ha, hb)) r = minmod_pipe(a.v, b.v);
+    return r;
+}
+template <> MLAU_HD ed minmod3<ed>(ed a, ed b, ed c)
+{
+    const uint32_t hc = x64::hi32(c.v);
+    double r = minmod(minmod(a, b), c).v;
+    if (ed_special(x64::hi32(a.v), x64::hi32(b.v)) || ed_special(hc, hc)) r = minmod3_pipe(a.v, b.v, c.v);
+    return r;
+}
+
+// The 4th-order linear face value 1/320 (9 f0 - 56 f1 + 234 f2 + 144 f3 - 11 f4)
+// of lin_l, products on the integer pipe (56 = 8 x 7, 234 = 2 x 117 and 144 =
+// 16 x 9: the powers of two ride on the sums), the four sums on the FP64 pipe.
+static __device__ __noinline__ double lin4_pipe(double f0, double f1, double f2, double f3, double f4)
+{
+    return lin_l<double>(4, f0, f1, f2, f3, f4);
+}
+__device__ __forceinline__ ed lin4_ed(double f0, double f1, double f2, double f3, double f4)
+{
+    using namespace x64;
+    const uint32_t z = opaque_zero();
+    auto K = [&](uint32_t h) { return __hiloint2double((int)(h + z), 0); };
+    uint32_t bad = off_wide(f0) | off_wide(f1) | off_wide(f2) | off_wide(f3) | off_wide(f4);
+    double s = __fma_rn(K(0xc0200000u), mulk<7>(f1), mulk<9>(f0));  // -8
+    s = __fma_rn(K(0x40000000u), mulk<117>(f2), s);                 // 2
+    s = __fma_rn(K(0x40300000u), mulk<9>(f3), s);                   // 16
+    s = __fma_rn(-mulk<11>(f4), K(0x3ff00000u), s);
+    double r = mul(s, 0.003125, bad);
+    if (bad) r = lin4_pipe(f0, f1, f2, f3, f4);
+    return r;
+}
+template <> MLAU_HD ed lin_l<ed>(int odr, ed f0, ed f1, ed f2, ed f3, ed f4)
+{
+#ifdef __CUDA_ARCH__
+    odr = lin_odr(odr);
+    if (odr == 4) return lin4_ed(f0.v, f1.v, f2.v, f3.v, f4.v);
+    if (odr == 2) return ed(0.25) * (-f1 + ed(4.0) * f2 + f3);
+    if (odr == 3) return ed(0.125) * (-f1 + ed(6.0) * f2 + ed(3.0) * f3);
+#endif
+    return f2;
+}
+template <> MLAU_HD ed lin_r<ed>(int odr, ed f0, ed f1, ed f2, ed f3, ed f4)
+{
+    return lin_l<ed>(odr, f4, f3, f2, f1, f0);
+}
+
 }  // namespace mlau

@@ -145,8 +145,27 @@ X64 uint32_t off_range(uint32_t h, uint32_t g)
     return ((h + 0x50000000u) | (g + 0x50000000u)) & 0x60000000u;
 }
 
+// Operands of the products below: zero, or exponent field 512..1535 (off_wide
+// is zero exactly for these).  Sums and products of such values that pass
+// through a computation stay normal as long as every product's result passes
+// too (its field cannot wrap around into the range), so a computation checks
+// its inputs once and its products by their results.
+X64 uint32_t off_field(uint32_t h) { return (h + 0x60000000u) & 0x40000000u; }
+X64 uint32_t off_wide(double x)
+{
+    const uint32_t h = hi32(x);
+    return ((h << 1) | lo32(x)) == 0 ? 0u : off_field(h);
+}
+
+// Significand's upper word, without the implicit bit for a zero.
+X64 uint32_t sig_hi(uint32_t h)
+{
+    const uint32_t e = h & 0x7ff00000u;
+    return (h & 0xfffffu) | (e < 0x100000u ? e : 0x100000u);
+}
+
 // Round (h:l | m as a fraction of 2^32 below l) to nearest even and add the
-// exponent and sign word e: the packed double.
+// sign and exponent word e.
 X64 double round_pack(uint32_t h, uint32_t l, uint32_t m, uint32_t e)
 {
 #ifdef __CUDA_ARCH__
@@ -162,20 +181,27 @@ X64 double round_pack(uint32_t h, uint32_t l, uint32_t m, uint32_t e)
 #endif
 }
 
-// 106-bit product w3:w2:w1:w0 of two 53-bit significands -> rounded double.
-// sg: sign and exponent word of the product before normalisation.
-X64 double norm_product(uint64_t p11, uint32_t w1, uint32_t w0, uint32_t sg)
+// 106-bit product of two 53-bit significands (upper half p11, then w1, w0) ->
+// rounded double; sg: the sum of the operands' sign and exponent words.
+X64 double norm_round(uint64_t p11, uint32_t w1, uint32_t w0, uint32_t sg)
 {
     const uint32_t w3 = (uint32_t)(p11 >> 32), w2 = (uint32_t)p11;
     const uint32_t s = 12u - (w3 >> 9);
     const uint32_t h = shfl_(w2, w3, (int)s), l = shfl_(w1, w2, (int)s);
     const uint32_t m = shfl_(w0, w1, (int)s) | (w0 < 1u ? w0 : 1u);
-    return round_pack(h, l, m, sg - (s << 20));
+    return round_pack(h, l, m, sg - ((1012u + s) << 20));
+}
+X64 double norm_product(uint64_t p11, uint32_t w1, uint32_t w0, uint32_t sg, uint32_t &bad)
+{
+    const double r = norm_round(p11, w1, w0, sg);
+    const uint32_t rh = hi32(r);
+    const bool zero = (uint32_t)(p11 >> 32) == 0;
+    bad |= zero ? 0u : off_field(rh);
+    return make(zero ? sg & 0x80000000u : rh, lo32(r));
 }
 
-// Product, square and small odd multiple of doubles in range (see off_range;
-// the caller checks).
-X64 double mul_fast(double a, double b)
+// a * b and a * a of operands in 2^-255 .. 2^256, zero excluded
+X64 double mul_nz(double a, double b, uint32_t &bad)
 {
     const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
     const uint32_t ma = (ah & 0xfffffu) | 0x100000u, mb = (bh & 0xfffffu) | 0x100000u;
@@ -183,39 +209,62 @@ X64 double mul_fast(double a, double b)
     const uint64_t p01 = wide(al, mb) + (p00 >> 32);
     const uint64_t p10 = wide(ma, bl) + (uint32_t)p01;
     const uint64_t p11 = wide(ma, mb) + (p01 >> 32) + (p10 >> 32);
-    const uint32_t sg = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) + ((ah ^ bh) & 0x80000000u) -
-                        (1012u << 20);
-    return norm_product(p11, (uint32_t)p10, (uint32_t)p00, sg);
+    bad |= off_range(ah, bh);
+    return norm_round(p11, (uint32_t)p10, (uint32_t)p00, (ah & 0xfff00000u) + (bh & 0xfff00000u));
 }
-
-X64 double sqr_fast(double a)
+X64 double sqr_nz(double a, uint32_t &bad)
 {
-    const uint32_t ah = hi32(a), al = lo32(a);
-    const uint32_t ma = (ah & 0xfffffu) | 0x100000u;
+    const uint32_t ah = hi32(a), al = lo32(a), ma = (ah & 0xfffffu) | 0x100000u;
     const uint64_t p00 = wide(al, al);
     const uint64_t p01 = wide(al, 2u * ma) + (p00 >> 32);
     const uint64_t p11 = wide(ma, ma) + (p01 >> 32);
-    const uint32_t sg = ((ah & 0x7ff00000u) << 1) - (1012u << 20);
-    return norm_product(p11, (uint32_t)p01, (uint32_t)p00, sg);
+    bad |= off_range(ah);
+    return norm_round(p11, (uint32_t)p01, (uint32_t)p00, (ah & 0x7ff00000u) << 1);
+}
+
+X64 double mul(double a, double b, uint32_t &bad)
+{
+    const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
+    const uint32_t ma = sig_hi(ah), mb = sig_hi(bh);
+    const uint64_t p00 = wide(al, bl);
+    const uint64_t p01 = wide(al, mb) + (p00 >> 32);
+    const uint64_t p10 = wide(ma, bl) + (uint32_t)p01;
+    const uint64_t p11 = wide(ma, mb) + (p01 >> 32) + (p10 >> 32);
+    return norm_product(p11, (uint32_t)p10, (uint32_t)p00, (ah & 0xfff00000u) + (bh & 0xfff00000u), bad);
+}
+
+X64 double sqr(double a, uint32_t &bad)
+{
+    const uint32_t ah = hi32(a), al = lo32(a), ma = sig_hi(ah);
+    const uint64_t p00 = wide(al, al);
+    const uint64_t p01 = wide(al, 2u * ma) + (p00 >> 32);
+    const uint64_t p11 = wide(ma, ma) + (p01 >> 32);
+    return norm_product(p11, (uint32_t)p01, (uint32_t)p00, (ah & 0x7ff00000u) << 1, bad);
 }
 
 // k * a for an odd integer k in [3, 255]
-template <int K> X64 double mulk_fast(double a)
+template <int K> X64 double mulk(double a)
 {
     constexpr int B = K < 4 ? 2 : K < 8 ? 3 : K < 16 ? 4 : K < 32 ? 5 : K < 64 ? 6 : K < 128 ? 7 : 8;
     // K << (11 - B) brings the 53-bit significand's product to bit 63 or 62
     constexpr uint32_t KS = (uint32_t)K << (11 - B);
-    const uint32_t ah = hi32(a), al = lo32(a);
-    const uint32_t ma = (ah & 0xfffffu) | 0x100000u;
+    const uint32_t ah = hi32(a), al = lo32(a), ma = sig_hi(ah);
     const uint64_t p0 = wide(al, KS);
     const uint32_t xl = (uint32_t)p0, xh = ma * KS + (uint32_t)(p0 >> 32);
     // significand = X >> (11 - s), s = 1 where bit 63 is clear
     const uint32_t t = 10u + (xh >> 31);
     const uint32_t h = xh >> t, l = shfr_(xl, xh, (int)t), f = xl << (32u - t);
     const uint32_t e = (ah & 0xfff00000u) + (t << 20) + ((uint32_t)(B - 12) << 20);
-    return round_pack(h, l, f, e);
+    const double r = round_pack(h, l, f, e);
+    return make(xh == 0 ? ah : hi32(r), lo32(r));
 }
 
+// a * 2^P, exact
+template <int P> X64 double scale(double a)
+{
+    const uint32_t h = hi32(a);
+    return make((h & 0x7ff00000u) ? h + ((uint32_t)P << 20) : h, lo32(a));
+}
 
 // Reciprocal seed of the 53-bit significand (mh:ml) in [2^52, 2^53): Y0 in
 // [2^23, 2^24) with Y0 ~ 2^76 / B, and e1 = (B Y0 - 2^76) >> 24.
@@ -297,7 +346,7 @@ X64 double div24(double x)
     return q;
 }
 
-X64 double div(double a, double b)
+X64 double div_fast(double a, double b, uint32_t &bad)
 {
     const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), ml = lo32(b);
     const uint32_t na = (ah & 0xfffffu) | 0x100000u, mh = (bh & 0xfffffu) | 0x100000u;
@@ -328,13 +377,19 @@ X64 double div(double a, double b)
     const uint64_t Qr = Q + (t > B ? 1u : 0u) - (t < -B ? 1u : 0u);
     const uint32_t e = (ah & 0x7ff00000u) - (bh & 0x7ff00000u) + ((lt ? 1021u : 1022u) << 20) +
                        ((ah ^ bh) & 0x80000000u);
-    const bool ok = off_range(ah, bh) == 0;
-    double q = make((uint32_t)(Qr >> 32) + e, (uint32_t)Qr);
-    if (!ok) q = div_hw(a, b);
+    bad |= off_range(ah, bh);
+    return make((uint32_t)(Qr >> 32) + e, (uint32_t)Qr);
+}
+
+X64 double div(double a, double b)
+{
+    uint32_t bad = 0;
+    double q = div_fast(a, b, bad);
+    if (bad) q = div_hw(a, b);
     return q;
 }
 
-X64 double sqrt(double x)
+X64 double sqrt_fast(double x, uint32_t &bad)
 {
     const uint32_t ah = hi32(x), al = lo32(x);
     // x = X 2^(2k - 52), X = B or 2 B in [2^52, 2^54)
@@ -365,9 +420,15 @@ X64 double sqrt(double x)
     const uint64_t S = S2 + (uint64_t)(int64_t)(T >> 20);
     const uint32_t e = (((ah + 0x100000u) >> 1) & 0x7ff00000u) + (510u << 20);
     // positive, mid-range and not near a midpoint
-    const bool ok = (ah + 0x50000000u) >> 29 == 4u && (((uint32_t)T + 64u) & 0xfffffu) > 128u;
-    double q = make((uint32_t)(S >> 32) + e, (uint32_t)S);
-    if (!ok) q = sqrt_hw(x);
+    bad |= (ah + 0x50000000u) >> 29 == 4u && (((uint32_t)T + 64u) & 0xfffffu) > 128u ? 0u : 1u;
+    return make((uint32_t)(S >> 32) + e, (uint32_t)S);
+}
+
+X64 double sqrt(double x)
+{
+    uint32_t bad = 0;
+    double q = sqrt_fast(x, bad);
+    if (bad) q = sqrt_hw(x);
     return q;
 }
 

@@ -9,6 +9,7 @@
 
 #include "stencil.cuh"
 #include "rec_exact.cuh"
+#include "flux_exact.cuh"
 
 namespace mlau {
 namespace {
@@ -86,7 +87,7 @@ __device__ __forceinline__ void rec_central2(const PlainFields &f, const View2 &
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
-        a5[m] = ed(bt[s]) * v.vn[s];
+        a5[m] = imul(bt[s], v.vn[s]);
         t5[m] = vt[s];
     }
     f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
@@ -125,7 +126,7 @@ k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, do
 }
 
 // WCNS4 with the drivers' eigen-systems.
-__global__ void __launch_bounds__(TPB, 4)
+__global__ void __launch_bounds__(TPB, 5)
 k_rec2_wcns4(PlainFields f, View2 v, Dims d, Box b, long long st, double gamma)
 {
     __shared__ double w[35][TPB];
@@ -135,13 +136,8 @@ k_rec2_wcns4(PlainFields f, View2 v, Dims d, Box b, long long st, double gamma)
     const double *src[7] = {f.s[0], v.vn, v.vt, v.vu, v.ct, v.cu, f.pr};
     auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
     const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
-    ed ul[7], ur[7];
-    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, ul, ur);
-#pragma unroll
-    for (int n = 0; n < 7; n++) {
-        f.ul[n][c + st] = ul[n].v;
-        f.ur[n][c] = ur[n].v;
-    }
+    auto PUT = [&](int s, int n, double u) { (s ? f.ur : f.ul)[n][s ? c : c + st] = u; };
+    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, PUT);
     rec_central2(f, v, c, st, 4);
 }
 
@@ -164,6 +160,28 @@ k_flux2(PlainFields f, View2 v, Dims d, Box b, long long st, int D, int which, d
     F[4 + v.split_u] -= fc;
 #pragma unroll
     for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n].v;
+    f.FC[D][0][c] = fc.v;
+}
+
+// MLAU, LHLLD and HLLD faces on both pipes (flux_exact.cuh).
+template <int WHICH>
+__global__ void __launch_bounds__(FXT, 2)
+k_flux2_ed(PlainFields f, View2 v, Dims d, Box b, long long st, int D, double gamma)
+{
+    extern __shared__ double fx_rows[];
+    int i, j, k;
+    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    const long long c = d.at(i, j, 0);
+    auto IN = [&](int s, int n) { return (s ? f.ur : f.ul)[n][c]; };
+    const double dv[2] = {v.dvt[c - st], v.dvt[c]};
+    const double bn = (ed(0.5) * (ed(v.bface[c]) + v.bface[c])).v;
+    double F[7];
+    riemann_ed<WHICH, 2>(IN, (double (*)[FXT])fx_rows, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]).v, dv, F);
+    const ed fc = ihalf(ed(f.ql[0][c]) + f.qr[0][c]);
+    if (v.split_u) F[5] = (F[5] - fc).v;
+    else F[4] = (F[4] - fc).v;
+#pragma unroll
+    for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n];
     f.FC[D][0][c] = fc.v;
 }
 
@@ -290,7 +308,10 @@ int plain2d_alloc(Sim *s)
         for (int v = 0; v < 7; v++) rc |= dalloc(s, &f.F[D][v], n);
         rc |= dalloc(s, &f.FC[D][0], n);
     }
-    return rc ? MLAU_ERR_NOMEM : MLAU_OK;
+    if (rc) return MLAU_ERR_NOMEM;
+    MLAU_CUDA(cudaFuncSetAttribute(k_flux2_ed<FLUX_MLAU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)fx_smem<FLUX_MLAU>()));
+    return MLAU_OK;
 }
 
 int plain2d_step(Sim *s, double dt)
@@ -336,8 +357,19 @@ int plain2d_step(Sim *s, double dt)
             }
             {
                 TimedLaunch tl(&s->timer, KK_FLUX);
-                k_flux2<<<blocks_for(fb.count(), TPB), TPB, 0, st>>>(f, v, d, fb, stride, D,
-                                                                     s->flux, s->gamma);
+                const unsigned nb = blocks_for(fb.count(), FXT);
+                if (s->flux == FLUX_MLAU)
+                    k_flux2_ed<FLUX_MLAU><<<nb, FXT, fx_smem<FLUX_MLAU>(), st>>>(f, v, d, fb, stride, D,
+                                                                                 s->gamma);
+                else if (s->flux == FLUX_LHLLD)
+                    k_flux2_ed<FLUX_LHLLD><<<nb, FXT, fx_smem<FLUX_LHLLD>(), st>>>(f, v, d, fb, stride,
+                                                                                   D, s->gamma);
+                else if (s->flux == FLUX_HLLD)
+                    k_flux2_ed<FLUX_HLLD><<<nb, FXT, fx_smem<FLUX_HLLD>(), st>>>(f, v, d, fb, stride, D,
+                                                                                 s->gamma);
+                else
+                    k_flux2<<<blocks_for(fb.count(), TPB), TPB, 0, st>>>(f, v, d, fb, stride, D, s->flux,
+                                                                         s->gamma);
             }
         }
         {

@@ -28,6 +28,7 @@
 #include "point.cuh"
 #include "stencil.cuh"
 #include "rec_exact.cuh"
+#include "flux_exact.cuh"
 
 namespace mlau {
 namespace {
@@ -120,7 +121,7 @@ __device__ __forceinline__ void rec_central(const PlainFields &f, const SweepVie
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
-        a5[m] = ed(v.ct[s]) * v.vn[s];
+        a5[m] = imul(v.ct[s], v.vn[s]);
         t5[m] = v.vt[s];
     }
     f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
@@ -130,7 +131,7 @@ __device__ __forceinline__ void rec_central(const PlainFields &f, const SweepVie
 #pragma unroll
     for (int m = 0; m < 5; m++) {
         const long long s = c + st * (m - 2);
-        a5[m] = ed(v.cu[s]) * v.vn[s];
+        a5[m] = imul(v.cu[s], v.vn[s]);
         u5[m] = v.vu[s];
     }
     f.ql[1][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
@@ -169,7 +170,7 @@ k_rec3(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, int eig
 }
 
 // WCNS4 with the drivers' eigen-systems.
-__global__ void __launch_bounds__(TPB, 4)
+__global__ void __launch_bounds__(TPB, 5)
 k_rec3_wcns4(PlainFields f, SweepView v, Dims d, Box b, long long st, double gamma)
 {
     __shared__ double w[35][TPB];
@@ -179,13 +180,8 @@ k_rec3_wcns4(PlainFields f, SweepView v, Dims d, Box b, long long st, double gam
     const double *src[7] = {f.s[0], v.vn, v.vt, v.vu, v.ct, v.cu, f.pr};
     auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
     const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
-    ed ul[7], ur[7];
-    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, ul, ur);
-#pragma unroll
-    for (int n = 0; n < 7; n++) {
-        f.ul[n][c + st] = ul[n].v;
-        f.ur[n][c] = ur[n].v;
-    }
+    auto PUT = [&](int s, int n, double u) { (s ? f.ur : f.ul)[n][s ? c : c + st] = u; };
+    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, PUT);
     rec_central(f, v, c, st, 4);
 }
 
@@ -210,6 +206,30 @@ k_flux3(PlainFields f, SweepView v, Dims d, Box b, long long st, int D, int whic
     F[5] -= fcu;
 #pragma unroll
     for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n].v;
+    f.FC[D][0][c] = fct.v;
+    f.FC[D][1][c] = fcu.v;
+}
+
+// MLAU, LHLLD and HLLD faces on both pipes (flux_exact.cuh).
+template <int WHICH>
+__global__ void __launch_bounds__(FXT, 2)
+k_flux3_ed(PlainFields f, SweepView v, Dims d, Box b, long long st, int D, double gamma)
+{
+    extern __shared__ double fx_rows[];
+    int i, j, k;
+    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    const long long c = d.at(i, j, k);
+    auto IN = [&](int s, int n) { return (s ? f.ur : f.ul)[n][c]; };
+    const double dv[4] = {v.dvt[c - st], v.dvt[c], v.dvu[c - st], v.dvu[c]};
+    const double bn = (ed(0.5) * (ed(v.bface[c]) + v.bface[c])).v;
+    double F[7];
+    riemann_ed<WHICH, 4>(IN, (double (*)[FXT])fx_rows, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]).v, dv, F);
+    const ed fct = ihalf(ed(f.ql[0][c]) + f.qr[0][c]);
+    const ed fcu = ihalf(ed(f.ql[1][c]) + f.qr[1][c]);
+    F[4] = (F[4] - fct).v;
+    F[5] = (F[5] - fcu).v;
+#pragma unroll
+    for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n];
     f.FC[D][0][c] = fct.v;
     f.FC[D][1][c] = fcu.v;
 }
@@ -377,7 +397,10 @@ int plain3d_alloc(Sim *s)
         for (int v = 0; v < 7; v++) rc |= dalloc(s, &f.F[D][v], n);
         rc |= dalloc(s, &f.FC[D][0], n) | dalloc(s, &f.FC[D][1], n);
     }
-    return rc ? MLAU_ERR_NOMEM : MLAU_OK;
+    if (rc) return MLAU_ERR_NOMEM;
+    MLAU_CUDA(cudaFuncSetAttribute(k_flux3_ed<FLUX_MLAU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)fx_smem<FLUX_MLAU>()));
+    return MLAU_OK;
 }
 
 // Ghost fill of the FP64 state with the simulation's 3D tables (also the
@@ -440,8 +463,19 @@ int plain3d_step(Sim *s, double dt)
             }
             {
                 TimedLaunch tl(&s->timer, KK_FLUX);
-                k_flux3<<<blocks_for(fb.count(), TPB), TPB, 0, st>>>(f, v, d, fb, strides[D], D,
-                                                                     s->flux, s->gamma);
+                const unsigned nb = blocks_for(fb.count(), FXT);
+                if (s->flux == FLUX_MLAU)
+                    k_flux3_ed<FLUX_MLAU><<<nb, FXT, fx_smem<FLUX_MLAU>(), st>>>(f, v, d, fb, strides[D],
+                                                                                 D, s->gamma);
+                else if (s->flux == FLUX_LHLLD)
+                    k_flux3_ed<FLUX_LHLLD><<<nb, FXT, fx_smem<FLUX_LHLLD>(), st>>>(
+                        f, v, d, fb, strides[D], D, s->gamma);
+                else if (s->flux == FLUX_HLLD)
+                    k_flux3_ed<FLUX_HLLD><<<nb, FXT, fx_smem<FLUX_HLLD>(), st>>>(f, v, d, fb, strides[D],
+                                                                                 D, s->gamma);
+                else
+                    k_flux3<<<blocks_for(fb.count(), TPB), TPB, 0, st>>>(f, v, d, fb, strides[D], D,
+                                                                         s->flux, s->gamma);
             }
         }
         {

@@ -42,6 +42,9 @@ template <class T> MLAU_HD T tdiv24(T x) { return x / T(24.0); }
 template <class T> MLAU_HD T tsqrt_two() { return tsqrt(T(2.0)); }
 template <class T> MLAU_HD T tsqrt_half() { return tsqrt(T(0.5)); }
 
+template <class T> MLAU_HD T thalf(T x) { return T(0.5) * x; }
+template <class T> MLAU_HD bool tzero(T x) { return x == T(0); }
+
 // Epsilon of the WCNS nonlinear weights (interp.h:154,194).  In FP32 the
 // reference's 1e-40 is a denormal that flush-to-zero removes, so FP32 uses a
 // normal number far below any weight that matters.
@@ -63,7 +66,7 @@ template <class T> MLAU_HD T minmod(T a, T b)
 // interp.h:30-37
 template <class T> MLAU_HD void muscl_mm_lr(T f1, T f2, T f3, T &fl, T &fr)
 {
-    T df = T(0.5) * minmod(f2 - f1, f3 - f2);
+    T df = thalf(minmod(f2 - f1, f3 - f2));
     fl = f2 + df;
     fr = f2 - df;
 }
@@ -79,7 +82,7 @@ template <class T> MLAU_HD T minmod3(T a, T b, T c)
 template <class T> MLAU_HD void muscl_mc_lr(T f1, T f2, T f3, T &fl, T &fr)
 {
     const T alpha = T(2.0);
-    T df = T(0.5) * minmod(alpha * minmod(f2 - f1, f3 - f2), T(0.5) * (f3 - f1));
+    T df = thalf(minmod(alpha * minmod(f2 - f1, f3 - f2), thalf(f3 - f1)));
     fl = f2 + df;
     fr = f2 - df;
 }
@@ -89,8 +92,8 @@ template <class T> MLAU_HD void muscl_kr_lr(T f1, T f2, T f3, T &fl, T &fr)
 {
     const T d1 = T(2.0) * (f2 - f1);
     const T d2 = T(2.0) * (f3 - f2);
-    const T dl = T(0.5) * minmod3(d1, d2, (T(0.5) * d1 + d2) / T(3.0));
-    const T dr = T(0.5) * minmod3(d1, d2, (d1 + T(0.5) * d2) / T(3.0));
+    const T dl = thalf(minmod3(d1, d2, (thalf(d1) + d2) / T(3.0)));
+    const T dr = thalf(minmod3(d1, d2, (d1 + thalf(d2)) / T(3.0)));
     fl = f2 + dl;
     fr = f2 - dr;
 }
@@ -276,8 +279,7 @@ MLAU_HD void zero_guard(const T q[7][5], T ul[7], T ur[7])
 {
 #pragma unroll
     for (int k = 1; k <= 5; k++) {
-        bool z = (q[k][0] == T(0)) && (q[k][1] == T(0)) && (q[k][2] == T(0)) &&
-                 (q[k][3] == T(0)) && (q[k][4] == T(0));
+        bool z = tzero(q[k][0]) && tzero(q[k][1]) && tzero(q[k][2]) && tzero(q[k][3]) && tzero(q[k][4]);
         if (z) { ul[k] = T(0); ur[k] = T(0); }
     }
 }

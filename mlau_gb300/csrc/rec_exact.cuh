@@ -3,18 +3,22 @@
 // for bit, with the work split between the FP64 pipe and the integer pipes.
 //
 // What bounds it: the FP64 pipe, 64 cycles per warp instruction and
-// sub-partition.  Of the 92 products and 41 sums of one field's wcns4_lr, the
-// sums stay on that pipe, those by 2 and 4 fused into them (exact scalings);
-// the other products and the five reciprocals run as integer instructions
-// (exact64.cuh: 51 / 45 / 24 / 75 cycles for a b, a a, k a, 1 / x), in the
-// issue slots the FP64 pipe leaves idle.  The seven fields go through one loop
-// over a shared-memory scratch, since unrolled the code would overflow the
-// instruction cache.  One flag collects the operands outside the integer path's
-// range and the undecided reciprocals; such a lane evaluates the field on the
-// FP64 pipe alone.  Five equal values (a uniform region) take constants.
+// sub-partition.  Of the 92 products and 41 sums of one field's wcns4_lr the
+// sums stay on that pipe, those with a product by 2, 4 or 0.25 as one operation
+// (exact scalings); the other products and the five reciprocals run as integer
+// instructions (exact64.cuh: 51 / 45 / 24 / 75 cycles for a b, a a, k a, 1 / x),
+// in the issue slots the FP64 pipe leaves idle, and so do the products of the
+// projections.  The seven fields, the three smoothness indicators and the two
+// sides go through loops over a shared-memory scratch and rotating registers:
+// unrolled, the code outgrows the instruction caches.  One flag collects the
+// operands outside the integer path's range and the undecided reciprocals; such
+// a lane evaluates the field on the FP64 pipe alone.  Five equal values (a
+// uniform region) take constants.
 //
-// Reconstruction of a 3D 128^3 MLAU step: 34.0 -> 20.5 ms (FP64 pipe 91 %
-// busy, issue slots 31 %); 2D 512^2 pass 4.31 -> 2.87 ms.
+// Reconstruction of a 3D 128^3 MLAU step: 34.0 ms on the FP64 pipe alone, 20.5
+// with the WCNS4 products moved, 18.0 as it stands (FP64 pipe 82 % busy, issue
+// slots 50 %, about what instruction supply allows without reuse); four, five
+// or six blocks per SM measured 18.1 / 18.0 / 17.9 ms.
 #pragma once
 
 #include "ed.cuh"
@@ -63,52 +67,52 @@ __device__ __forceinline__ double2 wcns4_ed(double f0, double f1, double f2, dou
          ((lo32(f0) ^ l2) | (lo32(f1) ^ l2)) | ((lo32(f3) ^ l2) | (lo32(f4) ^ l2))) == 0)
         return (h2 << 1 | l2) == 0 ? make_double2(0.0, 0.0) : wcns4_const(f2);
     const ConstReg K;
-    uint32_t bad = off_range(hi32(f0), hi32(f1)) | off_range(h2, hi32(f3)) | off_range(hi32(f4));
+    uint32_t bad = off_wide(f0) | off_wide(f1) | off_wide(f2) | off_wide(f3) | off_wide(f4);
     const double one = K(1.0), m4 = K(-4.0), m2 = K(-2.0), p2 = K(2.0), q4 = K(0.25), eps = K(1e-40);
     auto add = [&](double a, double b) { return __fma_rn(a, one, b); };
     auto sub = [&](double a, double b) { return __fma_rn(-b, one, a); };
-    auto mul = [&](double a, double b) {
-        bad |= off_range(hi32(a), hi32(b));
-        return mul_fast(a, b);
-    };
-    auto mulc = [&](double c, double b) {
-        bad |= off_range(hi32(b));
-        return mul_fast(c, b);
-    };
-    auto sqr = [&](double a) {
-        bad |= off_range(hi32(a));
-        return sqr_fast(a);
-    };
-    auto eighth = [&](double v) {
-        bad |= off_range(hi32(v));
-        return make(hi32(v) - (3u << 20), lo32(v));
-    };
-    const double t2 = mulk_fast<3>(f2);
-    auto ind = [&](double p, double q) {
-        const double s = __fma_rn(q4, sqr(p), mul(mulc(13. / 12., q), q));
-        return rcp_fast(add(sqr(s), eps), bad);
-    };
-    const double s0 = ind(add(__fma_rn(m4, f1, f0), t2), add(__fma_rn(m2, f1, f0), f2));
-    const double s1 = ind(sub(f1, f3), add(__fma_rn(m2, f2, f1), f3));
-    const double s2 = ind(add(__fma_rn(m4, f3, f4), t2), add(__fma_rn(m2, f3, f4), f2));
-    const double t1 = mulk_fast<3>(f1), t3 = mulk_fast<3>(f3), f15 = mulk_fast<15>(f2);
-    const double m1 = mulc(0.65, s1);
-    double2 r;
-    {
-        const double pa = add(__fma_rn(m2, mulk_fast<5>(f1), mulk_fast<3>(f0)), f15);
-        const double pb = add(__fma_rn(p2, t2, -f1), t3), pc = sub(__fma_rn(p2, t3, t2), f4);
-        const double w0 = mulc(0.075, s0);
-        const double d = rcp_fast(add(add(w0, m1), mulc(0.275, s2)), bad);
-        const double a = mul(w0, d), b = mul(m1, d), c = sub(sub(one, a), b);
-        r.x = eighth(add(add(mul(a, pa), mul(b, pb)), mul(c, pc)));
+    auto times = [&](double a, double b) { return mul_nz(a, b, bad); };
+    const double t0 = mulk<3>(f0), t1 = mulk<3>(f1), t2 = mulk<3>(f2), t3 = mulk<3>(f3), t4 = mulk<3>(f4);
+    const double f15 = mulk<15>(f2);
+    // the three smoothness indicators, then their inverse squares
+    double p = add(__fma_rn(m4, f1, f0), t2), q = add(__fma_rn(m2, f1, f0), f2);
+    double p1 = sub(f1, f3), q1 = add(__fma_rn(m2, f2, f1), f3);
+    double p2_ = add(__fma_rn(m4, f3, f4), t2), q2 = add(__fma_rn(m2, f3, f4), f2);
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+#pragma unroll 1
+    for (int n = 0; n < 3; n++) {
+        const double s = __fma_rn(q4, sqr_nz(p, bad), times(times(13. / 12., q), q));
+        const double g = rcp_fast(add(sqr_nz(s, bad), eps), bad);
+        s0 = s1;
+        s1 = s2;
+        s2 = g;
+        p = p1;
+        q = q1;
+        p1 = p2_;
+        q1 = q2;
     }
-    {
-        const double qa = add(__fma_rn(m2, mulk_fast<5>(f3), mulk_fast<3>(f4)), f15);
-        const double qb = add(__fma_rn(p2, t2, -f3), t1), qc = sub(__fma_rn(p2, t1, t2), f0);
-        const double w0 = mulc(0.275, s0);
-        const double d = rcp_fast(add(add(w0, m1), mulc(0.075, s2)), bad);
-        const double a = mul(w0, d), b = mul(m1, d), c = sub(sub(one, a), b);
-        r.y = eighth(add(add(mul(c, qa), mul(b, qb)), mul(a, qc)));
+    // candidate stencils of the left (+1/2) and right (-1/2) value, in the
+    // order of their sum: the left weights stencil 0 first, the right stencil 2
+    double x0 = add(__fma_rn(m2, mulk<5>(f1), t0), f15), x1 = add(__fma_rn(p2, t2, -f1), t3);
+    double x2 = sub(__fma_rn(p2, t3, t2), f4);
+    const double y0 = add(__fma_rn(m2, mulk<5>(f3), t4), f15), y1 = add(__fma_rn(p2, t2, -f3), t1);
+    const double y2 = sub(__fma_rn(p2, t1, t2), f0);
+    const double m1 = times(0.65, s1);
+    double c0 = 0.075, c2 = 0.275;
+    double2 r;
+#pragma unroll 1
+    for (int n = 0; n < 2; n++) {
+        const double w0 = times(c0, s0);
+        const double d = rcp_fast(add(add(w0, m1), times(c2, s2)), bad);
+        const double a = times(w0, d), b = times(m1, d), c = sub(sub(one, a), b);
+        const double v = add(add(times(n ? c : a, x0), times(b, x1)), times(n ? a : c, x2));
+        r.x = r.y;
+        r.y = scale<-3>(v);
+        x0 = y0;
+        x1 = y1;
+        x2 = y2;
+        c0 = 0.275;
+        c2 = 0.075;
     }
     if (bad) r = wcns4_pipe(f0, f1, f2, f3, f4);
     return r;
@@ -123,10 +127,11 @@ template <int NT> struct RecScratch {
 };
 
 // reconst_full / reconst_alfven (point.cuh) with WCNS4.  Q(k, m): variable k
-// at stencil point m; full: the full system.
-template <int NT, class LOAD>
+// at stencil point m; full: the full system; PUT(s, n, u): variable n of the
+// value at i+1/2 from the left (s = 0) and at i-1/2 from the right (s = 1).
+template <int NT, class LOAD, class STORE>
 __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed gamma,
-                                                 const RecScratch<NT> &W, ed ul[7], ed ur[7])
+                                                 const RecScratch<NT> &W, STORE PUT)
 {
     unsigned nz[7] = {0, 0, 0, 0, 0, 0, 0};
     auto column = [&](int m, ed c[7]) {
@@ -143,7 +148,7 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
         column(2, c);
         Eigen7<ed> E;
         eigen_full<ed>(c[0], c[1], bn, c[4], c[5], c[6], gamma, E);
-#pragma unroll
+#pragma unroll 1
         for (int m = 0; m < 5; m++) {
             ed wm[7];
             column(m, c);
@@ -165,15 +170,15 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
         const ed sro = tsqrt(ro);
         isroh = thalf_over(sro);
         icf2 = trcp(cf2);
-#pragma unroll
+#pragma unroll 1
         for (int m = 0; m < 5; m++) {
             column(m, c);
             const ed r = c[0], b1 = c[4], b2 = c[5], p = c[6];
-            const ed y1 = by * b1, z2 = bz * b2;
+            const ed y1 = imul(by, b1), z2 = imul(bz, b2);
             W(0, m) = c[1].v;
-            W(1, m) = (cf2 * r - y1 - z2 - p).v;
+            W(1, m) = (imul(cf2, r) - y1 - z2 - p).v;
             W(2, m) = (y1 + z2 + p).v;
-            const ed sy = sro * c[2], sz = sro * c[3];
+            const ed sy = imul(sro, c[2]), sz = imul(sro, c[3]);
             W(3, m) = (sy + b1).v;
             W(4, m) = (sy - b1).v;
             W(5, m) = (sz + b2).v;
@@ -186,9 +191,9 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
         W(n, 0) = v.x;
         W(n, 1) = v.y;
     }
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < 2; s++) {
-        ed w[7], *u = s ? ur : ul;
+        ed w[7], u[7];
 #pragma unroll
         for (int n = 0; n < 7; n++) w[n] = W(n, s);
         if (full) {
@@ -196,18 +201,20 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
             eigen_full<ed>(Q(0, 2), Q(1, 2), bn, Q(4, 2), Q(5, 2), Q(6, 2), gamma, E);
             back_full<ed>(E, w, u);
         } else {
-            const ed h = 0.5, byh = h * by, bzh = h * bz;
-            u[0] = icf2 * w[1] + icf2 * w[2];
+            const ed byh = ihalf(by), bzh = ihalf(bz);
+            u[0] = imul(icf2, w[1]) + imul(icf2, w[2]);
             u[1] = w[0];
-            u[2] = isroh * w[3] + isroh * w[4];
-            u[3] = isroh * w[5] + isroh * w[6];
-            u[4] = h * w[3] - h * w[4];
-            u[5] = h * w[5] - h * w[6];
-            u[6] = w[2] - byh * w[3] + byh * w[4] - bzh * w[5] + bzh * w[6];
+            u[2] = imul(isroh, w[3]) + imul(isroh, w[4]);
+            u[3] = imul(isroh, w[5]) + imul(isroh, w[6]);
+            u[4] = ihalf(w[3]) - ihalf(w[4]);
+            u[5] = ihalf(w[5]) - ihalf(w[6]);
+            u[6] = w[2] - imul(byh, w[3]) + imul(byh, w[4]) - imul(bzh, w[5]) + imul(bzh, w[6]);
         }
 #pragma unroll
         for (int k = 1; k <= 5; k++)
             if (nz[k] == 0) u[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 7; k++) PUT(s, k, u[k].v);
     }
 }
 

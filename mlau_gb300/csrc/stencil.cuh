@@ -25,7 +25,7 @@ struct Box {
         k = lo2 + c;
         return true;
     }
-    long long count() const { return (long long)e0 * e1 * e2; }
+    __host__ __device__ long long count() const { return (long long)e0 * e1 * e2; }
 };
 
 struct Dims {

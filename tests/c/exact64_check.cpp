@@ -48,13 +48,24 @@ extern "C" long exact64_check(int kind, int ulps, long n, long seed)
         bad += !same(x64::div(a, b), a / b);
         bad += !same(x64::div24(a), a / 24.0);
         bad += !same(x64::sqrt(a), std::sqrt(a));
-        if (!x64::off_range(x64::hi32(a))) {
-            bad += !same(x64::sqr_fast(a), a * a);
-            bad += !same(x64::mulk_fast<3>(a), 3.0 * a) + !same(x64::mulk_fast<5>(a), 5.0 * a) +
-                   !same(x64::mulk_fast<15>(a), 15.0 * a);
-            if (!x64::off_range(x64::hi32(b))) bad += !same(x64::mul_fast(a, b), a * b);
+        if (!x64::off_wide(a)) {
+            uint32_t out = 0;
+            const double q = x64::sqr(a, out);
+            if (!out) bad += !same(q, a * a);
+            bad += !same(x64::mulk<3>(a), 3.0 * a) + !same(x64::mulk<15>(a), 15.0 * a) +
+                   !same(x64::mulk<7>(a), 7.0 * a) + !same(x64::mulk<9>(a), 9.0 * a) +
+                   !same(x64::mulk<11>(a), 11.0 * a) + !same(x64::mulk<117>(a), 117.0 * a) + !same(x64::scale<-3>(a), 0.125 * a);
+            if (!x64::off_wide(b)) {
+                out = 0;
+                const double p = x64::mul(a, b, out);
+                if (!out) bad += !same(p, a * b);
+                uint32_t nz = 0;
+                const double r = x64::mul_nz(a, b, nz), s2 = x64::sqr_nz(a, nz);
+                if (!nz) bad += !same(r, a * b) + !same(s2, a * a);
+                if (a == 0.0 || b == 0.0) bad += nz == 0;
+                if (out) bad += a * b == 0.0 || (std::fabs(a * b) > 0x1p-500 && std::fabs(a * b) < 0x1p500);
+            }
         }
-        bad += !same(x64::sqrt(std::fabs(a)), std::sqrt(std::fabs(a)));
     }
     return bad;
 }
