@@ -90,30 +90,34 @@ template <> MLAU_HD ed tdiv24<ed>(ed x) { return x64::div24(x.v); }
 
 
 // a * b on the integer pipe.
-static __device__ __noinline__ double mul_pipe(double a, double b) { return a * b; }
-__device__ __forceinline__ ed imul(ed a, ed b)
+static X64_SLOW double mul_pipe(double a, double b) { return a * b; }
+MLAU_HD ed imul(ed a, ed b)
 {
     uint32_t bad = x64::off_wide(a.v) | x64::off_wide(b.v);
     double r = x64::mul(a.v, b.v, bad);
     if (bad) r = mul_pipe(a.v, b.v);
     return r;
 }
-// a / 2: exact for normal results
-__device__ __forceinline__ ed ihalf(ed a)
+// a 2^P, and k a for a small odd k
+template <int P> MLAU_HD ed iscale(ed a)
 {
-    double r = x64::scale<-1>(a.v);
-    if (x64::off_wide(a.v)) r = mul_pipe(a.v, 0.5);
+    double r = x64::scale<P>(a.v);
+    constexpr double c = P >= 0 ? (double)(1 << (P >= 0 ? P : 0)) : 1.0 / (double)(1 << (P < 0 ? -P : 0));
+    if (x64::off_wide(a.v)) r = mul_pipe(a.v, c);
+    return r;
+}
+MLAU_HD ed ihalf(ed a) { return iscale<-1>(a); }
+template <int K> MLAU_HD ed imulk(ed a)
+{
+    double r = x64::mulk<K>(a.v);
+    if (x64::off_wide(a.v)) r = mul_pipe(a.v, (double)K);
     return r;
 }
 
-template <> MLAU_HD ed thalf<ed>(ed x)
-{
-#ifdef __CUDA_ARCH__
-    return ihalf(x);
-#else
-    return x.v * 0.5;
-#endif
-}
+template <> MLAU_HD ed thalf<ed>(ed x) { return ihalf(x); }
+template <> MLAU_HD ed tsixteenth<ed>(ed x) { return iscale<-4>(x); }
+template <> MLAU_HD ed t9<ed>(ed x) { return imulk<9>(x); }
+template <> MLAU_HD ed t27<ed>(ed x) { return imulk<27>(x); }
 template <> MLAU_HD bool tzero<ed>(ed x) { return ((x64::hi32(x.v) << 1) | x64::lo32(x.v)) == 0; }
 
 // Comparisons (81 cycles each on the FP64 pipe) on the values' bits.  An
@@ -182,8 +186,10 @@ template <> MLAU_HD ed lin_l<ed>(int odr, ed f0, ed f1, ed f2, ed f3, ed f4)
 #ifdef __CUDA_ARCH__
     odr = lin_odr(odr);
     if (odr == 4) return lin4_ed(f0.v, f1.v, f2.v, f3.v, f4.v);
-    if (odr == 2) return ed(0.25) * (-f1 + ed(4.0) * f2 + f3);
-    if (odr == 3) return ed(0.125) * (-f1 + ed(6.0) * f2 + ed(3.0) * f3);
+    const double four = __hiloint2double((int)(0x40100000u + opaque_zero()), 0);
+    const double two = __hiloint2double((int)(0x40000000u + opaque_zero()), 0);
+    if (odr == 2) return iscale<-2>(ed(__fma_rn(four, f2.v, -f1.v)) + f3);
+    if (odr == 3) return iscale<-3>(ed(__fma_rn(two, imulk<3>(f2).v, -f1.v)) + imulk<3>(f3));
 #endif
     return f2;
 }

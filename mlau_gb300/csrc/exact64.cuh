@@ -181,15 +181,27 @@ X64 double round_pack(uint32_t h, uint32_t l, uint32_t m, uint32_t e)
 #endif
 }
 
-// 106-bit product of two 53-bit significands (upper half p11, then w1, w0) ->
-// rounded double; sg: the sum of the operands' sign and exponent words.
+// 106-bit product w of two 53-bit significands (upper half p11, then w1, w0),
+// normalised and rounded; sg: the sum of the operands' sign and exponent words.
 X64 double norm_round(uint64_t p11, uint32_t w1, uint32_t w0, uint32_t sg)
 {
-    const uint32_t w3 = (uint32_t)(p11 >> 32), w2 = (uint32_t)p11;
-    const uint32_t s = 12u - (w3 >> 9);
-    const uint32_t h = shfl_(w2, w3, (int)s), l = shfl_(w1, w2, (int)s);
-    const uint32_t m = shfl_(w0, w1, (int)s) | (w0 < 1u ? w0 : 1u);
-    return round_pack(h, l, m, sg - ((1012u + s) << 20));
+    const uint32_t w3 = (uint32_t)(p11 >> 32), w2 = (uint32_t)p11, t = w3 >> 9, s = 12u - t;
+    uint32_t h = shfl_(w2, w3, (int)s), l = shfl_(w1, w2, (int)s), m = shfl_(w0, w1, (int)s);
+    const uint32_t e = sg + (t << 20) - (1024u << 20);
+    // up when m > half, or m = half and something below it or an odd l: the
+    // carry of (m : v) + 0x7fffffff:ffffffff
+    const uint32_t v = w0 | (l & 1u);
+#ifdef __CUDA_ARCH__
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %3, 0xffffffff;\n\taddc.cc.u32 t, %2, 0x7fffffff;\n\t"
+        "addc.cc.u32 %0, %0, 0;\n\taddc.u32 %1, %1, %4;\n\t}"
+        : "+r"(l), "+r"(h)
+        : "r"(m), "r"(v), "r"(e));
+    return make(h, l);
+#else
+    const uint64_t c = ((uint64_t)m + 0x7fffffffu + (v ? 1u : 0u)) >> 32;
+    const uint64_t r = (((uint64_t)h << 32) | l) + c;
+    return make((uint32_t)(r >> 32) + e, (uint32_t)r);
+#endif
 }
 X64 double norm_product(uint64_t p11, uint32_t w1, uint32_t w0, uint32_t sg, uint32_t &bad)
 {
@@ -206,11 +218,10 @@ X64 double mul_nz(double a, double b, uint32_t &bad)
     const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
     const uint32_t ma = (ah & 0xfffffu) | 0x100000u, mb = (bh & 0xfffffu) | 0x100000u;
     const uint64_t p00 = wide(al, bl);
-    const uint64_t p01 = wide(al, mb) + (p00 >> 32);
-    const uint64_t p10 = wide(ma, bl) + (uint32_t)p01;
-    const uint64_t p11 = wide(ma, mb) + (p01 >> 32) + (p10 >> 32);
+    const uint64_t p01 = wide(ma, bl) + (wide(al, mb) + (p00 >> 32));  // below 2^55
+    const uint64_t p11 = wide(ma, mb) + (p01 >> 32);
     bad |= off_range(ah, bh);
-    return norm_round(p11, (uint32_t)p10, (uint32_t)p00, (ah & 0xfff00000u) + (bh & 0xfff00000u));
+    return norm_round(p11, (uint32_t)p01, (uint32_t)p00, (ah & 0xfff00000u) + (bh & 0xfff00000u));
 }
 X64 double sqr_nz(double a, uint32_t &bad)
 {
@@ -227,10 +238,9 @@ X64 double mul(double a, double b, uint32_t &bad)
     const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
     const uint32_t ma = sig_hi(ah), mb = sig_hi(bh);
     const uint64_t p00 = wide(al, bl);
-    const uint64_t p01 = wide(al, mb) + (p00 >> 32);
-    const uint64_t p10 = wide(ma, bl) + (uint32_t)p01;
-    const uint64_t p11 = wide(ma, mb) + (p01 >> 32) + (p10 >> 32);
-    return norm_product(p11, (uint32_t)p10, (uint32_t)p00, (ah & 0xfff00000u) + (bh & 0xfff00000u), bad);
+    const uint64_t p01 = wide(ma, bl) + (wide(al, mb) + (p00 >> 32));  // below 2^55
+    const uint64_t p11 = wide(ma, mb) + (p01 >> 32);
+    return norm_product(p11, (uint32_t)p01, (uint32_t)p00, (ah & 0xfff00000u) + (bh & 0xfff00000u), bad);
 }
 
 X64 double sqr(double a, uint32_t &bad)

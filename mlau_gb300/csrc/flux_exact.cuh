@@ -16,10 +16,10 @@
 // gets about one instruction per two cycles.  The two sides and the two
 // tangential components therefore share code in loops of two with their values
 // in shared memory, and blocks have 256 threads, two per SM (3D 128^3 step,
-// 9 launches: 9.1 ms; 128 threads, four per SM: 10.2; products out of line:
-// 10.2; every product an integer one: 9.5; all unrolled: 15.8).
+// 9 launches: 8.9 ms; 128 threads, four per SM, measured 1.1 ms more; products
+// out of line 10.2, all unrolled 15.8).
 //
-// Face fluxes of a 128^3 step: MLAU 15.5 -> 9.1 ms, LHLLD 8.8 -> 7.7 ms.
+// Face fluxes of a 128^3 step: MLAU 15.5 -> 8.9 ms, LHLLD 8.8 -> 7.2 ms.
 #pragma once
 
 #include "ed.cuh"
@@ -364,8 +364,8 @@ __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double
 #pragma unroll 1
         for (int p = 0; p < 2; p++) {
             const double v = IN(s, 2 + p), b = IN(s, 4 + p);
-            const double x = on ? o.add(v, o.hmul(gv, b)) : v, y = on ? o.hmul(gb, b) : b;
-            const double xy = o.hmul(x, y);
+            const double x = on ? o.add(v, o.mul(gv, b)) : v, y = on ? o.mul(gb, b) : b;
+            const double xy = o.mul(x, y);
             W(s, HX_V2 + p) = x;
             W(s, HX_B2 + p) = y;
             vb2 = p ? o.add(vb2, xy) : xy;
@@ -386,13 +386,13 @@ __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double
 #pragma unroll 1
     for (int p = 0; p < 2; p++) {
         const double v2l = W(0, HX_V2 + p), v2r = W(1, HX_V2 + p), b2l = W(0, HX_B2 + p), b2r = W(1, HX_B2 + p);
-        const double v3 = o.mul(o.in(o.add(o.add(o.hmul(qr, v2r), o.hmul(ql, v2l)), o.flip(o.sub(b2r, b2l), sgn))), qi);
-        const double b3 = o.mul(o.in(o.add(o.add(o.hmul(ql, b2r), o.hmul(qr, b2l)),
-                                           o.flip(o.hmul(qq, o.sub(v2r, v2l)), sgn))), qi);
-        const double w3 = o.hmul(v3, b3);
+        const double v3 = o.mul(o.in(o.add(o.add(o.mul(qr, v2r), o.mul(ql, v2l)), o.flip(o.sub(b2r, b2l), sgn))), qi);
+        const double b3 = o.mul(o.in(o.add(o.add(o.mul(ql, b2r), o.mul(qr, b2l)),
+                                           o.flip(o.mul(qq, o.sub(v2r, v2l)), sgn))), qi);
+        const double w3 = o.mul(v3, b3);
         vb3 = p ? o.add(vb3, w3) : w3;
         const double v = mid ? v3 : (outl ? v2l : v2r), b = mid ? b3 : (outl ? b2l : b2r);
-        const double w = o.hmul(v, b);
+        const double w = o.mul(v, b);
         vbu = p ? o.add(vbu, w) : w;
         vu[0] = vu[1];
         vu[1] = v;

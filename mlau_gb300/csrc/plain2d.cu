@@ -125,11 +125,15 @@ k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, do
     rec_central2(f, v, c, st, odr);
 }
 
-// WCNS4 with the drivers' eigen-systems.
-__global__ void __launch_bounds__(TPB, 5)
-k_rec2_wcns4(PlainFields f, View2 v, Dims d, Box b, long long st, double gamma)
+constexpr int RCT = 128;  // threads of a k_rec2_ed block
+
+// The drivers' eigen-systems (rec_exact.cuh); W4: WCNS4, else the code odr.
+template <bool W4>
+__global__ void __launch_bounds__(RCT, 5)
+k_rec2_ed(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, double gamma)
 {
-    __shared__ double w[35][TPB];
+    extern __shared__ double rec_rows[];
+    double (*w)[RCT] = (double (*)[RCT])rec_rows;
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
@@ -137,8 +141,8 @@ k_rec2_wcns4(PlainFields f, View2 v, Dims d, Box b, long long st, double gamma)
     auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
     const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
     auto PUT = [&](int s, int n, double u) { (s ? f.ur : f.ul)[n][s ? c : c + st] = u; };
-    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, PUT);
-    rec_central2(f, v, c, st, 4);
+    reconst_ed<W4, RCT>(odr, Q, full, v.cn[c], gamma, RecScratch<RCT>{w, (int)threadIdx.x}, PUT);
+    rec_central2(f, v, c, st, W4 ? 4 : odr);
 }
 
 __global__ void __launch_bounds__(TPB)
@@ -349,9 +353,11 @@ int plain2d_step(Sim *s, double dt)
             else { rb_.lo1 = 2; rb_.e1 = g.ny - 4; fb.lo1 = 3; fb.e1 = g.ny - 5; }
             {
                 TimedLaunch tl(&s->timer, KK_REC);
-                const unsigned nb = blocks_for(rb_.count(), TPB);
-                if (s->odr == 4 && s->eig == EIG_FULL)
-                    k_rec2_wcns4<<<nb, TPB, 0, st>>>(f, v, d, rb_, stride, s->gamma);
+                const unsigned nb = blocks_for(rb_.count(), TPB), nr = blocks_for(rb_.count(), RCT);
+                if (s->eig == EIG_FULL && s->odr == 4)
+                    k_rec2_ed<true><<<nr, RCT, rec_smem<RCT>(), st>>>(f, v, d, rb_, stride, 4, s->gamma);
+                else if (s->eig == EIG_FULL)
+                    k_rec2_ed<false><<<nr, RCT, rec_smem<RCT>(), st>>>(f, v, d, rb_, stride, s->odr, s->gamma);
                 else
                     k_rec2<<<nb, TPB, 0, st>>>(f, v, d, rb_, stride, s->odr, s->eig, s->gamma);
             }

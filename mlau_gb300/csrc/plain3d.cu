@@ -169,11 +169,15 @@ k_rec3(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, int eig
     rec_central(f, v, c, st, odr);
 }
 
-// WCNS4 with the drivers' eigen-systems.
-__global__ void __launch_bounds__(TPB, 5)
-k_rec3_wcns4(PlainFields f, SweepView v, Dims d, Box b, long long st, double gamma)
+constexpr int RCT = 256;  // threads of a k_rec3_ed block
+
+// The drivers' eigen-systems (rec_exact.cuh); W4: WCNS4, else the code odr.
+template <bool W4>
+__global__ void __launch_bounds__(RCT, 3)
+k_rec3_ed(PlainFields f, SweepView v, Dims d, Box b, long long st, int odr, double gamma)
 {
-    __shared__ double w[35][TPB];
+    extern __shared__ double rec_rows[];
+    double (*w)[RCT] = (double (*)[RCT])rec_rows;
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, k);
@@ -181,8 +185,8 @@ k_rec3_wcns4(PlainFields f, SweepView v, Dims d, Box b, long long st, double gam
     auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
     const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
     auto PUT = [&](int s, int n, double u) { (s ? f.ur : f.ul)[n][s ? c : c + st] = u; };
-    reconst_wcns4_ed<TPB>(Q, full, v.cn[c], gamma, RecScratch<TPB>{w, (int)threadIdx.x}, PUT);
-    rec_central(f, v, c, st, 4);
+    reconst_ed<W4, RCT>(odr, Q, full, v.cn[c], gamma, RecScratch<RCT>{w, (int)threadIdx.x}, PUT);
+    rec_central(f, v, c, st, W4 ? 4 : odr);
 }
 
 __global__ void __launch_bounds__(TPB)
@@ -283,7 +287,8 @@ k_update3(PlainFields f, Dims d, Box b, int odr, double ra_, double rb_, double 
         const ed d0 = fdiff<ed>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
         const ed d1 = fdiff<ed>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
         const ed d2 = fdiff<ed>(odr, fz[s - sz], fz[s], fz[s + sz], fz[s + 2 * sz]);
-        out[v] = (ra * f.u0[v][s] + rb * (ed(f.s[v][s]) - dtdx * d0 - dtdy * d1 - dtdz * d2)).v;
+        out[v] = (ra * f.u0[v][s] +
+                  rb * (ed(f.s[v][s]) - imul(dtdx, d0) - imul(dtdy, d1) - imul(dtdz, d2))).v;
     }
     const double *ex = f.e[0], *ey = f.e[1], *ez = f.e[2];
     {
@@ -398,6 +403,9 @@ int plain3d_alloc(Sim *s)
         rc |= dalloc(s, &f.FC[D][0], n) | dalloc(s, &f.FC[D][1], n);
     }
     if (rc) return MLAU_ERR_NOMEM;
+    for (auto k : {k_rec3_ed<true>, k_rec3_ed<false>})
+        MLAU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)rec_smem<RCT>()));
     MLAU_CUDA(cudaFuncSetAttribute(k_flux3_ed<FLUX_MLAU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)fx_smem<FLUX_MLAU>()));
     return MLAU_OK;
@@ -455,9 +463,11 @@ int plain3d_step(Sim *s, double dt)
             *e_f[D] = len - 5;  // faces [3, len-2)
             {
                 TimedLaunch tl(&s->timer, KK_REC);
-                const unsigned nb = blocks_for(rb_.count(), TPB);
-                if (s->odr == 4 && s->eig == EIG_FULL)
-                    k_rec3_wcns4<<<nb, TPB, 0, st>>>(f, v, d, rb_, strides[D], s->gamma);
+                const unsigned nb = blocks_for(rb_.count(), TPB), nr = blocks_for(rb_.count(), RCT);
+                if (s->eig == EIG_FULL && s->odr == 4)
+                    k_rec3_ed<true><<<nr, RCT, rec_smem<RCT>(), st>>>(f, v, d, rb_, strides[D], 4, s->gamma);
+                else if (s->eig == EIG_FULL)
+                    k_rec3_ed<false><<<nr, RCT, rec_smem<RCT>(), st>>>(f, v, d, rb_, strides[D], s->odr, s->gamma);
                 else
                     k_rec3<<<nb, TPB, 0, st>>>(f, v, d, rb_, strides[D], s->odr, s->eig, s->gamma);
             }

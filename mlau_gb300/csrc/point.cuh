@@ -43,6 +43,9 @@ template <class T> MLAU_HD T tsqrt_two() { return tsqrt(T(2.0)); }
 template <class T> MLAU_HD T tsqrt_half() { return tsqrt(T(0.5)); }
 
 template <class T> MLAU_HD T thalf(T x) { return T(0.5) * x; }
+template <class T> MLAU_HD T tsixteenth(T x) { return T(0.0625) * x; }
+template <class T> MLAU_HD T t9(T x) { return T(9.0) * x; }
+template <class T> MLAU_HD T t27(T x) { return T(27.0) * x; }
 template <class T> MLAU_HD bool tzero(T x) { return x == T(0); }
 
 // Epsilon of the WCNS nonlinear weights (interp.h:154,194).  In FP32 the
@@ -257,15 +260,15 @@ template <class T> MLAU_HD T lin_r(int odr, T f0, T f1, T f2, T f3, T f4)
 // calc_bc (mhd_fd_ct_3d.c:38-46)
 template <class T> MLAU_HD T face2cen(int odr, T f0, T f1, T f2, T f3)
 {
-    if (lin_odr(odr) <= 2) return T(0.5) * (f1 + f2);
-    return T(0.0625) * (T(9.0) * (f1 + f2) - (f0 + f3));
+    if (lin_odr(odr) <= 2) return thalf(f1 + f2);
+    return tsixteenth(t9(f1 + f2) - (f0 + f3));
 }
 
 // calc_df (mhd_fd_ct_3d.c:80-88)
 template <class T> MLAU_HD T fdiff(int odr, T f0, T f1, T f2, T f3)
 {
     if (lin_odr(odr) <= 2) return f2 - f1;
-    return tdiv24(T(27.0) * (f2 - f1) - (f3 - f0));
+    return tdiv24(t27(f2 - f1) - (f3 - f0));
 }
 
 // ---------------------------------------------------------------------------

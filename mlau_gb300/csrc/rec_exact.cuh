@@ -15,10 +15,12 @@
 // a lane evaluates the field on the FP64 pipe alone.  Five equal values (a
 // uniform region) take constants.
 //
-// Reconstruction of a 3D 128^3 MLAU step: 34.0 ms on the FP64 pipe alone, 20.5
-// with the WCNS4 products moved, 18.0 as it stands (FP64 pipe 82 % busy, issue
-// slots 50 %, about what instruction supply allows without reuse); four, five
-// or six blocks per SM measured 18.1 / 18.0 / 17.9 ms.
+// Reconstruction of a 3D 128^3 step (9 launches): WCNS4 34.0 ms on the FP64 pipe
+// alone, 20.5 with the WCNS4 products moved, 16.7 as it stands (FP64 pipe 85 %
+// busy, issue slots 46 %); MUSCL 9.3 -> 5.2 ms (three-point stencils project
+// three points only).  Block shapes (threads x blocks per SM) for 3D: 256 x 3
+// 16.7, 256 x 2 16.9, 128 x 5 17.3, 384 x 1 18.9 ms; the 2D grids' few waves
+// prefer 128 x 5 (512^2: 1.19 against 1.22 ms).
 #pragma once
 
 #include "ed.cuh"
@@ -126,11 +128,12 @@ template <int NT> struct RecScratch {
     __device__ __forceinline__ double &operator()(int n, int m) const { return w[5 * n + m][t]; }
 };
 
-// reconst_full / reconst_alfven (point.cuh) with WCNS4.  Q(k, m): variable k
-// at stencil point m; full: the full system; PUT(s, n, u): variable n of the
-// value at i+1/2 from the left (s = 0) and at i-1/2 from the right (s = 1).
-template <int NT, class LOAD, class STORE>
-__device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed gamma,
+// reconst_full / reconst_alfven (point.cuh).  Q(k, m): variable k at stencil
+// point m; full: the full system; PUT(s, n, u): variable n of the value at i+1/2
+// from the left (s = 0) and at i-1/2 from the right (s = 1).  W4: WCNS4; else
+// the code odr, whose stencil is three points (one point for first order).
+template <bool W4, int NT, class LOAD, class STORE>
+__device__ __forceinline__ void reconst_ed(int odr, LOAD Q, bool full, ed bn, ed gamma,
                                                  const RecScratch<NT> &W, STORE PUT)
 {
     unsigned nz[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -143,13 +146,20 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
         }
     };
     ed by, bz, icf2, isroh;
+    const int m0 = W4 ? 0 : (odr == 1 ? 2 : 1), m1 = 4 - m0;
+    if constexpr (!W4) {  // the points outside count for the zero guard only
+#pragma unroll
+        for (int k = 1; k <= 5; k++)
+            for (int m = 0; m < 5; m++)
+                if (m < m0 || m > m1) nz[k] |= (x64::hi32(Q(k, m)) << 1) | x64::lo32(Q(k, m));
+    }
     if (full) {
         ed c[7];
         column(2, c);
         Eigen7<ed> E;
         eigen_full<ed>(c[0], c[1], bn, c[4], c[5], c[6], gamma, E);
 #pragma unroll 1
-        for (int m = 0; m < 5; m++) {
+        for (int m = m0; m <= m1; m++) {
             ed wm[7];
             column(m, c);
             proj_full<ed>(E, c[0], c[1], c[2], c[3], c[4], c[5], c[6], wm);
@@ -171,7 +181,7 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
         isroh = thalf_over(sro);
         icf2 = trcp(cf2);
 #pragma unroll 1
-        for (int m = 0; m < 5; m++) {
+        for (int m = m0; m <= m1; m++) {
             column(m, c);
             const ed r = c[0], b1 = c[4], b2 = c[5], p = c[6];
             const ed y1 = imul(by, b1), z2 = imul(bz, b2);
@@ -187,9 +197,18 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
     }
 #pragma unroll 1
     for (int n = 0; n < 7; n++) {
-        const double2 v = wcns4_ed(W(n, 0), W(n, 1), W(n, 2), W(n, 3), W(n, 4));
-        W(n, 0) = v.x;
-        W(n, 1) = v.y;
+        if constexpr (W4) {
+            const double2 v = wcns4_ed(W(n, 0), W(n, 1), W(n, 2), W(n, 3), W(n, 4));
+            W(n, 0) = v.x;
+            W(n, 1) = v.y;
+        } else {
+            const double c = W(n, 2), a = odr == 1 ? c : W(n, 1), b = odr == 1 ? c : W(n, 3);
+            const ed f[5] = {a, a, c, b, b};
+            ed l, r;
+            rec_lr(odr, f, l, r);
+            W(n, 0) = l.v;
+            W(n, 1) = r.v;
+        }
     }
 #pragma unroll 1
     for (int s = 0; s < 2; s++) {
@@ -217,5 +236,7 @@ __device__ __forceinline__ void reconst_wcns4_ed(LOAD Q, bool full, ed bn, ed ga
         for (int k = 0; k < 7; k++) PUT(s, k, u[k].v);
     }
 }
+
+template <int NT> constexpr size_t rec_smem() { return sizeof(double) * 35 * NT; }
 
 }  // namespace mlau

@@ -44,16 +44,16 @@ __device__ __forceinline__ double ct_weight(const double *va, const double *vb, 
                                             const double *ba, const double *bbf, long long s,
                                             long long P, long long Q, long long oa, long long ob)
 {
-    const ed eps = 1e-6, h = 0.5, q = 0.25;
+    const ed eps = 1e-6;
     auto sum4 = [&](const double *f) { return ed(f[s - P - Q]) + f[s - P] + f[s - Q] + f[s]; };
-    ed a = q * sum4(va);
-    ed c = q * sum4(vb);
-    ed rc = q * sum4(ro);
+    ed a = iscale<-2>(sum4(va));
+    ed c = iscale<-2>(sum4(vb));
+    ed rc = iscale<-2>(sum4(ro));
     rc = trcp(tsqrt(rc));
-    const ed fa = h * (ed(ba[s - oa]) + ba[s]);
-    const ed fb = h * (ed(bbf[s - ob]) + bbf[s]);
-    a = tabs(a) + tabs(fa * rc);
-    c = tabs(c) + tabs(fb * rc);
+    const ed fa = ihalf(ed(ba[s - oa]) + ba[s]);
+    const ed fb = ihalf(ed(bbf[s - ob]) + bbf[s]);
+    a = tabs(a) + tabs(imul(fa, rc));
+    c = tabs(c) + tabs(imul(fb, rc));
     return ((a + ed(0.5 * 1e-6)) / (a + c + eps)).v;
 }
 
@@ -68,7 +68,8 @@ __device__ __forceinline__ ed emf_part(const double *fu, const double *fc, ed w,
     auto r = [&](const double *f) {
         return lin_r<ed>(odr, f[c - 2 * st], f[c - st], f[c], f[c + st], f[c + 2 * st]);
     };
-    return ed(sgn * 0.5) * ((l(fu) + r(fu)) + w * (l(fc) + r(fc)));
+    const ed e = ihalf((l(fu) + r(fu)) + w * (l(fc) + r(fc)));
+    return sgn < 0.0 ? -e : e;
 }
 
 inline void rk_coef(int nrk, int stage, double &a, double &b)
