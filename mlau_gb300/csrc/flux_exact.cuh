@@ -26,15 +26,17 @@
 
 namespace mlau {
 
-// Operations of one flux evaluation.  Sums run on the FP64 pipe, products,
-// quotients and roots as integer sequences; `bad` collects every input and
-// product outside the integer path's range (zero apart) and every undecided
-// rounding, so while it is zero all values are finite and comparisons can be
-// made on their bits.
-struct FxOps {
+// Operations of one flux evaluation.  Sums run on the FP64 pipe, quotients and
+// roots as integer sequences.  PIPE = false: products are integer sequences too,
+// and `bad` collects every input and product outside the integer path's range
+// (zero apart) and every undecided rounding.  PIPE = true, for grids that leave
+// the pipes idle and wait on instructions instead: products stay on the FP64
+// pipe, one instruction each.  Either way `bad` is zero only if every value
+// that was compared is finite, so comparisons can be made on the values' bits.
+template <bool PIPE> struct FxOpsT {
     uint32_t bad = 0;
     double one, mz;
-    __device__ __forceinline__ FxOps() : one(ed_one()), mz(ed_minus_zero()) {}
+    __device__ __forceinline__ FxOpsT() : one(ed_one()), mz(ed_minus_zero()) {}
 
     static __device__ __forceinline__ uint32_t hi(double x) { return x64::hi32(x); }
     static __device__ __forceinline__ uint32_t lo(double x) { return x64::lo32(x); }
@@ -42,16 +44,28 @@ struct FxOps {
     // an input: zero or in range
     __device__ __forceinline__ double in(double x)
     {
-        bad |= x64::off_wide(x);
+        if constexpr (!PIPE) bad |= x64::off_wide(x);
         return x;
+    }
+    // a value about to be compared: finite
+    __device__ __forceinline__ void cmp(double x)
+    {
+        if constexpr (PIPE) bad |= (hi(x) << 1) >= 0xffe00000u ? 1u : 0u;
     }
     __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
     __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(-b, one, a); }
     // on the FP64 pipe; the operands are looked at elsewhere
     __device__ __forceinline__ double hmul(double a, double b) const { return __fma_rn(a, b, mz); }
-    __device__ __forceinline__ double mul(double a, double b) { return x64::mul(a, b, bad); }
-    __device__ __forceinline__ double sqr(double a) { return x64::sqr(a, bad); }
-    template <int P> static __device__ __forceinline__ double scale(double a) { return x64::scale<P>(a); }
+    __device__ __forceinline__ double mul(double a, double b)
+    {
+        return PIPE ? hmul(a, b) : x64::mul(a, b, bad);
+    }
+    __device__ __forceinline__ double sqr(double a) { return PIPE ? hmul(a, a) : x64::sqr(a, bad); }
+    template <int P> __device__ __forceinline__ double scale(double a) const
+    {
+        constexpr double c = P >= 0 ? (double)(1 << (P >= 0 ? P : 0)) : 1.0 / (double)(1 << (P < 0 ? -P : 0));
+        return PIPE ? hmul(a, c) : x64::scale<P>(a);
+    }
     __device__ __forceinline__ double rcp(double a) { return x64::rcp_fast(a, bad); }
     // a may be zero
     __device__ __forceinline__ double div(double a, double b)
@@ -69,25 +83,40 @@ struct FxOps {
         return zero(a) ? a : r;
     }
     static __device__ __forceinline__ double abs(double a) { return x64::make(hi(a) & 0x7fffffffu, lo(a)); }
-    static __device__ __forceinline__ bool positive(double a) { return (int32_t)hi(a) > 0; }
-    static __device__ __forceinline__ bool ge(double a, double b)
+    __device__ __forceinline__ bool positive(double a)
     {
+        cmp(a);
+        return PIPE ? (int32_t)hi(a) > 0 || (hi(a) == 0 && lo(a) != 0) : (int32_t)hi(a) > 0;
+    }
+    __device__ __forceinline__ bool ge(double a, double b)
+    {
+        cmp(a);
+        cmp(b);
         const int32_t ha = (int32_t)hi(a), hb = (int32_t)hi(b), sa = ha >> 31, sb = hb >> 31;
         const int32_t ka = ha ^ (sa & 0x7fffffff), kb = hb ^ (sb & 0x7fffffff);
         return ka > kb || (ka == kb && (lo(a) ^ (uint32_t)sa) >= (lo(b) ^ (uint32_t)sb));
     }
-    static __device__ __forceinline__ double max(double a, double b) { return ge(a, b) ? a : b; }
-    static __device__ __forceinline__ double min(double a, double b) { return ge(a, b) ? b : a; }
-    static __device__ __forceinline__ double max0(double a) { return (int32_t)hi(a) < 0 ? 0.0 : a; }
-    static __device__ __forceinline__ double min0(double a) { return (int32_t)hi(a) < 0 ? a : 0.0; }
+    // a > b for a >= 0 and a constant b > 0
+    __device__ __forceinline__ bool above(double a, double b)
+    {
+        cmp(a);
+        return hi(a) > hi(b) || (hi(a) == hi(b) && lo(a) > lo(b));
+    }
+    __device__ __forceinline__ double max(double a, double b) { return ge(a, b) ? a : b; }
+    __device__ __forceinline__ double min(double a, double b) { return ge(a, b) ? b : a; }
+    __device__ __forceinline__ double max0(double a)
+    {
+        cmp(a);
+        return (int32_t)hi(a) < 0 ? 0.0 : a;
+    }
+    __device__ __forceinline__ double min0(double a)
+    {
+        cmp(a);
+        return (int32_t)hi(a) < 0 ? a : 0.0;
+    }
     static __device__ __forceinline__ double flip(double a, uint32_t sign) { return x64::make(hi(a) ^ sign, lo(a)); }
 };
-
-// a > b for a >= 0 and a constant b > 0
-__device__ __forceinline__ bool above(double a, double b)
-{
-    return x64::hi32(a) > x64::hi32(b) || (x64::hi32(a) == x64::hi32(b) && x64::lo32(a) > x64::lo32(b));
-}
+using FxOps = FxOpsT<false>;
 
 static __device__ __noinline__ void flux_mlau_pipe(const double *L, const double *R, double bn, double gamma,
                                                    double dv0, double dv1, double *f)
@@ -164,7 +193,7 @@ __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double
         const double ro = IN(s, 0), vn = IN(s, 1), m = o.mul(vn, cfni);
         const double m2 = o.sub(o.sqr(m), o.one), q = o.scale<-2>(o.sqr(o.add(m, o.flip(o.one, sp))));
         const double a = o.mul(o.mul(o.mul(m, 0.1875), m2), m2);
-        const bool sup = above(o.abs(m), 1.0);
+        const bool sup = o.above(o.abs(m), 1.0);
         const double bf = o.add(o.mul(q, o.sub(2.0, o.flip(m, sp))), o.flip(a, sp));
         const double ff = o.flip(o.add(q, o.scale<-3>(o.sqr(m2))), sp);
         const double on = o.positive(o.flip(m, sp)) ? 1.0 : 0.0;
@@ -188,7 +217,7 @@ __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double
                                      o.sub(o.add(bfl, bfr), o.one)), o.add(ptl, ptr)));
     const double snc = up ? sr : sl;
     const double vndnm = o.add(mflux, W(up, FX_RS));
-    const bool has = above(o.abs(vndnm), EPS) && !o.zero(snc);
+    const bool has = o.above(o.abs(vndnm), EPS) && !o.zero(snc);
     const double vq = o.div(o.mul(mflux, snc), has ? vndnm : 1.0);
     const double vnc = has ? vq : IN(up, 1);
     // each side's star state
@@ -196,7 +225,7 @@ __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double
     for (int s = 0; s < 2; s++) {
         const double sc = o.sub(s ? sr : sl, vnc), sci = o.rcp(sc);
         const double rhd = o.sub(o.mul(W(s, FX_RS), sc), bnc2);
-        const bool on = above(o.abs(rhd), EPS);
+        const bool on = o.above(o.abs(rhd), EPS);
         const double gq = o.div(o.sub(vnc, IN(s, 1)), on ? rhd : 1.0), g = on ? gq : 0.0;
         const double c = o.mul(W(s, FX_SV), sci);
         W(s, FX_SCI) = sci;
@@ -245,7 +274,7 @@ __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double
         vb3 = p ? o.add(vb3, w3) : w3;
     }
     const double rv = o.sqr(o.sub(o.mul(mflux, vnc), bnc2));
-    const bool on = above(rv, EPS * EPS);
+    const bool on = o.above(rv, EPS * EPS);
     vb3 = o.div(vb3, on ? rv : 1.0);
     vb3 = on ? vb3 : 0.0;
     const double nvb = o.add(o.mul(o.mul(bnca, o.sub(o.mul(snc, vb2), o.mul(vnc, vb1))), W(up, FX_SCI)),
@@ -356,7 +385,7 @@ __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double
         const double sc = o.sub(s ? sr : sl, vnc);
         const double ro2 = o.div(rs, sc);
         const double rhd = o.sub(o.mul(rs, sc), bnc2);
-        const bool on = above(o.abs(rhd), EPS);
+        const bool on = o.above(o.abs(rhd), EPS);
         const double rhdi = o.rcp(on ? rhd : 1.0);
         const double gv = o.mul(o.mul(o.sub(vn, vnc), bnc), rhdi);
         const double gb = o.mul(o.sub(o.mul(rs, sv), bnc2), rhdi);

@@ -6,25 +6,26 @@
 // long-running service that admits work under a fixed device-memory budget,
 // or host code between graph captures that must not change the device memory
 // map.  mlau_fd4c_1d_noalloc serves them: it advances one 1D step on arrays
-// the caller already has on the device, and keeps its own scratch (the U^n
-// copy, primitives, face states and fluxes) in one statically sized device
-// array of this file, so it allocates nothing.
+// the caller already has on the device, and keeps its own scratch (the states
+// between the stages) in one statically sized device array of this file, so it
+// allocates nothing.
 #include <mutex>
 
+#include "point.cuh"
 #include "sim.cuh"
 
 namespace mlau {
-int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int flux, int nrk, int bc,
+int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int eig, int flux, int nrk, int bc,
                     double bx, double dt, double dx, double gamma, cudaStream_t st);
 }
 
 namespace {
 
 constexpr int kMaxNx = MLAU_NOALLOC_1D_MAX_NX;
-// u0 (7 x nx) + vx, vy, vz, pr (4 x nx) + face states (14 x (nx+1)) + fluxes
-// (7 x nx) + the open boundary's two ghost states (14): 32 nx + 28 doubles
+// the two buffers the stages go through: 14 nx doubles (the array's size is the
+// one the header states)
 constexpr long long kScratch = 32LL * (kMaxNx + 1);
-static_assert(32LL * kMaxNx + 28 <= kScratch, "noalloc scratch too small");
+static_assert(14LL * kMaxNx <= kScratch, "noalloc scratch too small");
 
 // One array per process and device; it lives until the process exits.
 static __device__ __align__(256) double g_noalloc_scratch[kScratch];
@@ -88,19 +89,8 @@ extern "C" int mlau_fd4c_1d_noalloc(double *ro, double *mx, double *my, double *
     PlainFields f{};
     f.s[0] = ro; f.s[1] = mx; f.s[2] = my; f.s[3] = mz; f.s[4] = en; f.s[6] = by; f.s[7] = bz;
     double *p = base;
-    for (int v = 0; v < 8; v++) {
-        if (v == 5) continue;
-        f.u0[v] = p;
-        p += nx;
-    }
-    f.vx = p; p += nx;
-    f.vy = p; p += nx;
-    f.vz = p; p += nx;
-    f.pr = p; p += nx;
-    for (int v = 0; v < 7; v++) { f.ul[v] = p; p += nx + 1; }
-    for (int v = 0; v < 7; v++) { f.ur[v] = p; p += nx + 1; }
-    for (int v = 0; v < 7; v++) { f.F[0][v] = p; p += nx; }
-    f.obc = p;
-    return plain1d_enqueue(f, nx, xoff, odr, flux, nrk, bc, bx, dt, dx, gamma,
+    for (int v = 0; v < 7; v++) { f.ul[v] = p; p += nx; }
+    for (int v = 0; v < 7; v++) { f.ur[v] = p; p += nx; }
+    return plain1d_enqueue(f, nx, xoff, odr, EIG_FULL, flux, nrk, bc, bx, dt, dx, gamma,
                            (cudaStream_t)stream);
 }
