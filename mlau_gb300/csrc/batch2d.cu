@@ -39,6 +39,7 @@ struct mlau_batch {
     int graph_steps = 0;
     long long launches = 0;
     const void *kernel = nullptr;
+    size_t smem = 0;  // dynamic shared memory of a block
 };
 
 namespace {
@@ -102,7 +103,9 @@ int occupancy(mlau_batch *b)
     int dev = 0, sms = 0, per_sm = 0;
     MLAU_CUDA(cudaGetDevice(&dev));
     MLAU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MLAU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->kernel, b->tw * b->th, 0));
+    b->smem = b->dim == 1 ? batch1d_smem(b->tw) : 0;
+    MLAU_CUDA(cudaFuncSetAttribute(b->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
+    MLAU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->kernel, b->tw * b->th, b->smem));
     if (per_sm < 1) { set_error("batch: step kernel does not fit on an SM"); return MLAU_ERR_ARG; }
     b->max_blocks = (unsigned)(sms * per_sm);
     b->nblocks = b->want_blocks ? std::min(b->want_blocks, b->max_blocks) : b->max_blocks;
@@ -118,6 +121,12 @@ int build_tiles(mlau_batch *b)
         if (!b->used[n] || !b->h_inst[n].active) continue;
         const BInst &I = b->h_inst[n];
         per.emplace_back();
+        if (b->dim == 1) {  // b->tw: the threads of a tile
+            const int no = batch1d_tile_cells(b->tw, b->odr);
+            for (int x = I.off; x < I.nx - I.off; x += no) per.back().push_back({n, x, 0, 0});
+            if (I.bc == MLAU_BC1D_OPEN) per.back().push_back({n, 0, 0, 1});
+            continue;
+        }
         for (int y = 0; y < I.ny; y += b->th)
             for (int x = 0; x < I.nx; x += b->tw) per.back().push_back({n, x, y, 0});
     }
@@ -164,6 +173,7 @@ int launch_step(mlau_batch *b)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(b->nblocks);
     cfg.blockDim = dim3(b->tw, b->th);
+    cfg.dynamicSmemBytes = b->smem;
     cfg.stream = b->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -337,7 +347,7 @@ int mlau_batch1d_open(mlau_batch **out, long long capacity_cells, int max_inst, 
     b->h_inst.assign(max_inst, BInst{});
     b->used.assign(max_inst, 0);
     b->free_[0] = capacity_cells;
-    b->kernel = batch1d_plain_kernel();
+    b->kernel = batch1d_plain_kernel(b->tw, odr);
     if (make_stream(&b->stream) != cudaSuccess) {
         set_error("batch1d: stream creation failed");
         delete b;
@@ -347,15 +357,10 @@ int mlau_batch1d_open(mlau_batch **out, long long capacity_cells, int max_inst, 
     BArrays &a = b->a;
     int rc = MLAU_OK;
     for (int v = 0; v < 8 && !rc; v++) {
-        if (v == 5) continue;
-        rc |= balloc(b, (void **)&a.s[v], n8) | balloc(b, (void **)&a.u0[v], n8);
+        if (v == 5) continue;  // the state and the two pools the stages go through
+        rc |= balloc(b, (void **)&a.s[v], n8) | balloc(b, (void **)&a.ul[v], n8) |
+              balloc(b, (void **)&a.ur[v], n8);
     }
-    double **singles[] = {&a.vx, &a.vy, &a.vz, &a.pr};
-    for (auto p : singles)
-        if (!rc) rc |= balloc(b, (void **)p, n8);
-    for (int v = 0; v < 7 && !rc; v++)
-        rc |= balloc(b, (void **)&a.ul[v], n8) | balloc(b, (void **)&a.ur[v], n8) |
-              balloc(b, (void **)&a.F[0][v], n8);
     if (!rc)
         rc |= balloc(b, (void **)&b->d_inst, sizeof(BInst) * max_inst) |
               balloc(b, (void **)&b->d_sync, sizeof(BSync));
@@ -622,6 +627,7 @@ int mlau_batch_set_tile(mlau_batch *b, int tw, int th)
     }
     b->tw = tw;
     b->th = th;
+    if (b->dim == 1) b->kernel = batch1d_plain_kernel(tw, b->odr);
     b->tiles_dirty = true;
     if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
     return occupancy(b);

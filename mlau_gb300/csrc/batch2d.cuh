@@ -34,7 +34,7 @@ struct BInst {
     signed char bcx[8], bcy[8];
 };
 
-struct BTile { int inst, x0, y0, pad; };
+struct BTile { int inst, x0, y0, open; };  // open: the open boundary of a 1D instance
 
 struct BSync {
     unsigned count, gen;
@@ -99,6 +99,21 @@ __device__ __forceinline__ bool grid_barrier(BSync *sy, unsigned nblocks)
     }
     __syncthreads();
     return stop != 0;
+}
+
+// True in the block that gets here last, which then sees what all wrote.
+__device__ __forceinline__ bool grid_last(BSync *sy, unsigned nblocks)
+{
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        __threadfence();
+        last = atomicAdd(&sy->count, 1u) == nblocks - 1;
+        if (last) sy->count = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    return last != 0;
 }
 
 __device__ __forceinline__ int bwrap(int i, int n, int off)
@@ -199,6 +214,8 @@ __device__ __forceinline__ void batch_vmax(BInst &I, double vt)
 // Kernel entry points (one per arithmetic), for the host launcher.
 const void *batch2d_split_kernel();
 const void *batch2d_plain_kernel();
-const void *batch1d_plain_kernel();
+const void *batch1d_plain_kernel(int threads, int odr);
+int batch1d_tile_cells(int threads, int odr);
+size_t batch1d_smem(int threads);
 
 }  // namespace mlau

@@ -116,7 +116,6 @@ template <bool PIPE> struct FxOpsT {
     }
     static __device__ __forceinline__ double flip(double a, uint32_t sign) { return x64::make(hi(a) ^ sign, lo(a)); }
 };
-using FxOps = FxOpsT<false>;
 
 static __device__ __noinline__ void flux_mlau_pipe(const double *L, const double *R, double bn, double gamma,
                                                    double dv0, double dv1, double *f)
@@ -138,7 +137,7 @@ template <int ND, int NT, class LOAD>
 __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
                                              const double dv[ND], double f[7])
 {
-    FxOps o;
+    FxOpsT<false> o;
     const int t = threadIdx.x;
     auto W = [&](int s, int k) -> double & { return rows[s * FX_ROWS + k][t]; };
     double dv1 = dv[0];
@@ -316,7 +315,7 @@ template <bool LOWDISS, int ND, int NT, class LOAD>
 __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
                                              const double dv[ND], double f[7])
 {
-    FxOps o;
+    FxOpsT<false> o;
     const int t = threadIdx.x;
     auto W = [&](int s, int k) -> double & { return rows[s * HX_ROWS + k][t]; };
     double dv1 = dv[0];

@@ -132,7 +132,10 @@ template <int NT> struct RecScratch {
 // point m; full: the full system; PUT(s, n, u): variable n of the value at i+1/2
 // from the left (s = 0) and at i-1/2 from the right (s = 1).  W4: WCNS4; else
 // the code odr, whose stencil is three points (one point for first order).
-template <bool W4, int NT, class LOAD, class STORE>
+// KEEP: hold the full system in registers between projection and
+// back-projection, else form it again (kernels where it is rare and registers
+// are short).
+template <bool W4, int NT, bool KEEP = false, class LOAD, class STORE>
 __device__ __forceinline__ void reconst_ed(int odr, LOAD Q, bool full, ed bn, ed gamma,
                                                  const RecScratch<NT> &W, STORE PUT)
 {
@@ -153,10 +156,10 @@ __device__ __forceinline__ void reconst_ed(int odr, LOAD Q, bool full, ed bn, ed
             for (int m = 0; m < 5; m++)
                 if (m < m0 || m > m1) nz[k] |= (x64::hi32(Q(k, m)) << 1) | x64::lo32(Q(k, m));
     }
+    Eigen7<ed> E;
     if (full) {
         ed c[7];
         column(2, c);
-        Eigen7<ed> E;
         eigen_full<ed>(c[0], c[1], bn, c[4], c[5], c[6], gamma, E);
 #pragma unroll 1
         for (int m = m0; m <= m1; m++) {
@@ -216,8 +219,7 @@ __device__ __forceinline__ void reconst_ed(int odr, LOAD Q, bool full, ed bn, ed
 #pragma unroll
         for (int n = 0; n < 7; n++) w[n] = W(n, s);
         if (full) {
-            Eigen7<ed> E;
-            eigen_full<ed>(Q(0, 2), Q(1, 2), bn, Q(4, 2), Q(5, 2), Q(6, 2), gamma, E);
+            if constexpr (!KEEP) eigen_full<ed>(Q(0, 2), Q(1, 2), bn, Q(4, 2), Q(5, 2), Q(6, 2), gamma, E);
             back_full<ed>(E, w, u);
         } else {
             const ed byh = ihalf(by), bzh = ihalf(bz);
