@@ -50,6 +50,8 @@
 #include "point.cuh"
 #include "tma.cuh"
 #include "split_conv.cuh"
+#include "ed.cuh"
+#include "emf_diff.cuh"
 #include "ff.cuh"
 #include "point_x2.cuh"
 #include "slab_plan.h"
@@ -655,9 +657,37 @@ ks_sweep(const __grid_constant__ SweepMaps M, SplitPtrs g, Dims d, int odr_rt, i
 }
 
 // --- edge EMFs (FP32) --------------------------------------------------------
+// ODR: 4, or 0 for the order at run time.  Knowing the order saves a fifth of the
+// instructions (256^3, one step: 1.43 -> 1.22 ms); the waits for the 76 loads of a
+// cell are what is left.
+// lin_l and lin_r (mirrored) of 4th order.  Which products join which sums in
+// FMAs is written out in the forms for this order here and in ks_update: left
+// to the compiler it changes with what stands around them, and the step's FP32
+// roundings with it.
+__device__ __forceinline__ float lin4_fma(float f0, float f1, float f2, float f3, float f4)
+{
+    const float a = __fmaf_rn(9.f, f0, __fmul_rn(-56.f, f1));
+    return __fmul_rn(0.003125f, __fmaf_rn(-11.f, f4, __fmaf_rn(144.f, f3, __fmaf_rn(234.f, f2, a))));
+}
+__device__ __forceinline__ float emf_part4(const float *fu, const float *fc, float w, float h, long long c,
+                                           long long st)
+{
+    float u[6], v[6];
+#pragma unroll
+    for (int m = 0; m < 6; m++) {
+        u[m] = fu[c + (m - 3) * st];
+        v[m] = fc[c + (m - 3) * st];
+    }
+    const float ul0 = lin4_fma(u[0], u[1], u[2], u[3], u[4]), ul1 = lin4_fma(v[0], v[1], v[2], v[3], v[4]);
+    const float ur0 = lin4_fma(u[5], u[4], u[3], u[2], u[1]), ur1 = lin4_fma(v[5], v[4], v[3], v[2], v[1]);
+    return h * __fmaf_rn(w, __fadd_rn(ul1, ur1), __fadd_rn(ul0, ur0));
+}
+
+template <int ODR>
 __device__ __forceinline__ float emf_part32(const float *fu, const float *fc, float w, float h,
                                             long long c, long long st, int odr)
 {
+    if constexpr (ODR == 4) return emf_part4(fu, fc, w, h, c, st);
     const float ul0 = lin_l(odr, fu[c - 3 * st], fu[c - 2 * st], fu[c - st], fu[c], fu[c + st]);
     const float ul1 = lin_l(odr, fc[c - 3 * st], fc[c - 2 * st], fc[c - st], fc[c], fc[c + st]);
     const float ur0 = lin_r(odr, fu[c - 2 * st], fu[c - st], fu[c], fu[c + st], fu[c + 2 * st]);
@@ -665,8 +695,10 @@ __device__ __forceinline__ float emf_part32(const float *fu, const float *fc, fl
     return h * ((ul0 + ur0) + w * (ul1 + ur1));
 }
 
-__global__ void __launch_bounds__(256) ks_emf(SplitPtrs g, Dims d, int odr, int k0)
+template <int ODR>
+__global__ void __launch_bounds__(256) ks_emf(SplitPtrs g, Dims d, int odr_rt, int k0)
 {
+    const int odr = ODR ? ODR : odr_rt;
     int i, j, k;
     if (!plane_cell(d, i, j, k, k0)) return;
     const long long sy = d.px, sz = d.px * d.ny;
@@ -676,18 +708,18 @@ __global__ void __launch_bounds__(256) ks_emf(SplitPtrs g, Dims d, int odr, int 
     float ez = 0.f, ex = 0.f, ey = 0.f;
     if (xi && yj) {
         const float w = g.ct[0][c];
-        ez = emf_part32(g.F[0][4], g.FC[0][0], 1.f - w, -0.5f, c, sy, odr)
-             + emf_part32(g.F[1][5], g.FC[1][1], w, 0.5f, c, 1, odr);
+        ez = emf_part32<ODR>(g.F[0][4], g.FC[0][0], 1.f - w, -0.5f, c, sy, odr)
+             + emf_part32<ODR>(g.F[1][5], g.FC[1][1], w, 0.5f, c, 1, odr);
     }
     if (yj && zk) {
         const float w = g.ct[1][c];
-        ex = emf_part32(g.F[1][4], g.FC[1][0], 1.f - w, -0.5f, c, sz, odr)
-             + emf_part32(g.F[2][5], g.FC[2][1], w, 0.5f, c, sy, odr);
+        ex = emf_part32<ODR>(g.F[1][4], g.FC[1][0], 1.f - w, -0.5f, c, sz, odr)
+             + emf_part32<ODR>(g.F[2][5], g.FC[2][1], w, 0.5f, c, sy, odr);
     }
     if (zk && xi) {
         const float w = g.ct[2][c];
-        ey = emf_part32(g.F[0][5], g.FC[0][1], w, 0.5f, c, sz, odr)
-             + emf_part32(g.F[2][4], g.FC[2][0], 1.f - w, -0.5f, c, 1, odr);
+        ey = emf_part32<ODR>(g.F[0][5], g.FC[0][1], w, 0.5f, c, sz, odr)
+             + emf_part32<ODR>(g.F[2][4], g.FC[2][0], 1.f - w, -0.5f, c, 1, odr);
     }
     g.e[0][c] = ex;
     g.e[1][c] = ey;
@@ -700,10 +732,14 @@ __global__ void __launch_bounds__(256) ks_emf(SplitPtrs g, Dims d, int odr, int 
 // magnitude) and accumulated into the state in float-float.
 //
 // The kernel streams some 60 flux values, 24 edge EMFs and 16 state values
-// per cell with little arithmetic between them, so it is bound by memory
-// latency unless the loads are in flight together: every value is read into
-// registers first (read-only data through the non-coherent path), and the
-// arithmetic follows.
+// per cell; every value is read into registers first (read-only data through
+// the non-coherent path), so that the loads are in flight together, and the
+// arithmetic follows.  The FP64 pipe bounded it with the curl's differences
+// (36 instructions of 64 cycles a cell); these are formed on the integer pipe
+// (emf_diff.cuh), and instruction issue bounds it now: 256^3, one step, 4.50 ->
+// 3.59 ms (more or fewer registers: 3.60 at 80, 4.00 at 64).  One thread per
+// cell of an x-y plane, flattened: rows of blocks left 38 % of the threads idle
+// at nx = 160 and half of them at 61.
 
 // The RK combine ra u0 + rb u in float-float (ra = 0, rb = 1 at the first stage).
 struct RkFF {
@@ -723,13 +759,12 @@ __device__ __forceinline__ void ld4(float v[4], const float *f, long long s, lon
     for (int m = 0; m < 4; m++) v[m] = __ldg(f + s + (m - 1) * st);
 }
 
-// FP64 difference of the FP32 edge EMFs f0..f3 along one axis (the values
-// converted exactly), without the 1/24 of the 4th-order stencil.
+// FP64 difference of the FP32 edge EMFs e[0..3] along one axis (the values
+// taken exactly), without the 1/24 of the 4th-order stencil.
 __device__ __forceinline__ double df_f64(int odr, const float e[4])
 {
-    const double e0 = to_f64(e[0]), e1 = to_f64(e[1]), e2 = to_f64(e[2]), e3 = to_f64(e[3]);
-    if (lin_odr(odr) <= 2) return e2 - e1;
-    return 27.0 * (e2 - e1) - (e3 - e0);
+    if (lin_odr(odr) <= 2) return to_f64(e[2]) - to_f64(e[1]);
+    return emf_diff4(e);
 }
 
 // F64: the RK combine of the cell-centred variables in FP64 arithmetic (the
@@ -741,14 +776,26 @@ struct RkF64 {
     double ra, rb, ddx, ddy, ddz;
 };
 
-template <bool F64>
+// fdiff of 4th order
+__device__ __forceinline__ float fdiff4(const float f[4])
+{
+    return __fmul_rn(__fmaf_rn(27.f, __fsub_rn(f[2], f[1]), -__fsub_rn(f[3], f[0])), 1.f / 24.f);
+}
+
+__device__ __forceinline__ double curl(double u, double a, double x, double b, double y)
+{
+    return __fma_rn(b, y, __fma_rn(-a, x, u));
+}
+
+template <bool F64, int ODR>
 __global__ void __launch_bounds__(128)
-ks_update(PlainFields f, SplitPtrs g, Dims d, int odr, RkFF rk, RkF64 rd, float dtdx, float dtdy,
+ks_update(PlainFields f, SplitPtrs g, Dims d, int odr_rt, RkFF rk, RkF64 rd, float dtdx, float dtdy,
           float dtdz, int images, int k0)
 {
-    const int i = d.ox + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = d.oy + blockIdx.y, k = k0 + blockIdx.z;
-    if (i >= d.nx - d.ox) return;
+    const int odr = ODR ? ODR : odr_rt;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, row = d.nx - 2 * d.ox;
+    if (q >= row * (d.ny - 2 * d.oy)) return;
+    const int j = d.oy + q / row, i = d.ox + q - row * (q / row), k = k0 + blockIdx.y;
     const long long sy = d.px, sz = d.px * d.ny;  // scratch strides
     const long long s = d.at(i, j, k), sp = d.ap(i, j, k);
     const int cX[5] = {0, 1, 2, 3, 6}, cY[5] = {0, 3, 1, 2, 6}, cZ[5] = {0, 2, 3, 1, 6};
@@ -777,9 +824,15 @@ ks_update(PlainFields f, SplitPtrs g, Dims d, int odr, RkFF rk, RkF64 rd, float 
     double out[8];
 #pragma unroll
     for (int v = 0; v < 5; v++) {
-        const float div = dtdx * fdiff(odr, fx[v][0], fx[v][1], fx[v][2], fx[v][3])
-                          + dtdy * fdiff(odr, fy[v][0], fy[v][1], fy[v][2], fy[v][3])
-                          + dtdz * fdiff(odr, fz[v][0], fz[v][1], fz[v][2], fz[v][3]);
+        float div;
+        if constexpr (ODR == 4)
+            div = __fmaf_rn(dtdz, fdiff4(fz[v]),
+                            v < 4 ? __fmaf_rn(dtdx, fdiff4(fx[v]), __fmul_rn(dtdy, fdiff4(fy[v])))
+                                  : __fmaf_rn(dtdy, fdiff4(fy[v]), __fmul_rn(dtdx, fdiff4(fx[v]))));
+        else
+            div = dtdx * fdiff(odr, fx[v][0], fx[v][1], fx[v][2], fx[v][3])
+                  + dtdy * fdiff(odr, fy[v][0], fy[v][1], fy[v][2], fy[v][3])
+                  + dtdz * fdiff(odr, fz[v][0], fz[v][1], fz[v][2], fz[v][3]);
         if constexpr (F64) {
             const double w = u[v] - to_f64(div);
             out[v] = rk.first ? w : rd.ra * u0[v] + rd.rb * w;
@@ -793,9 +846,9 @@ ks_update(PlainFields f, SplitPtrs g, Dims d, int odr, RkFF rk, RkF64 rd, float 
     // converted FP32 values and their products with dt/dx are rounded to 53
     // bits, so the discrete divergence of the B increment cancels to FP64
     // round-off (float-float, 48 bits, let it grow some 30 times faster).
-    const double b5 = u[5] - rd.ddy * df_f64(odr, ezy) + rd.ddz * df_f64(odr, eyz);
-    const double b6 = u[6] - rd.ddz * df_f64(odr, exz) + rd.ddx * df_f64(odr, ezx);
-    const double b7 = u[7] - rd.ddx * df_f64(odr, eyx) + rd.ddy * df_f64(odr, exy);
+    const double b5 = curl(u[5], rd.ddy, df_f64(odr, ezy), rd.ddz, df_f64(odr, eyz));
+    const double b6 = curl(u[6], rd.ddz, df_f64(odr, exz), rd.ddx, df_f64(odr, ezx));
+    const double b7 = curl(u[7], rd.ddx, df_f64(odr, eyx), rd.ddy, df_f64(odr, exy));
     out[5] = rk.first ? b5 : rd.ra * u0[5] + rd.rb * b5;
     out[6] = rk.first ? b6 : rd.ra * u0[6] + rd.rb * b6;
     out[7] = rk.first ? b7 : rd.ra * u0[7] + rd.rb * b7;
@@ -1088,8 +1141,7 @@ struct StepCtx {
     explicit StepCtx(Sim *sim)
         : s(sim), d{sim->g.nx, sim->g.ny, sim->g.nz, sim->g.ox, sim->g.oy, sim->g.oz, sim->sp->px},
           cb(128), cg(blocks_for((long long)sim->g.nx * sim->g.ny, 128), sim->g.nz),
-          ug(blocks_for(sim->g.nx - 2 * sim->g.ox, 128), sim->g.ny - 2 * sim->g.oy,
-             sim->g.nz - 2 * sim->g.oz)
+          ug(blocks_for((long long)(sim->g.nx - 2 * sim->g.ox) * (sim->g.ny - 2 * sim->g.oy), 128))
     {
     }
     // primitive recovery of planes [k0, k0 + nk)
@@ -1125,7 +1177,8 @@ struct StepCtx {
     }
     void emf(int k0, int nk) const
     {
-        ks_emf<<<dim3(cg.x, nk), cb, 0, s->stream>>>(s->sp->p, d, s->odr, k0);
+        auto kern = s->odr == 4 ? ks_emf<4> : ks_emf<0>;
+        kern<<<dim3(cg.x, nk), cb, 0, s->stream>>>(s->sp->p, d, s->odr, k0);
     }
     // RK combine + CT curl of the interior planes [k0, k0 + nk)
     void update(int rk, double dt, int k0, int nk) const
@@ -1138,8 +1191,10 @@ struct StepCtx {
         const double c24 = lin_odr(s->odr) > 2 ? 1.0 / 24.0 : 1.0;
         const RkFF c{host_ff(ra), host_ff(rb), ra == 0.0 && rb == 1.0};
         const RkF64 c64{ra, rb, dt / G.dx * c24, dt / G.dy * c24, dt / G.dz * c24};
-        auto kern = s->sp->f64 ? ks_update<true> : ks_update<false>;
-        kern<<<dim3(ug.x, ug.y, nk), cb, 0, s->stream>>>(
+        const bool o4 = s->odr == 4;
+        auto kern = s->sp->f64 ? (o4 ? ks_update<true, 4> : ks_update<true, 0>)
+                               : (o4 ? ks_update<false, 4> : ks_update<false, 0>);
+        kern<<<dim3(ug.x, nk), cb, 0, s->stream>>>(
             s->f, s->sp->p, d, s->odr, c, c64, (float)(dt / G.dx), (float)(dt / G.dy),
             (float)(dt / G.dz), !s->walls3d, k0);
         if (s->walls3d && k0 + nk == G.nz - G.oz) {
