@@ -28,6 +28,10 @@ struct BInst {
     int active, steps;
     int status, pad;  // status: 1 once a NaN or non-positive density/pressure was seen
     unsigned long long vkey;  // order-preserving key of this step's max speed
+    // 2D instances, formed once a step (batch_dt): dt/dx and dt/dy, the same with
+    // the 4th-order stencil's 1/24, and in FP32
+    double rdx, rdy, cdx, cdy;
+    float fdx, fdy;
     // 2D boundary tables (the problem's dnxs / dnys: 0 periodic, -1 Dirichlet,
     // +1 Neumann per variable), walls: some entry is not periodic
     int walls, pad2;
@@ -41,7 +45,8 @@ struct BSync {
     int err, active_left;
     int ntiles, fresh;  // fresh: some 1D instance still needs its one-off dt
     BTile *tiles;
-    int walls, pad;      // some active 2D instance has non-periodic tables
+    int walls;           // some active 2D instance has non-periodic tables
+    int pad;
 };
 
 struct BArrays {
@@ -49,6 +54,8 @@ struct BArrays {
     // FP32-split workspace
     float2 *q[8];  // ro, vx, vy, vz, cx, cy, bz, pr as (hi, lo)
     float *bf[2], *m2f, *ctf, *dvf[2];
+    // fluxes and their central parts, before them the faces' left states; right
+    // states along x (ulf) and y (urf)
     float *ulf[8], *urf[8], *Ff[2][7], *FCf[2], *ezf;
     // FP64 plain workspace
     double *vx, *vy, *vz, *pr, *m2, *cx, *cy, *ct, *dv[2];
@@ -133,7 +140,10 @@ __device__ __forceinline__ long long bsrc(const BInst &I, int i, int j, int stx,
            bc_src(i, I.nx, I.off, stx, dnx, g);
 }
 
-// Visit every cell of every active instance's tiles; body(I, i, j, c).
+// Visit every cell of every active instance's tiles; body(I, i, j, c).  A block
+// has the same tiles in every phase, which finds them in its L1 and its side of
+// the L2: handing tiles out as blocks finish, or shifting them from round to
+// round, evens the blocks out and is slower (873 -> 964 and 900 us a step).
 template <class Body>
 __device__ __forceinline__ void for_cells(const BArgs &A, int ntiles, const BTile *tiles, Body body)
 {
@@ -149,9 +159,9 @@ __device__ __forceinline__ void for_cells(const BArgs &A, int ntiles, const BTil
 }
 
 // Record a bad cell state (NaN, or density or pressure not positive).
-__device__ __forceinline__ void batch_check(BInst &I, double ro, double pr)
+template <class T> __device__ __forceinline__ void batch_check(BInst &I, T ro, T pr)
 {
-    if (!(ro > 0.0) || !(pr > 0.0)) atomicOr(&I.status, 1);
+    if (!(ro > T(0)) || !(pr > T(0))) atomicOr(&I.status, 1);
 }
 
 // dt of every active instance: fixed, or cfl*min(dx,dy)/vmax; clipped to
@@ -175,6 +185,13 @@ __device__ __forceinline__ void batch_dt(const BArgs &A)
         }
         if (I.t + dt > I.t_end) dt = I.t_end - I.t;
         I.dt = dt;
+        const double c24 = lin_odr(A.odr) > 2 ? 1.0 / 24.0 : 1.0;
+        I.rdx = dt / I.dx;
+        I.rdy = dt / I.dy;
+        I.cdx = I.rdx * c24;
+        I.cdy = I.rdy * c24;
+        I.fdx = (float)I.rdx;
+        I.fdy = (float)I.rdy;
     }
 }
 
@@ -194,19 +211,21 @@ __device__ __forceinline__ void batch_advance(const BArgs &A)
     }
 }
 
-// Block max of a non-negative speed, folded into the instance's key.
-__device__ __forceinline__ void batch_vmax(BInst &I, double vt)
+// Block max of a speed, which is not negative or NaN, folded into the instance's
+// key.  Such values order as their bits, so the FP64 pipe stays out of it.
+__device__ __forceinline__ void batch_vmax(BInst &I, double v)
 {
-    __shared__ double red[32];
+    __shared__ unsigned long long red[32];
+    unsigned long long vt = (unsigned long long)__double_as_longlong(v);
     const int lin = threadIdx.y * blockDim.x + threadIdx.x;
     const int lane = lin & 31, wid = lin >> 5, nw = (blockDim.x * blockDim.y) >> 5;
-    for (int o = 16; o > 0; o >>= 1) vt = fmax(vt, __shfl_xor_sync(0xffffffffu, vt, o));
+    for (int o = 16; o > 0; o >>= 1) vt = max(vt, __shfl_xor_sync(0xffffffffu, vt, o));
     if (lane == 0) red[wid] = vt;
     __syncthreads();
     if (wid == 0) {
-        vt = lane < nw ? red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) vt = fmax(vt, __shfl_xor_sync(0xffffffffu, vt, o));
-        if (lane == 0 && vt > 0.0) atomicMax(&I.vkey, (unsigned long long)__double_as_longlong(vt));
+        vt = lane < nw ? red[lane] : 0ull;
+        for (int o = 16; o > 0; o >>= 1) vt = max(vt, __shfl_xor_sync(0xffffffffu, vt, o));
+        if (lane == 0 && vt > 0ull) atomicMax(&I.vkey, vt);
     }
     __syncthreads();
 }

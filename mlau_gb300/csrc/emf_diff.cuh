@@ -43,7 +43,7 @@ X64 int clz64(uint64_t v)
 #endif
 }
 
-X64_SLOW double emf_diff4_slow(float e0, float e1, float e2, float e3)
+static X64_SLOW double emf_diff4_slow(float e0, float e1, float e2, float e3)
 {
     return 27.0 * ((double)e2 - (double)e1) - ((double)e3 - (double)e0);
 }
