@@ -40,6 +40,7 @@ UNITS = {
     "batch1d_plain.cu": EXACT,
     "dataio.cu": EXACT,
     "diff2d.cu": EXACT,
+    "hostcopy.cu": EXACT,
     "cxx_linkage.cpp": [],
 }
 

@@ -8,6 +8,7 @@
 #include <mutex>
 
 #include "sim.cuh"
+#include "hostcopy.h"
 
 namespace mlau {
 
@@ -191,28 +192,23 @@ int mlau_sim_destroy(mlau_sim *s)
     return MLAU_OK;
 }
 
-static int nvars(const Sim *) { return 8; }
-
-int mlau_sim_upload(mlau_sim *s, const double *const *h)
+static int upload(mlau_sim *s, const double *const *h, bool wait)
 {
     if (!s || !h) { set_error("null argument"); return MLAU_ERR_ARG; }
-    for (int v = 0; v < nvars(s); v++) {
-        if ((s->g.dim == 1 && v == 5) || !h[v]) continue;
-        MLAU_CUDA(cudaMemcpyAsync(s->f.s[v], h[v], sizeof(double) * s->g.n,
-                                  cudaMemcpyHostToDevice, s->stream));
-    }
-    return MLAU_OK;
+    double *host[8];
+    for (int v = 0; v < 8; v++) host[v] = s->g.dim == 1 && v == 5 ? nullptr : const_cast<double *>(h[v]);
+    return copy_fields(s->f.s, host, 8, s->g.n, false, wait, s->stream);
 }
+
+int mlau_sim_upload(mlau_sim *s, const double *const *h) { return upload(s, h, true); }
 
 int mlau_sim_download(mlau_sim *s, double *const *h)
 {
     if (!s || !h) { set_error("null argument"); return MLAU_ERR_ARG; }
-    for (int v = 0; v < nvars(s); v++) {
-        if ((s->g.dim == 1 && v == 5) || !h[v]) continue;
-        MLAU_CUDA(cudaMemcpyAsync(h[v], s->f.s[v], sizeof(double) * s->g.n,
-                                  cudaMemcpyDeviceToHost, s->stream));
-    }
-    MLAU_CUDA(cudaStreamSynchronize(s->stream));
+    double *host[8];
+    for (int v = 0; v < 8; v++) host[v] = s->g.dim == 1 && v == 5 ? nullptr : h[v];
+    const int rc = copy_fields(s->f.s, host, 8, s->g.n, true, true, s->stream);
+    if (rc != MLAU_OK) return rc;
     return s->sp ? split3d_check(s) : MLAU_OK;
 }
 
@@ -597,9 +593,10 @@ int run_dropin(mlau_sim *c, double *const *h, double dt)
 {
     // FP32-split: the host link's copies overlap the step where the data allow
     if (c->sp && !c->walls3d) return split3d_step_host(c, dt, h);
-    int rc = mlau_sim_upload(c, (const double *const *)h);
+    int rc = upload(c, (const double *const *)h, false);
     if (rc == MLAU_OK) rc = mlau_sim_step(c, dt, 1);
     if (rc == MLAU_OK) rc = mlau_sim_download(c, h);
+    else cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read
     return rc;
 }
 
@@ -758,7 +755,7 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
     const int *tx = dnxs, *ty = dnys;
     mlau_sim *c = get_ctx(2, nx, ny, 1, xoff, yoff, 0, dx, dy, 1.0, gamma);
     int rc = c ? mlau_sim_set_bc_2d(c, tx, ty) : MLAU_ERR_NOMEM;
-    if (rc == MLAU_OK) rc = mlau_sim_upload(c, (const double *const *)h);
+    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, false);
     if (rc == MLAU_OK) {
         if (op == MRX_RESISTIVE) rc = diff2d_resistive(c, coef, dt);
         else if (op == MRX_VISCOUS) rc = diff2d_viscous(c, coef, dt);
@@ -769,6 +766,8 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
         for (int v = 0; v < 8; v++) out[v] = back[v] ? h[v] : nullptr;
         const int rd = mlau_sim_download(c, out);
         if (rd != MLAU_OK) rc = rd;
+    } else if (c) {
+        cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read
     }
     if (rc != MLAU_OK && rc != MLAU_ERR_CONVERGE) report(who);
     return rc;

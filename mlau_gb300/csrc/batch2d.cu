@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "batch2d.cuh"
+#include "hostcopy.h"
 
 using namespace mlau;
 
@@ -249,6 +250,17 @@ int make_graph(mlau_batch *b, int steps)
     return MLAU_OK;
 }
 
+// An instance's state to the host or from it.
+int move_fields(mlau_batch *b, const BInst &I, double *const *host, bool to_host)
+{
+    double *dev[8];
+    for (int v = 0; v < 8; v++) dev[v] = b->a.s[v] ? b->a.s[v] + I.base : nullptr;
+    const int rc = copy_fields(dev, host, 8, (long long)I.nx * I.ny, to_host, true, b->stream);
+    if (rc != MLAU_OK) return rc;
+    MLAU_CUDA(cudaStreamSynchronize(b->stream));
+    return MLAU_OK;
+}
+
 int check_inst(mlau_batch *b, int n)
 {
     if (!b || n < 0 || n >= b->max_inst || !b->used[n]) {
@@ -403,6 +415,11 @@ int mlau_batch_add(mlau_batch *b, int nx, int ny, double dx, double dy, double g
         set_error("batch: bad instance");
         return MLAU_ERR_ARG;
     }
+    for (int v = 0; v < 8; v++)
+        if (!host8[v]) {
+            set_error("batch: missing state array %d", v);
+            return MLAU_ERR_ARG;
+        }
     int n = -1;
     for (int k = 0; k < b->max_inst; k++)
         if (!b->used[k]) { n = k; break; }
@@ -425,11 +442,8 @@ int mlau_batch_add(mlau_batch *b, int nx, int ny, double dx, double dy, double g
     b->h_inst[n] = I;
     b->used[n] = 1;
     b->tiles_dirty = true;
-    const size_t bytes = sizeof(double) * cells;
-    for (int v = 0; v < 8; v++)
-        MLAU_CUDA(cudaMemcpyAsync(b->a.s[v] + base, host8[v], bytes, cudaMemcpyHostToDevice,
-                                  b->stream));
-    MLAU_CUDA(cudaStreamSynchronize(b->stream));
+    const int rc = move_fields(b, I, const_cast<double *const *>(host8), false);
+    if (rc != MLAU_OK) return rc;
     *slot = n;
     return MLAU_OK;
 }
@@ -472,11 +486,8 @@ int mlau_batch1d_add(mlau_batch *b, int nx, double dx, double bx, double gamma, 
     b->h_inst[n] = I;
     b->used[n] = 1;
     b->tiles_dirty = true;
-    for (int v = 0; v < 8; v++)
-        if (v != 5)
-            MLAU_CUDA(cudaMemcpyAsync(b->a.s[v] + base, host8[v], sizeof(double) * nx,
-                                      cudaMemcpyHostToDevice, b->stream));
-    MLAU_CUDA(cudaStreamSynchronize(b->stream));
+    const int rc = move_fields(b, I, const_cast<double *const *>(host8), false);
+    if (rc != MLAU_OK) return rc;
     *slot = n;
     return MLAU_OK;
 }
@@ -517,27 +528,13 @@ int mlau_batch_create(mlau_batch **out, int ninst, const int *nx, const int *ny,
 int mlau_batch_upload(mlau_batch *b, int n, const double *const *h)
 {
     if (!check_inst(b, n) || !h) return MLAU_ERR_ARG;
-    const BInst &I = b->h_inst[n];
-    const size_t bytes = sizeof(double) * I.nx * I.ny;
-    for (int v = 0; v < 8; v++)
-        if (b->a.s[v] && h[v])
-            MLAU_CUDA(cudaMemcpyAsync(b->a.s[v] + I.base, h[v], bytes, cudaMemcpyHostToDevice,
-                                      b->stream));
-    MLAU_CUDA(cudaStreamSynchronize(b->stream));
-    return MLAU_OK;
+    return move_fields(b, b->h_inst[n], const_cast<double *const *>(h), false);
 }
 
 int mlau_batch_download(mlau_batch *b, int n, double *const *h)
 {
     if (!check_inst(b, n) || !h) return MLAU_ERR_ARG;
-    const BInst &I = b->h_inst[n];
-    const size_t bytes = sizeof(double) * I.nx * I.ny;
-    for (int v = 0; v < 8; v++)
-        if (b->a.s[v] && h[v])
-            MLAU_CUDA(cudaMemcpyAsync(h[v], b->a.s[v] + I.base, bytes, cudaMemcpyDeviceToHost,
-                                      b->stream));
-    MLAU_CUDA(cudaStreamSynchronize(b->stream));
-    return MLAU_OK;
+    return move_fields(b, b->h_inst[n], h, true);
 }
 
 int mlau_batch_set_bc(mlau_batch *b, int n, const int *dnx, const int *dny)

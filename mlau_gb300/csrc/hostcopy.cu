@@ -1,0 +1,112 @@
+// Host arrays to and from the device in one launch.
+//
+// A call of a driver on host arrays moves up to eight arrays each way, and a
+// copy from or to pageable memory costs 2 to 10 us of the driver's time (staging
+// and, to the host, waiting) before its bytes count: more than the step itself
+// for small grids.  Where the GPU reaches pageable host memory through the
+// host's page tables (Grace and Blackwell share them over NVLink-C2C) a kernel
+// reads and writes the arrays where they are.  Eight arrays there / back, copies
+// against the kernel: 2056 doubles each 23 / 66 against 11 / 10 us, 26624 79 / 74
+// against 18 / 19, 327352 198 / 178 against 113 / 129; at 4.7M doubles
+// 1782 / 1649 against 1512 / 1791, so arrays above 4 MB are copied, as are
+// device or managed arrays and where the GPU cannot reach host memory.
+#include <algorithm>
+
+#include "hostcopy.h"
+
+namespace mlau {
+namespace {
+
+struct Fields8 {
+    const double *src[8];
+    double *dst[8];
+};
+
+constexpr long long kKernelBytes = 4 << 20;  // the largest array the kernel moves
+
+// Array blockIdx.y, by pairs where both sides are aligned for it.
+__global__ void __launch_bounds__(256) k_copy8(const __grid_constant__ Fields8 a, long long n)
+{
+    const double *s = a.src[blockIdx.y];
+    double *d = a.dst[blockIdx.y];
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    if ((((unsigned long long)s | (unsigned long long)d) & 15) == 0) {
+        for (long long i = t; i < n / 2; i += nt)
+            reinterpret_cast<double2 *>(d)[i] = reinterpret_cast<const double2 *>(s)[i];
+        if (t == 0 && (n & 1)) d[n - 1] = s[n - 1];
+    } else {
+        for (long long i = t; i < n; i += nt) d[i] = s[i];
+    }
+}
+
+bool reaches_host_memory()
+{
+    int dev = 0, direct = 0, tables = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) ==
+               cudaSuccess &&
+           direct && tables;
+}
+
+// 2: ordinary host memory, 1: pinned; 0: anything else, or not aligned for a double
+int host_array(const void *p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if ((unsigned long long)p & 7) return 0;
+    return at.type == cudaMemoryTypeUnregistered ? 2 : at.type == cudaMemoryTypeHost ? 1 : 0;
+}
+
+// Have the pages of a host array there before the GPU writes to them: it would
+// wait for each (the bytes stay as they are).
+void touch(double *p, long long n)
+{
+    volatile char *b = (volatile char *)p;
+    const long long bytes = n * (long long)sizeof(double);
+    for (long long i = 0; i < bytes; i += 4096) b[i] = b[i];
+    b[bytes - 1] = b[bytes - 1];
+}
+
+}  // namespace
+
+int copy_fields(double *const *dev, double *const *host, int nv, long long n, bool to_host, bool wait,
+                cudaStream_t st)
+{
+    Fields8 a{};
+    int m = 0, kind = 0;
+    bool kernel = n > 0 && (long long)sizeof(double) * n <= kKernelBytes && nv <= 8 && reaches_host_memory();
+    for (int v = 0; v < nv && kernel; v++) {
+        if (!dev[v] || !host[v]) continue;
+        const int k = host_array(host[v]);
+        kernel = k != 0;
+        kind = std::max(kind, k);
+        // arrays that overlap are written one after the other
+        for (int w = 0; w < v && to_host; w++)
+            if (dev[w] && host[w] && host[w] < host[v] + n && host[v] < host[w] + n) kernel = false;
+        a.src[m] = to_host ? dev[v] : host[v];
+        a.dst[m++] = to_host ? host[v] : dev[v];
+    }
+    if (kernel) {
+        if (m == 0) return MLAU_OK;
+        for (int v = 0; v < m && to_host; v++) touch(a.dst[v], n);
+        const unsigned nb = (unsigned)std::min(152LL, (n / 2 + 255) / 256 + 1);
+        k_copy8<<<dim3(nb, m), 256, 0, st>>>(a, n);
+        MLAU_CUDA(cudaGetLastError());
+        // a copy from ordinary memory has read it when it returns
+        if (wait && (to_host || kind == 2)) MLAU_CUDA(cudaStreamSynchronize(st));
+        return MLAU_OK;
+    }
+    for (int v = 0; v < nv; v++) {
+        if (!dev[v] || !host[v]) continue;
+        MLAU_CUDA(to_host ? cudaMemcpyAsync(host[v], dev[v], sizeof(double) * n, cudaMemcpyDeviceToHost, st)
+                          : cudaMemcpyAsync(dev[v], host[v], sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    }
+    if (wait && to_host) MLAU_CUDA(cudaStreamSynchronize(st));
+    return MLAU_OK;
+}
+
+}  // namespace mlau
