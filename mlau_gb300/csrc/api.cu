@@ -113,7 +113,7 @@ int launches_per_step(const Sim *s)
     // kernels per RK stage (device-to-device copies are not counted)
     if (s->sp) return s->nrk * (s->walls3d ? 9 : 7);
     if (s->g.dim == 3) return s->nrk * (s->walls3d ? 12 : 10);
-    if (s->g.dim == 2) return s->nrk * (s->walls2d ? 10 : 8);
+    if (s->g.dim == 2) return s->nrk * (s->walls2d ? 8 : 6);
     return s->nrk;  // 1D: one per stage
 }
 

@@ -455,19 +455,19 @@ __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double
     }
 }
 
-constexpr int FXT = 256;  // threads of a flux block
-template <int WHICH> constexpr size_t fx_smem()
+// shared memory of a block of NT threads
+template <int WHICH, int NT> constexpr size_t fx_smem()
 {
-    return sizeof(double) * 2 * (WHICH == FLUX_MLAU ? (int)FX_ROWS : (int)HX_ROWS) * FXT;
+    return sizeof(double) * 2 * (WHICH == FLUX_MLAU ? (int)FX_ROWS : (int)HX_ROWS) * NT;
 }
 
 // riemann (point.cuh) of one face.
-template <int WHICH, int ND, class LOAD>
-__device__ __forceinline__ void riemann_ed(LOAD IN, double (*rows)[FXT], double bn, double gamma, double dv0,
+template <int WHICH, int ND, int NT, class LOAD>
+__device__ __forceinline__ void riemann_ed(LOAD IN, double (*rows)[NT], double bn, double gamma, double dv0,
                                            const double dv[ND], double f[7])
 {
-    if constexpr (WHICH == FLUX_MLAU) flux_mlau_ed<ND, FXT>(IN, rows, bn, gamma, dv0, dv, f);
-    else flux_hlld_ed<WHICH == FLUX_LHLLD, ND, FXT>(IN, rows, bn, gamma, dv0, dv, f);
+    if constexpr (WHICH == FLUX_MLAU) flux_mlau_ed<ND, NT>(IN, rows, bn, gamma, dv0, dv, f);
+    else flux_hlld_ed<WHICH == FLUX_LHLLD, ND, NT>(IN, rows, bn, gamma, dv0, dv, f);
 }
 
 }  // namespace mlau

@@ -18,7 +18,7 @@ namespace {
 // boundary source times the table's sign (calc_bc then bc2d with dnxs[5..6],
 // :186-200).
 __global__ void __launch_bounds__(TPB)
-k_prim2(PlainFields f, Dims d, Box b, int odr, double gamma, Bc2 bc)
+k_prim2(PlainFields f, Dims d, Box b, int odr, double gamma, Bc2 bc, int save_u0)
 {
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
@@ -31,6 +31,9 @@ k_prim2(PlainFields f, Dims d, Box b, int odr, double gamma, Bc2 bc)
     const ed cx = ed(gx) * face2cen<ed>(odr, bx[wx - 1], bx[wx], bx[wx + 1], bx[wx + 2]);
     const ed cy = ed(gy) * face2cen<ed>(odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
     const long long s = d.at(i, j, 0);
+    if (save_u0)  // the first stage keeps U^n
+#pragma unroll
+        for (int v = 0; v < 8; v++) f.u0[v][s] = f.s[v][s];
     const ed ro = f.s[0][s];
     const ed iro = trcp(ro);
     const ed vx = f.s[1][s] * iro, vy = f.s[2][s] * iro, vz = f.s[3][s] * iro;
@@ -67,22 +70,48 @@ __global__ void __launch_bounds__(TPB) k_aux2(PlainFields f, Dims d, Box b, Bc2 
 
 // Sweep along x (D=0): (vn, vt, vu) = (vx, vy, vz), (bt, bu) = (cy, bz), the
 // By flux is split.  Along y (D=1): (vy, vz, vx), (bz, cx), the Bx flux is split.
-struct View2 {
+// Both sweeps run in one launch, side by side (blockIdx.y), so that grids of a
+// few thousand cells have twice the warps to hide each other's latency (200 x 120
+// cells, a step: LHLLD + MUSCL 425 -> 268 us, MLAU + WCNS4 627 -> 413).  A face's
+// left state lies where its flux goes.
+struct Sweep2 {
     const double *vn, *vt, *vu, *cn, *ct, *cu, *bface, *dvt;
+    double *ul[7], *ur[7], *ql, *qr;  // face states, central parts of the split flux
+    Box rec, flux;                    // cells reconstructed, faces
+    long long st;
     int split_u;  // 0: split the bt flux; 1: split the bu flux
 };
+struct Sweeps2 {
+    Sweep2 s[2];
+};
 
-View2 make_view2(const PlainFields &f, int D)
+Sweeps2 make_sweeps2(const PlainFields &f, const Geometry &g)
 {
-    if (D == 0) return {f.vx, f.vy, f.vz, f.cx, f.cy, f.s[7], f.s[5], f.dv[1], 0};
-    return {f.vy, f.vz, f.vx, f.cy, f.s[7], f.cx, f.s[6], f.dv[0], 1};
+    Sweeps2 S{};
+    Sweep2 &x = S.s[0], &y = S.s[1];
+    x = {f.vx, f.vy, f.vz, f.cx, f.cy, f.s[7], f.s[5], f.dv[1]};
+    y = {f.vy, f.vz, f.vx, f.cy, f.s[7], f.cx, f.s[6], f.dv[0]};
+    y.split_u = 1;
+    for (int D = 0; D < 2; D++) {
+        for (int n = 0; n < 7; n++) S.s[D].ul[n] = f.F[D][n];
+        for (int n = 0; n < 7; n++) S.s[D].ur[n] = D ? f.ur[n] : f.ul[n];
+        S.s[D].ql = f.FC[D][0];
+        S.s[D].qr = D ? f.qr[0] : f.ql[0];
+    }
+    x.st = 1;
+    y.st = g.nx;
+    x.rec = {2, 0, 0, g.nx - 4, g.ny, 1};
+    x.flux = {3, 0, 0, g.nx - 5, g.ny, 1};
+    y.rec = {0, 2, 0, g.nx, g.ny - 4, 1};
+    y.flux = {0, 3, 0, g.nx, g.ny - 5, 1};
+    return S;
 }
 
 // The linear interpolation of the central part of the split tangential B flux.
-__device__ __forceinline__ void rec_central2(const PlainFields &f, const View2 &v, long long c,
-                                             long long st, int odr)
+__device__ __forceinline__ void rec_central2(const Sweep2 &v, long long c, int odr)
 {
     const double *bt = v.split_u ? v.cu : v.ct, *vt = v.split_u ? v.vu : v.vt;
+    const long long st = v.st;
     ed a5[5], t5[5];
 #pragma unroll
     for (int m = 0; m < 5; m++) {
@@ -90,17 +119,19 @@ __device__ __forceinline__ void rec_central2(const PlainFields &f, const View2 &
         a5[m] = imul(bt[s], v.vn[s]);
         t5[m] = vt[s];
     }
-    f.ql[0][c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                      - ed(v.bface[c + st]) * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
-    f.qr[0][c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
-                 - ed(v.bface[c]) * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    v.ql[c + st] = (lin_l(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+                    - ed(v.bface[c + st]) * lin_l(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
+    v.qr[c] = (lin_r(odr, a5[0], a5[1], a5[2], a5[3], a5[4])
+               - ed(v.bface[c]) * lin_r(odr, t5[0], t5[1], t5[2], t5[3], t5[4])).v;
 }
 
 __global__ void __launch_bounds__(TPB)
-k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, double gamma)
+k_rec2(PlainFields f, const __grid_constant__ Sweeps2 S, Dims d, int odr, int eig, double gamma)
 {
+    const Sweep2 &v = S.s[blockIdx.y];
+    const long long st = v.st;
     int i, j, k;
-    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    if (!v.rec.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
     ed q[7][5];
 #pragma unroll
@@ -119,48 +150,52 @@ k_rec2(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, int eig, do
                      ul, ur);
 #pragma unroll
     for (int n = 0; n < 7; n++) {
-        f.ul[n][c + st] = ul[n].v;
-        f.ur[n][c] = ur[n].v;
+        v.ul[n][c + st] = ul[n].v;
+        v.ur[n][c] = ur[n].v;
     }
-    rec_central2(f, v, c, st, odr);
+    rec_central2(v, c, odr);
 }
 
-constexpr int RCT = 128;  // threads of a k_rec2_ed block
-
-// The drivers' eigen-systems (rec_exact.cuh); W4: WCNS4, else the code odr.
-template <bool W4>
-__global__ void __launch_bounds__(RCT, 5)
-k_rec2_ed(PlainFields f, View2 v, Dims d, Box b, long long st, int odr, double gamma)
+// The drivers' eigen-systems (rec_exact.cuh); W4: WCNS4, else the code odr;
+// blocks of NT threads.
+template <bool W4, int NT>
+__global__ void __launch_bounds__(NT, 640 / NT)
+k_rec2_ed(PlainFields f, const __grid_constant__ Sweeps2 S, Dims d, int odr, double gamma)
 {
     extern __shared__ double rec_rows[];
-    double (*w)[RCT] = (double (*)[RCT])rec_rows;
+    double (*w)[NT] = (double (*)[NT])rec_rows;
+    const Sweep2 &v = S.s[blockIdx.y];
+    const long long st = v.st;
     int i, j, k;
-    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    if (!v.rec.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
     const double *src[7] = {f.s[0], v.vn, v.vt, v.vu, v.ct, v.cu, f.pr};
     auto Q = [&](int n, int m) { return src[n][c + st * (m - 2)]; };
     const bool full = vmax(f.m2[c - st], vmax(f.m2[c], f.m2[c + st])) >= 1.0;
-    auto PUT = [&](int s, int n, double u) { (s ? f.ur : f.ul)[n][s ? c : c + st] = u; };
-    reconst_ed<W4, RCT>(odr, Q, full, v.cn[c], gamma, RecScratch<RCT>{w, (int)threadIdx.x}, PUT);
-    rec_central2(f, v, c, st, W4 ? 4 : odr);
+    auto PUT = [&](int s, int n, double u) { (s ? v.ur : v.ul)[n][s ? c : c + st] = u; };
+    reconst_ed<W4, NT>(odr, Q, full, v.cn[c], gamma, RecScratch<NT>{w, (int)threadIdx.x}, PUT);
+    rec_central2(v, c, W4 ? 4 : odr);
 }
 
 __global__ void __launch_bounds__(TPB)
-k_flux2(PlainFields f, View2 v, Dims d, Box b, long long st, int D, int which, double gamma)
+k_flux2(PlainFields f, const __grid_constant__ Sweeps2 S, Dims d, int which, double gamma)
 {
+    const int D = blockIdx.y;
+    const Sweep2 &v = S.s[D];
+    const long long st = v.st;
     int i, j, k;
-    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    if (!v.flux.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
     ed L[7], R[7], F[7];
 #pragma unroll
     for (int n = 0; n < 7; n++) {
-        L[n] = f.ul[n][c];
-        R[n] = f.ur[n][c];
+        L[n] = v.ul[n][c];
+        R[n] = v.ur[n][c];
     }
     const ed bn = ed(0.5) * (ed(v.bface[c]) + v.bface[c]);
     riemann<ed>(which, L, R, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]),
                 vmin(v.dvt[c - st], v.dvt[c]), F);
-    const ed fc = ed(0.5) * (ed(f.ql[0][c]) + f.qr[0][c]);
+    const ed fc = ed(0.5) * (ed(v.ql[c]) + v.qr[c]);
     F[4 + v.split_u] -= fc;
 #pragma unroll
     for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n].v;
@@ -168,25 +203,61 @@ k_flux2(PlainFields f, View2 v, Dims d, Box b, long long st, int D, int which, d
 }
 
 // MLAU, LHLLD and HLLD faces on both pipes (flux_exact.cuh).
-template <int WHICH>
-__global__ void __launch_bounds__(FXT, 2)
-k_flux2_ed(PlainFields f, View2 v, Dims d, Box b, long long st, int D, double gamma)
+template <int WHICH, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
+k_flux2_ed(PlainFields f, const __grid_constant__ Sweeps2 S, Dims d, double gamma)
 {
     extern __shared__ double fx_rows[];
+    const int D = blockIdx.y;
+    const Sweep2 &v = S.s[D];
+    const long long st = v.st;
     int i, j, k;
-    if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    if (!v.flux.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long c = d.at(i, j, 0);
-    auto IN = [&](int s, int n) { return (s ? f.ur : f.ul)[n][c]; };
+    auto IN = [&](int s, int n) { return (s ? v.ur : v.ul)[n][c]; };
     const double dv[2] = {v.dvt[c - st], v.dvt[c]};
     const double bn = (ed(0.5) * (ed(v.bface[c]) + v.bface[c])).v;
     double F[7];
-    riemann_ed<WHICH, 2>(IN, (double (*)[FXT])fx_rows, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]).v, dv, F);
-    const ed fc = ihalf(ed(f.ql[0][c]) + f.qr[0][c]);
+    riemann_ed<WHICH, 2, NT>(IN, (double (*)[NT])fx_rows, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]).v, dv, F);
+    const ed fc = ihalf(ed(v.ql[c]) + v.qr[c]);
     if (v.split_u) F[5] = (F[5] - fc).v;
     else F[4] = (F[4] - fc).v;
 #pragma unroll
     for (int n = 0; n < 7; n++) f.F[D][n][c] = F[n];
     f.FC[D][0][c] = fc.v;
+}
+
+// Reconstruction and fluxes of both sweeps.  Blocks are large for the sake of the
+// instruction caches, which a block's warps share, and small where the grid is
+// less than what the GPU holds at a time, so that it spreads evenly (200 x 120
+// cells, a step of LHLLD + MUSCL: 268 us with blocks of 32, 273 of 64, 289 of 128
+// and 256; 300 x 300: no difference beyond 2 %).
+constexpr long long kSmall2 = 97280;  // threads: 5 reconstruction blocks of 128 on each SM
+
+template <int NR> void launch_rec2(Sim *s, const Sweeps2 &S, const Dims &d)
+{
+    const long long n = std::max(S.s[0].rec.count(), S.s[1].rec.count());
+    if (s->eig != EIG_FULL)
+        k_rec2<<<dim3(blocks_for(n, TPB), 2), TPB, 0, s->stream>>>(s->f, S, d, s->odr, s->eig, s->gamma);
+    else if (s->odr == 4)
+        k_rec2_ed<true, NR><<<dim3(blocks_for(n, NR), 2), NR, rec_smem<NR>(), s->stream>>>(s->f, S, d, 4, s->gamma);
+    else
+        k_rec2_ed<false, NR><<<dim3(blocks_for(n, NR), 2), NR, rec_smem<NR>(), s->stream>>>(s->f, S, d, s->odr,
+                                                                                         s->gamma);
+}
+
+template <int NF> void launch_flux2(Sim *s, const Sweeps2 &S, const Dims &d)
+{
+    const long long n = std::max(S.s[0].flux.count(), S.s[1].flux.count());
+    const dim3 g(blocks_for(n, NF), 2);
+    if (s->flux == FLUX_MLAU)
+        k_flux2_ed<FLUX_MLAU, NF><<<g, NF, fx_smem<FLUX_MLAU, NF>(), s->stream>>>(s->f, S, d, s->gamma);
+    else if (s->flux == FLUX_LHLLD)
+        k_flux2_ed<FLUX_LHLLD, NF><<<g, NF, fx_smem<FLUX_LHLLD, NF>(), s->stream>>>(s->f, S, d, s->gamma);
+    else if (s->flux == FLUX_HLLD)
+        k_flux2_ed<FLUX_HLLD, NF><<<g, NF, fx_smem<FLUX_HLLD, NF>(), s->stream>>>(s->f, S, d, s->gamma);
+    else
+        k_flux2<<<dim3(blocks_for(n, TPB), 2), TPB, 0, s->stream>>>(s->f, S, d, s->flux, s->gamma);
 }
 
 __global__ void __launch_bounds__(TPB) k_emf2(PlainFields f, Dims d, Box b, int odr)
@@ -313,8 +384,8 @@ int plain2d_alloc(Sim *s)
         rc |= dalloc(s, &f.FC[D][0], n);
     }
     if (rc) return MLAU_ERR_NOMEM;
-    MLAU_CUDA(cudaFuncSetAttribute(k_flux2_ed<FLUX_MLAU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)fx_smem<FLUX_MLAU>()));
+    MLAU_CUDA(cudaFuncSetAttribute(k_flux2_ed<FLUX_MLAU, 256>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx_smem<FLUX_MLAU, 256>()));
     return MLAU_OK;
 }
 
@@ -324,59 +395,31 @@ int plain2d_step(Sim *s, double dt)
     PlainFields &f = s->f;
     cudaStream_t st = s->stream;
     const Dims d{g.nx, g.ny, 1, g.ox, g.oy, 0};
-    {
-        TimedLaunch tl(&s->timer, KK_COPY);
-        for (int v = 0; v < 8; v++)
-            MLAU_CUDA(cudaMemcpyAsync(f.u0[v], f.s[v], sizeof(double) * g.n,
-                                      cudaMemcpyDeviceToDevice, st));
-    }
     const Box all{0, 0, 0, g.nx, g.ny, 1};
     const Box inner{g.ox, g.oy, 0, g.nx - 2 * g.ox, g.ny - 2 * g.oy, 1};
     const double dtdx = dt / g.dx, dtdy = dt / g.dy;
+    const Sweeps2 S = make_sweeps2(f, g);
     for (int rk = 0; rk < s->nrk; rk++) {
         double ra, rb;
         rk_coef(s->nrk, rk, ra, rb);
         {
             TimedLaunch tl(&s->timer, KK_PRIM);
             k_prim2<<<blocks_for(all.count(), TPB), TPB, 0, st>>>(f, d, all, s->odr, s->gamma,
-                                                                  s->bc2);
+                                                                  s->bc2, rk == 0);
         }
         {
             TimedLaunch tl(&s->timer, KK_AUX);
             k_aux2<<<blocks_for(all.count(), TPB), TPB, 0, st>>>(f, d, all, s->bc2);
         }
-        for (int D = 0; D < 2; D++) {
-            const View2 v = make_view2(f, D);
-            const long long stride = D == 0 ? 1 : g.nx;
-            Box rb_ = all, fb = all;
-            if (D == 0) { rb_.lo0 = 2; rb_.e0 = g.nx - 4; fb.lo0 = 3; fb.e0 = g.nx - 5; }
-            else { rb_.lo1 = 2; rb_.e1 = g.ny - 4; fb.lo1 = 3; fb.e1 = g.ny - 5; }
-            {
-                TimedLaunch tl(&s->timer, KK_REC);
-                const unsigned nb = blocks_for(rb_.count(), TPB), nr = blocks_for(rb_.count(), RCT);
-                if (s->eig == EIG_FULL && s->odr == 4)
-                    k_rec2_ed<true><<<nr, RCT, rec_smem<RCT>(), st>>>(f, v, d, rb_, stride, 4, s->gamma);
-                else if (s->eig == EIG_FULL)
-                    k_rec2_ed<false><<<nr, RCT, rec_smem<RCT>(), st>>>(f, v, d, rb_, stride, s->odr, s->gamma);
-                else
-                    k_rec2<<<nb, TPB, 0, st>>>(f, v, d, rb_, stride, s->odr, s->eig, s->gamma);
-            }
-            {
-                TimedLaunch tl(&s->timer, KK_FLUX);
-                const unsigned nb = blocks_for(fb.count(), FXT);
-                if (s->flux == FLUX_MLAU)
-                    k_flux2_ed<FLUX_MLAU><<<nb, FXT, fx_smem<FLUX_MLAU>(), st>>>(f, v, d, fb, stride, D,
-                                                                                 s->gamma);
-                else if (s->flux == FLUX_LHLLD)
-                    k_flux2_ed<FLUX_LHLLD><<<nb, FXT, fx_smem<FLUX_LHLLD>(), st>>>(f, v, d, fb, stride,
-                                                                                   D, s->gamma);
-                else if (s->flux == FLUX_HLLD)
-                    k_flux2_ed<FLUX_HLLD><<<nb, FXT, fx_smem<FLUX_HLLD>(), st>>>(f, v, d, fb, stride, D,
-                                                                                 s->gamma);
-                else
-                    k_flux2<<<blocks_for(fb.count(), TPB), TPB, 0, st>>>(f, v, d, fb, stride, D, s->flux,
-                                                                         s->gamma);
-            }
+        {
+            TimedLaunch tl(&s->timer, KK_REC);
+            if (2 * g.n <= kSmall2) launch_rec2<32>(s, S, d);
+            else launch_rec2<128>(s, S, d);
+        }
+        {
+            TimedLaunch tl(&s->timer, KK_FLUX);
+            if (2 * g.n <= kSmall2) launch_flux2<32>(s, S, d);
+            else launch_flux2<256>(s, S, d);
         }
         {
             TimedLaunch tl(&s->timer, KK_EMF);

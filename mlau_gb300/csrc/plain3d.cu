@@ -43,7 +43,7 @@ __device__ __forceinline__ long long src3(const Dims &d, int i, int j, int k, in
 }
 
 __global__ void __launch_bounds__(TPB)
-k_prim3(PlainFields f, Dims d, Box b, int odr, double gamma, Bc3 bc)
+k_prim3(PlainFields f, Dims d, Box b, int odr, double gamma, Bc3 bc, int save_u0)
 {
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
@@ -57,6 +57,9 @@ k_prim3(PlainFields f, Dims d, Box b, int odr, double gamma, Bc3 bc)
     const ed cy = ed(gy) * face2cen<ed>(odr, by[wy - sy], by[wy], by[wy + sy], by[wy + 2 * sy]);
     const ed cz = ed(gz) * face2cen<ed>(odr, bz[wz - sz], bz[wz], bz[wz + sz], bz[wz + 2 * sz]);
     const long long s = d.at(i, j, k);
+    if (save_u0)  // the first stage keeps U^n
+#pragma unroll
+        for (int v = 0; v < 8; v++) f.u0[v][s] = f.s[v][s];
     const ed ro = f.s[0][s];
     const ed iro = trcp(ro);
     const ed vx = f.s[1][s] * iro, vy = f.s[2][s] * iro, vz = f.s[3][s] * iro;
@@ -215,6 +218,8 @@ k_flux3(PlainFields f, SweepView v, Dims d, Box b, long long st, int D, int whic
 }
 
 // MLAU, LHLLD and HLLD faces on both pipes (flux_exact.cuh).
+constexpr int FXT = 256;  // threads of a k_flux3_ed block
+
 template <int WHICH>
 __global__ void __launch_bounds__(FXT, 2)
 k_flux3_ed(PlainFields f, SweepView v, Dims d, Box b, long long st, int D, double gamma)
@@ -227,7 +232,7 @@ k_flux3_ed(PlainFields f, SweepView v, Dims d, Box b, long long st, int D, doubl
     const double dv[4] = {v.dvt[c - st], v.dvt[c], v.dvu[c - st], v.dvu[c]};
     const double bn = (ed(0.5) * (ed(v.bface[c]) + v.bface[c])).v;
     double F[7];
-    riemann_ed<WHICH, 4>(IN, (double (*)[FXT])fx_rows, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]).v, dv, F);
+    riemann_ed<WHICH, 4, FXT>(IN, (double (*)[FXT])fx_rows, bn, gamma, (ed(v.vn[c]) - v.vn[c - st]).v, dv, F);
     const ed fct = ihalf(ed(f.ql[0][c]) + f.qr[0][c]);
     const ed fcu = ihalf(ed(f.ql[1][c]) + f.qr[1][c]);
     F[4] = (F[4] - fct).v;
@@ -407,7 +412,7 @@ int plain3d_alloc(Sim *s)
         MLAU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)rec_smem<RCT>()));
     MLAU_CUDA(cudaFuncSetAttribute(k_flux3_ed<FLUX_MLAU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)fx_smem<FLUX_MLAU>()));
+                                   (int)fx_smem<FLUX_MLAU, FXT>()));
     return MLAU_OK;
 }
 
@@ -429,12 +434,6 @@ int plain3d_step(Sim *s, double dt)
     cudaStream_t st = s->stream;
     const Dims d{g.nx, g.ny, g.nz, g.ox, g.oy, g.oz};
     const long long sy = g.nx, sz = (long long)g.nx * g.ny;
-    {
-        TimedLaunch tl(&s->timer, KK_COPY);
-        for (int v = 0; v < 8; v++)
-            MLAU_CUDA(cudaMemcpyAsync(f.u0[v], f.s[v], sizeof(double) * g.n,
-                                      cudaMemcpyDeviceToDevice, st));
-    }
     const Box all{0, 0, 0, g.nx, g.ny, g.nz};
     const Box inner{g.ox, g.oy, g.oz, g.nx - 2 * g.ox, g.ny - 2 * g.oy, g.nz - 2 * g.oz};
     const long long strides[3] = {1, sy, sz};
@@ -445,7 +444,7 @@ int plain3d_step(Sim *s, double dt)
         {
             TimedLaunch tl(&s->timer, KK_PRIM);
             k_prim3<<<blocks_for(all.count(), TPB), TPB, 0, st>>>(f, d, all, s->odr, s->gamma,
-                                                                  s->bc3);
+                                                                  s->bc3, rk == 0);
         }
         {
             TimedLaunch tl(&s->timer, KK_AUX);
@@ -475,13 +474,13 @@ int plain3d_step(Sim *s, double dt)
                 TimedLaunch tl(&s->timer, KK_FLUX);
                 const unsigned nb = blocks_for(fb.count(), FXT);
                 if (s->flux == FLUX_MLAU)
-                    k_flux3_ed<FLUX_MLAU><<<nb, FXT, fx_smem<FLUX_MLAU>(), st>>>(f, v, d, fb, strides[D],
+                    k_flux3_ed<FLUX_MLAU><<<nb, FXT, fx_smem<FLUX_MLAU, FXT>(), st>>>(f, v, d, fb, strides[D],
                                                                                  D, s->gamma);
                 else if (s->flux == FLUX_LHLLD)
-                    k_flux3_ed<FLUX_LHLLD><<<nb, FXT, fx_smem<FLUX_LHLLD>(), st>>>(
+                    k_flux3_ed<FLUX_LHLLD><<<nb, FXT, fx_smem<FLUX_LHLLD, FXT>(), st>>>(
                         f, v, d, fb, strides[D], D, s->gamma);
                 else if (s->flux == FLUX_HLLD)
-                    k_flux3_ed<FLUX_HLLD><<<nb, FXT, fx_smem<FLUX_HLLD>(), st>>>(f, v, d, fb, strides[D],
+                    k_flux3_ed<FLUX_HLLD><<<nb, FXT, fx_smem<FLUX_HLLD, FXT>(), st>>>(f, v, d, fb, strides[D],
                                                                                  D, s->gamma);
                 else
                     k_flux3<<<blocks_for(fb.count(), TPB), TPB, 0, st>>>(f, v, d, fb, strides[D], D,
