@@ -15,7 +15,7 @@
 // last does the step's bookkeeping.  What bounds a stage is the latency of one
 // cell's chain of operations, most of it the full eigen-system where the flow is
 // supersonic.  24 instances of 256 to 4096 cells, mixed solvers, 29k cells in
-// all: 238 us a step with MUSCL, 436 with WCNS4; as eleven phases over arrays in
+// all: 238 us a step with MUSCL, 345 with WCNS4; as eleven phases over arrays in
 // memory, each with a barrier, 422 and 686.  The eight lanes to a cell of the
 // single simulation take 536 us for this load: they repeat too much of the
 // FP64 work to fill the chip with.

@@ -7,19 +7,23 @@
 // it; the other products, the quotients and roots run as integer sequences
 // (exact64.cuh), comparisons look at the values' bits, products by powers of
 // two move exponents, and weights that are 0 or 1 become selections (which can
-// change the sign of a zero, no value).  `bad` collects what the integer path
-// cannot decide or represent; such a face is evaluated again by
-// riemann<double>.
+// change the sign of a zero, no value).  A quotient or root whose rounding is
+// undecided (one in 2^15) is settled by the pipe on the spot: collected instead,
+// one lane in a warp of some 600 evaluations sent the whole face through
+// riemann<double>, and every small launch waited for such a warp (200 x 120
+// cells, fluxes of a step 139 -> 83 us; 128^3 8.9 -> 7.7 ms).  `bad` collects
+// products outside the integer path's range and values that are not finite;
+// such a face is evaluated again with the products on the pipe, and by
+// riemann<double> if that is not enough.
 //
 // The new bound is instruction supply: integer products make the code long
 // (some 35 instructions each), and beyond the instruction caches a sub-partition
 // gets about one instruction per two cycles.  The two sides and the two
 // tangential components therefore share code in loops of two with their values
-// in shared memory, and blocks have 256 threads, two per SM (3D 128^3 step,
-// 9 launches: 8.9 ms; 128 threads, four per SM, measured 1.1 ms more; products
-// out of line 10.2, all unrolled 15.8).
+// in shared memory, and blocks have 256 threads, two per SM (of 128 threads,
+// four per SM, 1.1 ms more; products out of line 1.3, all unrolled 6.9 more).
 //
-// Face fluxes of a 128^3 step: MLAU 15.5 -> 8.9 ms, LHLLD 8.8 -> 7.2 ms.
+// Face fluxes of a 128^3 step: MLAU 15.5 -> 7.7 ms.
 #pragma once
 
 #include "ed.cuh"
@@ -29,10 +33,11 @@ namespace mlau {
 // Operations of one flux evaluation.  Sums run on the FP64 pipe, quotients and
 // roots as integer sequences.  PIPE = false: products are integer sequences too,
 // and `bad` collects every input and product outside the integer path's range
-// (zero apart) and every undecided rounding.  PIPE = true, for grids that leave
-// the pipes idle and wait on instructions instead: products stay on the FP64
-// pipe, one instruction each.  Either way `bad` is zero only if every value
-// that was compared is finite, so comparisons can be made on the values' bits.
+// (zero apart).  PIPE = true, for grids that leave the pipes idle and wait on
+// instructions instead, and for magnitudes beyond that range: products stay on
+// the FP64 pipe, one instruction each.  Either way `bad` is zero only if every
+// value that was compared is finite, so comparisons can be made on the values'
+// bits.
 template <bool PIPE> struct FxOpsT {
     uint32_t bad = 0;
     double one, mz;
@@ -66,21 +71,26 @@ template <bool PIPE> struct FxOpsT {
         constexpr double c = P >= 0 ? (double)(1 << (P >= 0 ? P : 0)) : 1.0 / (double)(1 << (P < 0 ? -P : 0));
         return PIPE ? hmul(a, c) : x64::scale<P>(a);
     }
-    __device__ __forceinline__ double rcp(double a) { return x64::rcp_fast(a, bad); }
+    // an undecided rounding or an operand out of range is settled where it occurs;
+    // results that are not finite hand the face over
+    __device__ __forceinline__ double finite(double r)
+    {
+        bad |= (hi(r) << 1) >= 0xffe00000u ? 1u : 0u;
+        return r;
+    }
+    __device__ __forceinline__ double rcp(double a) { return finite(x64::rcp(a)); }
     // a may be zero
     __device__ __forceinline__ double div(double a, double b)
     {
-        uint32_t b0 = 0;
-        const double r = x64::div_fast(a, b, b0);
-        bad |= zero(a) ? x64::off_range(hi(b)) : b0;
-        return zero(a) ? x64::make((hi(a) ^ hi(b)) & 0x80000000u, 0) : r;
+        const bool z = zero(a);
+        const double r = finite(x64::div(z ? 1.0 : a, b));
+        return z ? x64::make((hi(a) ^ hi(b)) & 0x80000000u, 0) : r;
     }
     __device__ __forceinline__ double sqrt(double a)
     {
-        uint32_t b = 0;
-        const double r = x64::sqrt_fast(a, b);
-        bad |= zero(a) ? 0u : b;
-        return zero(a) ? a : r;
+        const bool z = zero(a);
+        const double r = finite(x64::sqrt(z ? 1.0 : a));
+        return z ? a : r;
     }
     static __device__ __forceinline__ double abs(double a) { return x64::make(hi(a) & 0x7fffffffu, lo(a)); }
     __device__ __forceinline__ bool positive(double a)
@@ -133,11 +143,11 @@ enum { FX_SCI = FX_CF2, FX_SRO = FX_CC2, FX_FB = FX_BF, FX_FV = FX_FF };
 // dv: the ND shock sensors, of which the smallest counts.  The two sides, and
 // the two tangential components, run through the same code in loops of two:
 // written out twice it overflows the instruction cache.
-template <int ND, int NT, class LOAD>
-__device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
-                                             const double dv[ND], double f[7])
+template <int ND, int NT, bool PIPE, class LOAD>
+__device__ __forceinline__ bool flux_mlau_core(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
+                                               const double dv[ND], double f[7])
 {
-    FxOpsT<false> o;
+    FxOpsT<PIPE> o;
     const int t = threadIdx.x;
     auto W = [&](int s, int k) -> double & { return rows[s * FX_ROWS + k][t]; };
     double dv1 = dv[0];
@@ -285,7 +295,25 @@ __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double
     f[4] = W(0, FX_DB);
     f[5] = W(0, FX_DB + 1);
     f[6] = o.sub(o.mul(mflux, W(up, FX_HN)), o.flip(nvb, sgn));
-    if (o.bad) {
+    return o.bad != 0;
+}
+
+// Faces the integer path hands over: first with the products on the FP64 pipe,
+// which take any magnitude, then all of it.
+template <int NT>
+__device__ __noinline__ void flux_mlau_over(const double *c, double (*rows)[NT], double bnc, double gamma, double dv0,
+                                          double dv1, double *f)
+{
+    const double dv[1] = {dv1};
+    if (flux_mlau_core<1, NT, true>([&](int s, int n) { return c[7 * s + n]; }, rows, bnc, gamma, dv0, dv, f))
+        flux_mlau_pipe(c, c + 7, bnc, gamma, dv0, dv1, f);
+}
+
+template <int ND, int NT, class LOAD>
+__device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
+                                             const double dv[ND], double f[7])
+{
+    if (flux_mlau_core<ND, NT, false>(IN, rows, bnc, gamma, dv0, dv, f)) {
         double c[14], g[7];
 #pragma unroll
         for (int n = 0; n < 7; n++) {
@@ -294,7 +322,7 @@ __device__ __forceinline__ void flux_mlau_ed(LOAD IN, double (*rows)[NT], double
         }
         double d1 = vmin(dv[0], dv[ND > 1 ? 1 : 0]);
         if constexpr (ND == 4) d1 = vmin(d1, vmin(dv[2], dv[3]));
-        flux_mlau_pipe(c, c + 7, bnc, gamma, dv0, d1, g);
+        flux_mlau_over<NT>(c, rows, bnc, gamma, dv0, d1, g);
 #pragma unroll
         for (int n = 0; n < 7; n++) f[n] = g[n];
     }
@@ -311,11 +339,11 @@ static __device__ __noinline__ void flux_hlld_pipe(const double *L, const double
 enum { HX_PT, HX_EN, HX_VB, HX_CF2, HX_CC2, HX_V2, HX_B2 = HX_V2 + 2, HX_ROWS = HX_B2 + 2 };
 enum { HX_RO2 = HX_PT, HX_RRO = HX_VB, HX_VB2 = HX_CF2, HX_EN2 = HX_EN };
 
-template <bool LOWDISS, int ND, int NT, class LOAD>
-__device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
-                                             const double dv[ND], double f[7])
+template <bool LOWDISS, int ND, int NT, bool PIPE, class LOAD>
+__device__ __forceinline__ bool flux_hlld_core(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
+                                               const double dv[ND], double f[7])
 {
-    FxOpsT<false> o;
+    FxOpsT<PIPE> o;
     const int t = threadIdx.x;
     auto W = [&](int s, int k) -> double & { return rows[s * HX_ROWS + k][t]; };
     double dv1 = dv[0];
@@ -440,7 +468,25 @@ __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double
     f[4] = o.sub(o.hmul(bu[0], vnc), o.hmul(bnc, vu[0]));
     f[5] = o.sub(o.hmul(bu[1], vnc), o.hmul(bnc, vu[1]));
     f[6] = o.sub(o.hmul(o.add(en, ptc), vnc), o.hmul(bnc, vbu));
-    if (o.bad) {
+    return o.bad != 0;
+}
+
+// Faces the integer path hands over: first with the products on the FP64 pipe,
+// which take any magnitude, then all of it.
+template <bool LOWDISS, int NT>
+__device__ __noinline__ void flux_hlld_over(const double *c, double (*rows)[NT], double bnc, double gamma, double dv0,
+                                          double dv1, double *f)
+{
+    const double dv[1] = {dv1};
+    if (flux_hlld_core<LOWDISS, 1, NT, true>([&](int s, int n) { return c[7 * s + n]; }, rows, bnc, gamma, dv0, dv, f))
+        flux_hlld_pipe<LOWDISS>(c, c + 7, bnc, gamma, dv0, dv1, f);
+}
+
+template <bool LOWDISS, int ND, int NT, class LOAD>
+__device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double bnc, double gamma, double dv0,
+                                             const double dv[ND], double f[7])
+{
+    if (flux_hlld_core<LOWDISS, ND, NT, false>(IN, rows, bnc, gamma, dv0, dv, f)) {
         double c[14], g[7];
 #pragma unroll
         for (int n = 0; n < 7; n++) {
@@ -449,7 +495,7 @@ __device__ __forceinline__ void flux_hlld_ed(LOAD IN, double (*rows)[NT], double
         }
         double d1 = vmin(dv[0], dv[ND > 1 ? 1 : 0]);
         if constexpr (ND == 4) d1 = vmin(d1, vmin(dv[2], dv[3]));
-        flux_hlld_pipe<LOWDISS>(c, c + 7, bnc, gamma, dv0, d1, g);
+        flux_hlld_over<LOWDISS, NT>(c, rows, bnc, gamma, dv0, d1, g);
 #pragma unroll
         for (int n = 0; n < 7; n++) f[n] = g[n];
     }

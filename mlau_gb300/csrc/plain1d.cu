@@ -20,11 +20,12 @@
 // overwrites what a neighbour reads; U^n stays in the state until then.
 //
 // One step, RK3, against separate kernels for primitives, reconstruction, fluxes,
-// boundary and update: 2048 cells MLAU + MUSCL 104 -> 60 us, LHLLD 100 -> 51 us,
-// MLAU + WCNS4 136 -> 97 us; 16384 cells MLAU + MUSCL 319 -> 164 us.  Products stay
+// boundary and update: 2048 cells MLAU + MUSCL 104 -> 47 us, LHLLD 100 -> 41 us,
+// MLAU + WCNS4 136 -> 71 us; 16384 cells MLAU + MUSCL 319 -> 162 us.  Products stay
 // FP64 instructions here, unlike in the 2D and 3D kernels: with one or two warps
 // to a sub-partition the 30 instructions of an integer product cost more than
-// the pipe's 64 cycles (2048 cells: 87 us with integer products).
+// the pipe's 64 cycles (2048 cells: 87 against 60 us, before the fallbacks were
+// made local).
 #include "stage1d.cuh"
 
 namespace mlau {

@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(TPB) k_aux2(PlainFields f, Dims d, Box b, Bc2 
 // By flux is split.  Along y (D=1): (vy, vz, vx), (bz, cx), the Bx flux is split.
 // Both sweeps run in one launch, side by side (blockIdx.y), so that grids of a
 // few thousand cells have twice the warps to hide each other's latency (200 x 120
-// cells, a step: LHLLD + MUSCL 425 -> 268 us, MLAU + WCNS4 627 -> 413).  A face's
+// cells, a step: LHLLD + MUSCL 425 -> 268 us, MLAU + WCNS4 627 -> 413; with the
+// flux and weight fallbacks made local 217 and 348).  A face's
 // left state lies where its flux goes.
 struct Sweep2 {
     const double *vn, *vt, *vu, *cn, *ct, *cu, *bface, *dvt;

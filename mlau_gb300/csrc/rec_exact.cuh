@@ -11,15 +11,18 @@
 // projections.  The seven fields, the three smoothness indicators and the two
 // sides go through loops over a shared-memory scratch and rotating registers:
 // unrolled, the code outgrows the instruction caches.  One flag collects the
-// operands outside the integer path's range and the undecided reciprocals; such
-// a lane evaluates the field on the FP64 pipe alone.  Five equal values (a
+// operands outside the integer path's range; such a lane evaluates the field on
+// the FP64 pipe alone.  Undecided reciprocals are settled on the spot, and
+// differences that vanish (uniform on one side of a jump) stay on the integer
+// path: its products by zero cost 0.7 % here and save the lanes of a shock tube
+// the other path (1D, 2048 cells, a step 90 -> 71 us).  Five equal values (a
 // uniform region) take constants.
 //
 // Reconstruction of a 3D 128^3 step (9 launches): WCNS4 34.0 ms on the FP64 pipe
-// alone, 20.5 with the WCNS4 products moved, 16.7 as it stands (FP64 pipe 85 %
-// busy, issue slots 46 %); MUSCL 9.3 -> 5.2 ms (three-point stencils project
-// three points only).  Block shapes (threads x blocks per SM) for 3D: 256 x 3
-// 16.7, 256 x 2 16.9, 128 x 5 17.3, 384 x 1 18.9 ms; the 2D grids' few waves
+// alone, 20.5 with the WCNS4 products moved, 16.7 with the projections' (FP64 pipe
+// 85 % busy, issue slots 46 %), 15.9 as it stands; MUSCL 9.3 -> 5.2 ms (three-point stencils project
+// three points only).  Block shapes (threads x blocks per SM) for 3D, at 16.7:
+// 256 x 3; 256 x 2 16.9, 128 x 5 17.3, 384 x 1 18.9 ms; the 2D grids' few waves
 // prefer 128 x 5 (512^2: 1.19 against 1.22 ms).
 #pragma once
 
@@ -83,8 +86,8 @@ __device__ __forceinline__ double2 wcns4_ed(double f0, double f1, double f2, dou
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
 #pragma unroll 1
     for (int n = 0; n < 3; n++) {
-        const double s = __fma_rn(q4, sqr_nz(p, bad), times(times(13. / 12., q), q));
-        const double g = rcp_fast(add(sqr_nz(s, bad), eps), bad);
+        const double s = __fma_rn(q4, sqr(p, bad), mul(mul(13. / 12., q, bad), q, bad));
+        const double g = rcp(add(sqr(s, bad), eps));
         s0 = s1;
         s1 = s2;
         s2 = g;
@@ -105,9 +108,9 @@ __device__ __forceinline__ double2 wcns4_ed(double f0, double f1, double f2, dou
 #pragma unroll 1
     for (int n = 0; n < 2; n++) {
         const double w0 = times(c0, s0);
-        const double d = rcp_fast(add(add(w0, m1), times(c2, s2)), bad);
+        const double d = rcp(add(add(w0, m1), times(c2, s2)));
         const double a = times(w0, d), b = times(m1, d), c = sub(sub(one, a), b);
-        const double v = add(add(times(n ? c : a, x0), times(b, x1)), times(n ? a : c, x2));
+        const double v = add(add(mul(n ? c : a, x0, bad), mul(b, x1, bad)), mul(n ? a : c, x2, bad));
         r.x = r.y;
         r.y = scale<-3>(v);
         x0 = y0;
