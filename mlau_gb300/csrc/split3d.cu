@@ -154,6 +154,20 @@ __device__ __forceinline__ ff face2cen_ff(int odr, const double b[4])
     return ff_scale(ff_sub(ff_mul_f(ff_add(f1, f2), 9.0f), ff_add(f0, f3)), 0.0625f);
 }
 
+// The FP64 form's sums of products, as FMAs of three registers (ed.cuh): with
+// those and the integer reciprocal prep takes 0.14 ms of a 61 x 90 x 72 step
+// instead of 0.17.
+__device__ __forceinline__ double face2cen_reg(int odr, const double b[4])
+{
+    if (lin_odr(odr) <= 2) return ihalf(ed(b[1]) + b[2]).v;
+    const double nine = __hiloint2double((int)(0x40220000u + opaque_zero()), 0);
+    return iscale<-4>(__fma_rn(nine, (ed(b[1]) + b[2]).v, -(ed(b[0]) + b[3]).v)).v;
+}
+__device__ __forceinline__ double norm2_reg(const double a[3])
+{
+    return __fma_rn(a[2], a[2], __fma_rn(a[0], a[0], (ed(a[1]) * a[1]).v));
+}
+
 // F64: pressure recovery and cell B in FP64 arithmetic (the split form with
 // FP64 kept for the state arithmetic) instead of float-float; the primitives
 // then leave as the (hi, lo) splits of their FP64 values, velocities included.
@@ -194,13 +208,16 @@ ks_prim(PlainFields f, SplitPtrs g, Dims d, Bc3 bc, int odr, float2 gm1, double 
     for (int v = 0; v < 8; v++) u[v] = f.s[v][s];
     if constexpr (F64) {
         // p = (gamma-1)(E - rho v^2/2 - B^2/2) and cell B in FP64
-        const double ro = u[0], iro = 1.0 / ro;
-        const double cx = gb[0] * face2cen(odr, bs[0][0], bs[0][1], bs[0][2], bs[0][3]);
-        const double cy = gb[1] * face2cen(odr, bs[1][0], bs[1][1], bs[1][2], bs[1][3]);
-        const double cz = gb[2] * face2cen(odr, bs[2][0], bs[2][1], bs[2][2], bs[2][3]);
-        const double vx = u[1] * iro, vy = u[2] * iro, vz = u[3] * iro;
-        const double pr = gm1d * (u[4] - 0.5 * (ro * (vx * vx + vy * vy + vz * vz)
-                                                + (cx * cx + cy * cy + cz * cz)));
+        const double ro = u[0], iro = x64::rcp(ro);
+        double c[3], v[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            c[a] = face2cen_reg(odr, bs[a]);
+            if constexpr (WALLS) c[a] = (ed(gb[a]) * c[a]).v;
+            v[a] = (ed(u[1 + a]) * iro).v;
+        }
+        const double cx = c[0], cy = c[1], cz = c[2], vx = v[0], vy = v[1], vz = v[2];
+        const double pr = (ed(gm1d) * (ed(u[4]) - ihalf(__fma_rn(ro, norm2_reg(v), norm2_reg(c))))).v;
         const float2 ro2 = split2(ro), vx2 = split2(vx), vy2 = split2(vy), vz2 = split2(vz);
         const float2 pr2 = split2(pr);
         g.q[0][sp] = ro2;
@@ -736,8 +753,9 @@ __global__ void __launch_bounds__(256) ks_emf(SplitPtrs g, Dims d, int odr_rt, i
 // the non-coherent path), so that the loads are in flight together, and the
 // arithmetic follows.  The FP64 pipe bounded it with the curl's differences
 // (36 instructions of 64 cycles a cell); these are formed on the integer pipe
-// (emf_diff.cuh), and instruction issue bounds it now: 256^3, one step, 4.50 ->
-// 3.59 ms (more or fewer registers: 3.60 at 80, 4.00 at 64).  One thread per
+// (emf_diff.cuh) and the rest are register FMAs; instruction issue bounds it now:
+// 256^3, one step, 4.50 -> 3.36 ms (at 3.59, fewer registers: 3.60 at 80, 4.00 at
+// 64).  One thread per
 // cell of an x-y plane, flattened: rows of blocks left 38 % of the threads idle
 // at nx = 160 and half of them at 61.
 
@@ -834,11 +852,11 @@ ks_update(PlainFields f, SplitPtrs g, Dims d, int odr_rt, RkFF rk, RkF64 rd, flo
                   + dtdy * fdiff(odr, fy[v][0], fy[v][1], fy[v][2], fy[v][3])
                   + dtdz * fdiff(odr, fz[v][0], fz[v][1], fz[v][2], fz[v][3]);
         if constexpr (F64) {
-            const double w = u[v] - to_f64(div);
+            const double w = (ed(u[v]) - to_f64(div)).v;
             out[v] = rk.first ? w : rd.ra * u0[v] + rd.rb * w;
         } else {
             // the first stage is u - div: one FP64 addition beats its float-float form
-            out[v] = rk.first ? u[v] - to_f64(div)
+            out[v] = rk.first ? (ed(u[v]) - to_f64(div)).v
                               : rk_ff(rk, u0[v], ff_add_f(ff_from(u[v]), -div));
         }
     }
