@@ -7,10 +7,13 @@
 //
 // What bounds a step: FP32 instructions and load latency in the
 // reconstruction and solver phases, and what the blocks wait for each other at
-// the barriers.  24 instances, 0.59M cells: 905 -> 873 us a step, with the
-// quotients dt/dx once per instance, the curl's differences on the integer pipe
-// (emf_diff.cuh; update 67 -> 45 us), the speeds' maximum on it too (47 -> 31) and
-// both directions between the same barriers (five a stage instead of seven).
+// the barriers.  24 instances, 0.59M cells: 898 -> 843 us a step; 64 instances
+// with 7.5M cells 8.31 -> 7.92 ms, 9.34 -> 9.09 ms where most are supersonic.  The
+// quotients dt/dx are formed once per instance, the curl's differences and the
+// speeds' maximum on the integer pipe (emf_diff.cuh; update 67 -> 45 us, speeds
+// 47 -> 31), the step lengths and the CT weights without a barrier of their
+// own, and a face's left state lies where its flux goes.  Both directions between
+// the same barriers: 856 us, but 10.25 ms for the supersonic mix (registers).
 #include "batch2d.cuh"
 #include "split_conv.cuh"
 #include "ed.cuh"
@@ -443,10 +446,12 @@ __global__ void __launch_bounds__(256, 3) kb_step_split(BArgs A)
         ph_prep(A, nt, tl, rk);
         if (grid_barrier(A.sync, A.nblocks)) return;
         ph_aux(A, nt, tl);
-        for (int D = 0; D < 2; D++) ph_rec(A, nt, tl, D);
-        if (grid_barrier(A.sync, A.nblocks)) return;
-        for (int D = 0; D < 2; D++) ph_flux(A, nt, tl, D);
-        if (grid_barrier(A.sync, A.nblocks)) return;
+        for (int D = 0; D < 2; D++) {
+            ph_rec(A, nt, tl, D);
+            if (grid_barrier(A.sync, A.nblocks)) return;
+            ph_flux(A, nt, tl, D);
+            if (grid_barrier(A.sync, A.nblocks)) return;
+        }
         ph_emf(A, nt, tl);
         if (grid_barrier(A.sync, A.nblocks)) return;
         ph_update(A, nt, tl, rk);
