@@ -94,8 +94,9 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
         if (m == 0) return MLAU_OK;
         for (int v = 0; v < m && to_host; v++) touch(a.dst[v], n);
         const unsigned nb = (unsigned)std::min(152LL, (n / 2 + 255) / 256 + 1);
-        k_copy8<<<dim3(nb, m), 256, 0, st>>>(a, n);
-        MLAU_CUDA(cudaGetLastError());
+        // the launch's own status: an error that an earlier call left behind is not this one's
+        void *args[] = {&a, &n};
+        MLAU_CUDA(cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(256), args, 0, st));
         // a copy from ordinary memory has read it when it returns
         if (wait && (to_host || kind == 2)) MLAU_CUDA(cudaStreamSynchronize(st));
         return MLAU_OK;

@@ -1,0 +1,77 @@
+// csrc/hostcopy.cu on a fake CUDA runtime whose "device" is host memory: the
+// kernel's launch copies, and notes in `launched` that it ran; `pending` is the
+// error an earlier call of the caller's left behind.
+#include <cstdarg>
+#include <cstring>
+#include <sys/mman.h>
+#include <sys/wait.h>
+#include <unistd.h>
+
+#include "hostcopy_fake.h"
+#include "hostcopy.cu"
+
+static int *launched;  // shared with the children
+static int copies;
+static cudaError_t pending = cudaSuccess;
+
+namespace mlau {
+void set_error(const char *, ...) {}
+}
+extern "C" {
+cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 1; return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *)
+{
+    memset(a, 0, sizeof(*a));
+    a->type = cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+cudaError_t cudaGetLastError() { const cudaError_t e = pending; pending = cudaSuccess; return e; }
+const char *cudaGetErrorString(cudaError_t) { return ""; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t)
+{
+    copies++;
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchKernel(const void *, dim3 grid, dim3, void **args, size_t, cudaStream_t)
+{
+    ++*launched;
+    const mlau::Fields8 &f = *(const mlau::Fields8 *)args[0];
+    const long long n = *(const long long *)args[1];
+    for (unsigned v = 0; v < grid.y; v++) memcpy(f.dst[v], f.src[v], sizeof(double) * n);
+    return cudaSuccess;
+}
+}
+
+static double g_dev[8 << 16];
+
+static int move(double *host, long long n, bool to_host)
+{
+    double *dev[8] = {}, *h[8] = {};
+    dev[3] = g_dev;
+    h[3] = host;
+    return mlau::copy_fields(dev, h, 8, n, to_host, true, nullptr);
+}
+
+static void setup()
+{
+    if (!launched)
+        launched = (int *)mmap(nullptr, 4096, PROT_READ | PROT_WRITE, MAP_SHARED | MAP_ANONYMOUS, -1, 0);
+    *launched = 0;
+    copies = 0;
+}
+
+// 0: moved by the kernel although an error of another call was pending
+extern "C" int pending_error_check()
+{
+    setup();
+    static double host[100];
+    for (int i = 0; i < 100; i++) host[i] = i;
+    pending = cudaErrorInvalidDevice;
+    const int up = move(host, 100, false);
+    memset(host, 0, sizeof(host));
+    const int down = move(host, 100, true);
+    return up || down || host[99] != 99.0 || *launched != 2;
+}

@@ -1,0 +1,26 @@
+"""The host side of the array moves (csrc/hostcopy.cu), compiled by the host
+compiler against a fake CUDA runtime: no GPU."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+from mlau_gb300 import _build
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("hostcopy") / "libhostcopy.so")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_build.nvcc()))), "include")
+    # -Bsymbolic: the fake runtime's own functions, whatever else the process loaded
+    subprocess.run(["g++", "-O2", "-std=c++17", "-w", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I" + cuda,
+                    "-I" + _build.INCLUDE, "-I" + _build.CSRC,
+                    os.path.join(ROOT, "tests", "c", "hostcopy_check.cpp"), "-o", out], check=True)
+    return C.CDLL(out)
+
+
+def test_an_earlier_error_is_not_the_moves(fake):
+    assert fake.pending_error_check() == 0
