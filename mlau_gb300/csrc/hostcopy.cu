@@ -61,14 +61,21 @@ int host_array(const void *p)
     return at.type == cudaMemoryTypeUnregistered ? 2 : at.type == cudaMemoryTypeHost ? 1 : 0;
 }
 
-// Have the pages of a host array there before the GPU writes to them: it would
-// wait for each (the bytes stay as they are).
-void touch(double *p, long long n)
+// One access by the CPU to every page of a host array before the GPU's.  An
+// array that is too short or not mapped then fails here, as it does in a copy from
+// pageable memory: the GPU's first access to a bad page would be a fault that takes
+// the context with it.  Before a write the pages are also made present (the GPU
+// would wait for each; the bytes stay as they are).  4 KB is the smallest page;
+// at 4 MB an array takes 1024 accesses.
+void touch(const double *p, long long n, bool write)
 {
     volatile char *b = (volatile char *)p;
     const long long bytes = n * (long long)sizeof(double);
-    for (long long i = 0; i < bytes; i += 4096) b[i] = b[i];
-    b[bytes - 1] = b[bytes - 1];
+    for (long long i = 0;; i = i + 4096 < bytes ? i + 4096 : bytes - 1) {
+        const char c = b[i];
+        if (write) b[i] = c;
+        if (i == bytes - 1) return;
+    }
 }
 
 }  // namespace
@@ -92,7 +99,7 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
     }
     if (kernel) {
         if (m == 0) return MLAU_OK;
-        for (int v = 0; v < m && to_host; v++) touch(a.dst[v], n);
+        for (int v = 0; v < m; v++) touch(to_host ? a.dst[v] : a.src[v], n, to_host);
         const unsigned nb = (unsigned)std::min(152LL, (n / 2 + 255) / 256 + 1);
         // the launch's own status: an error that an earlier call left behind is not this one's
         void *args[] = {&a, &n};

@@ -2,6 +2,7 @@
 // kernel's launch copies, and notes in `launched` that it ran; `pending` is the
 // error an earlier call of the caller's left behind.
 #include <cstdarg>
+#include <csignal>
 #include <cstring>
 #include <sys/mman.h>
 #include <sys/wait.h>
@@ -74,4 +75,29 @@ extern "C" int pending_error_check()
     memset(host, 0, sizeof(host));
     const int down = move(host, 100, true);
     return up || down || host[99] != 99.0 || *launched != 2;
+}
+
+// A child moves n doubles from or to an array at the end of `pages` accessible
+// pages, `shift` doubles further on, beyond which (hole: whose third page) no
+// access is allowed.  Returns 0: moved; 1: the CPU's access failed and nothing was
+// launched; 2: launched all the same; 3: anything else.
+extern "C" int bad_array_check(int pages, long long n, int shift, int hole, int to_host)
+{
+    setup();
+    const long pg = sysconf(_SC_PAGESIZE);
+    char *m = (char *)mmap(nullptr, (pages + 1) * pg, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    mprotect(m + (hole ? 2 * pg : pages * pg), pg, PROT_NONE);
+    double *host = (double *)(m + pages * pg) - n + shift;
+    const pid_t pid = fork();
+    if (pid == 0) {
+        signal(SIGSEGV, SIG_DFL);
+        signal(SIGBUS, SIG_DFL);
+        _exit(move(host, n, to_host != 0) ? 9 : 0);
+    }
+    int st = 0;
+    waitpid(pid, &st, 0);
+    munmap(m, (pages + 1) * pg);
+    if (WIFEXITED(st) && WEXITSTATUS(st) == 0) return *launched == 1 ? 0 : 3;
+    if (!WIFSIGNALED(st) || (WTERMSIG(st) != SIGSEGV && WTERMSIG(st) != SIGBUS)) return 3;
+    return *launched ? 2 : 1;
 }

@@ -24,3 +24,18 @@ def fake(tmp_path_factory):
 
 def test_an_earlier_error_is_not_the_moves(fake):
     assert fake.pending_error_check() == 0
+
+
+@pytest.mark.parametrize("to_host", [0, 1])
+@pytest.mark.parametrize("back", [0, 1, 511])
+def test_a_bad_array_fails_on_the_host(fake, back, to_host):
+    """An array one double too long for its mapping, or with a page of it not
+    accessible, is met by the CPU before anything is launched; one that just
+    fits moves."""
+    page = os.sysconf("SC_PAGESIZE") // 8
+    n = 3 * page - back
+    assert fake.bad_array_check(4, C.c_longlong(n), 0, 0, to_host) == 0
+    assert fake.bad_array_check(4, C.c_longlong(n), 1, 0, to_host) == 1
+    assert fake.bad_array_check(4, C.c_longlong(n), 0, 1, to_host) == 1
+    assert fake.bad_array_check(1, C.c_longlong(1), 0, 0, to_host) == 0
+    assert fake.bad_array_check(1, C.c_longlong(1), 1, 0, to_host) == 1
