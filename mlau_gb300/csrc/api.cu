@@ -192,25 +192,27 @@ int mlau_sim_destroy(mlau_sim *s)
     return MLAU_OK;
 }
 
-static int upload(mlau_sim *s, const double *const *h, bool wait)
+static int upload(mlau_sim *s, const double *const *h, Move how)
 {
     if (!s || !h) { set_error("null argument"); return MLAU_ERR_ARG; }
     double *host[8];
     for (int v = 0; v < 8; v++) host[v] = s->g.dim == 1 && v == 5 ? nullptr : const_cast<double *>(h[v]);
-    return copy_fields(s->f.s, host, 8, s->g.n, false, wait, s->stream);
+    return copy_fields(s->f.s, host, 8, s->g.n, false, how, s->stream);
 }
 
-int mlau_sim_upload(mlau_sim *s, const double *const *h) { return upload(s, h, true); }
+int mlau_sim_upload(mlau_sim *s, const double *const *h) { return upload(s, h, Move::Copies); }
 
-int mlau_sim_download(mlau_sim *s, double *const *h)
+static int download(mlau_sim *s, double *const *h, Move how)
 {
     if (!s || !h) { set_error("null argument"); return MLAU_ERR_ARG; }
     double *host[8];
     for (int v = 0; v < 8; v++) host[v] = s->g.dim == 1 && v == 5 ? nullptr : h[v];
-    const int rc = copy_fields(s->f.s, host, 8, s->g.n, true, true, s->stream);
+    const int rc = copy_fields(s->f.s, host, 8, s->g.n, true, how, s->stream);
     if (rc != MLAU_OK) return rc;
     return s->sp ? split3d_check(s) : MLAU_OK;
 }
+
+int mlau_sim_download(mlau_sim *s, double *const *h) { return download(s, h, Move::Copies); }
 
 // A captured step graph holds the scheme parameters of its capture.
 static void drop_graph(mlau_sim *s)
@@ -593,9 +595,9 @@ int run_dropin(mlau_sim *c, double *const *h, double dt)
 {
     // FP32-split: the host link's copies overlap the step where the data allow
     if (c->sp && !c->walls3d) return split3d_step_host(c, dt, h);
-    int rc = upload(c, (const double *const *)h, false);
+    int rc = upload(c, (const double *const *)h, Move::Kernel);
     if (rc == MLAU_OK) rc = mlau_sim_step(c, dt, 1);
-    if (rc == MLAU_OK) rc = mlau_sim_download(c, h);
+    if (rc == MLAU_OK) rc = download(c, h, Move::Kernel);
     else cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read
     return rc;
 }
@@ -755,7 +757,7 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
     const int *tx = dnxs, *ty = dnys;
     mlau_sim *c = get_ctx(2, nx, ny, 1, xoff, yoff, 0, dx, dy, 1.0, gamma);
     int rc = c ? mlau_sim_set_bc_2d(c, tx, ty) : MLAU_ERR_NOMEM;
-    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, false);
+    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, Move::Kernel);
     if (rc == MLAU_OK) {
         if (op == MRX_RESISTIVE) rc = diff2d_resistive(c, coef, dt);
         else if (op == MRX_VISCOUS) rc = diff2d_viscous(c, coef, dt);
@@ -764,7 +766,7 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
     if (rc == MLAU_OK || rc == MLAU_ERR_CONVERGE) {
         double *out[8];
         for (int v = 0; v < 8; v++) out[v] = back[v] ? h[v] : nullptr;
-        const int rd = mlau_sim_download(c, out);
+        const int rd = download(c, out, Move::Kernel);
         if (rd != MLAU_OK) rc = rd;
     } else if (c) {
         cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read

@@ -10,6 +10,15 @@
 // against 18 / 19, 327352 198 / 178 against 113 / 129; at 4.7M doubles
 // 1782 / 1649 against 1512 / 1791, so arrays above 4 MB are copied, as are
 // device or managed arrays and where the GPU cannot reach host memory.
+//
+// Only the drivers' calls on host arrays ask for the kernel: they wait for their
+// result and need the SMs for the step in between.  The handles' and engines' own
+// uploads and downloads are copies, which need no SM: the kernel had them wait for
+// a step of whatever else ran on the GPU (24 kB to 0.7 MB beside a batch with 2.4 ms
+// steps: 38 to 140 us by copies, 2400 by the kernel), an upload for all that was
+// queued on its stream (51 kB arrays behind 39 ms of steps: 33 us by copies), and
+// a download into arrays not used before, as Sim.download makes them, for the
+// pages (2 MB each: 0.2 to 1.2 ms by copies, 3.3 to 5.5 by the kernel).
 #include <algorithm>
 
 #include "hostcopy.h"
@@ -49,16 +58,16 @@ bool reaches_host_memory()
            direct && tables;
 }
 
-// 2: ordinary host memory, 1: pinned; 0: anything else, or not aligned for a double
-int host_array(const void *p)
+// Ordinary or pinned host memory, aligned for a double.
+bool host_array(const void *p)
 {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
-        return 0;
+        return false;
     }
-    if ((unsigned long long)p & 7) return 0;
-    return at.type == cudaMemoryTypeUnregistered ? 2 : at.type == cudaMemoryTypeHost ? 1 : 0;
+    return ((unsigned long long)p & 7) == 0 &&
+           (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost);
 }
 
 // One access by the CPU to every page of a host array before the GPU's.  An
@@ -80,17 +89,15 @@ void touch(const double *p, long long n, bool write)
 
 }  // namespace
 
-int copy_fields(double *const *dev, double *const *host, int nv, long long n, bool to_host, bool wait,
+int copy_fields(double *const *dev, double *const *host, int nv, long long n, bool to_host, Move how,
                 cudaStream_t st)
 {
     Fields8 a{};
-    int m = 0, kind = 0;
-    bool kernel = n > 0 && (long long)sizeof(double) * n <= kKernelBytes && nv <= 8 && reaches_host_memory();
+    int m = 0;
+    bool kernel = how == Move::Kernel && n > 0 && (long long)sizeof(double) * n <= kKernelBytes && nv <= 8 && reaches_host_memory();
     for (int v = 0; v < nv && kernel; v++) {
         if (!dev[v] || !host[v]) continue;
-        const int k = host_array(host[v]);
-        kernel = k != 0;
-        kind = std::max(kind, k);
+        kernel = host_array(host[v]);
         // arrays that overlap are written one after the other
         for (int w = 0; w < v && to_host; w++)
             if (dev[w] && host[w] && host[w] < host[v] + n && host[v] < host[w] + n) kernel = false;
@@ -104,8 +111,7 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
         // the launch's own status: an error that an earlier call left behind is not this one's
         void *args[] = {&a, &n};
         MLAU_CUDA(cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(256), args, 0, st));
-        // a copy from ordinary memory has read it when it returns
-        if (wait && (to_host || kind == 2)) MLAU_CUDA(cudaStreamSynchronize(st));
+        if (to_host) MLAU_CUDA(cudaStreamSynchronize(st));
         return MLAU_OK;
     }
     for (int v = 0; v < nv; v++) {
@@ -113,7 +119,7 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
         MLAU_CUDA(to_host ? cudaMemcpyAsync(host[v], dev[v], sizeof(double) * n, cudaMemcpyDeviceToHost, st)
                           : cudaMemcpyAsync(dev[v], host[v], sizeof(double) * n, cudaMemcpyHostToDevice, st));
     }
-    if (wait && to_host) MLAU_CUDA(cudaStreamSynchronize(st));
+    if (to_host) MLAU_CUDA(cudaStreamSynchronize(st));
     return MLAU_OK;
 }
 

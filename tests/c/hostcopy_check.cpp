@@ -53,7 +53,7 @@ static int move(double *host, long long n, bool to_host)
     double *dev[8] = {}, *h[8] = {};
     dev[3] = g_dev;
     h[3] = host;
-    return mlau::copy_fields(dev, h, 8, n, to_host, true, nullptr);
+    return mlau::copy_fields(dev, h, 8, n, to_host, mlau::Move::Kernel, nullptr);
 }
 
 static void setup()
