@@ -7,18 +7,23 @@
 // host's page tables (Grace and Blackwell share them over NVLink-C2C) a kernel
 // reads and writes the arrays where they are.  Eight arrays there / back, copies
 // against the kernel: 2056 doubles each 23 / 66 against 11 / 10 us, 26624 79 / 74
-// against 18 / 19, 327352 198 / 178 against 113 / 129; at 4.7M doubles
-// 1782 / 1649 against 1512 / 1791, so arrays above 4 MB are copied, as are
-// device or managed arrays and where the GPU cannot reach host memory.
+// against 18 / 19.  Arrays above 256 KB are copied, as are device or managed
+// arrays and where the GPU cannot reach host memory: the bytes count there, and
+// the kernel gains less or loses (pinned arrays to the host: 213 KB 30 against
+// 23 us, 0.7 MB 51 against 56, 2 MB 108 against 145; ordinary ones 3.8 MB 233
+// against 266), and where another engine's steps hold the SMs, which copies do
+// without, a driver's call waits for them (beside 2.4 ms steps, a 2D call with
+// arrays of 0.7 / 2 MB 12 / 11 ms by copies, 22 / 28 by the kernel; 192 KB 15.8
+// and 15.7).
 //
 // Only the drivers' calls on host arrays ask for the kernel: they wait for their
 // result and need the SMs for the step in between.  The handles' and engines' own
 // uploads and downloads are copies, which need no SM: the kernel had them wait for
-// a step of whatever else ran on the GPU (24 kB to 0.7 MB beside a batch with 2.4 ms
+// a step of whatever else ran on the GPU (16 kB to 0.7 MB beside a batch with 2.4 ms
 // steps: 38 to 140 us by copies, 2400 by the kernel), an upload for all that was
 // queued on its stream (51 kB arrays behind 39 ms of steps: 33 us by copies), and
 // a download into arrays not used before, as Sim.download makes them, for the
-// pages (2 MB each: 0.2 to 1.2 ms by copies, 3.3 to 5.5 by the kernel).
+// pages (2 MB each: 0.2 to 1.6 ms by copies, 3.3 to 5.5 by the kernel).
 #include <algorithm>
 
 #include "hostcopy.h"
@@ -31,7 +36,7 @@ struct Fields8 {
     double *dst[8];
 };
 
-constexpr long long kKernelBytes = 4 << 20;  // the largest array the kernel moves
+constexpr long long kKernelBytes = 256 << 10;  // the largest array the kernel moves
 
 // Array blockIdx.y, by pairs where both sides are aligned for it.
 __global__ void __launch_bounds__(256) k_copy8(const __grid_constant__ Fields8 a, long long n)
@@ -75,7 +80,7 @@ bool host_array(const void *p)
 // pageable memory: the GPU's first access to a bad page would be a fault that takes
 // the context with it.  Before a write the pages are also made present (the GPU
 // would wait for each; the bytes stay as they are).  4 KB is the smallest page;
-// at 4 MB an array takes 1024 accesses.
+// the largest array here takes 65 accesses.
 void touch(const double *p, long long n, bool write)
 {
     volatile char *b = (volatile char *)p;

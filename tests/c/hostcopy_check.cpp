@@ -101,3 +101,12 @@ extern "C" int bad_array_check(int pages, long long n, int shift, int hole, int 
     if (!WIFSIGNALED(st) || (WTERMSIG(st) != SIGSEGV && WTERMSIG(st) != SIGBUS)) return 3;
     return *launched ? 2 : 1;
 }
+
+// moves of n doubles there and back: 1 by the kernel, 2 by copies
+extern "C" int moved_by(long long n)
+{
+    setup();
+    static double host[8 << 16];
+    if (move(host, n, false) || move(host, n, true)) return 0;
+    return *launched == 2 && copies == 0 ? 1 : *launched == 0 && copies == 2 ? 2 : 0;
+}

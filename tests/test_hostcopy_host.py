@@ -39,3 +39,10 @@ def test_a_bad_array_fails_on_the_host(fake, back, to_host):
     assert fake.bad_array_check(4, C.c_longlong(n), 0, 1, to_host) == 1
     assert fake.bad_array_check(1, C.c_longlong(1), 0, 0, to_host) == 0
     assert fake.bad_array_check(1, C.c_longlong(1), 1, 0, to_host) == 1
+
+
+def test_large_arrays_are_copied(fake):
+    """Above 256 KB the kernel is slower than copies beside another engine's
+    steps and for pinned downloads."""
+    for n, by in ((1, 1), (4096, 1), (32768, 1), (32769, 2), (90000, 2), (400000, 2)):
+        assert fake.moved_by(C.c_longlong(n)) == by, n
