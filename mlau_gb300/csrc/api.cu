@@ -595,9 +595,10 @@ int run_dropin(mlau_sim *c, double *const *h, double dt)
 {
     // FP32-split: the host link's copies overlap the step where the data allow
     if (c->sp && !c->walls3d) return split3d_step_host(c, dt, h);
-    int rc = upload(c, (const double *const *)h, Move::Kernel);
+    const Move how = c->g.dim < 3 ? Move::Kernel : Move::Copies;
+    int rc = upload(c, (const double *const *)h, how);
     if (rc == MLAU_OK) rc = mlau_sim_step(c, dt, 1);
-    if (rc == MLAU_OK) rc = download(c, h, Move::Kernel);
+    if (rc == MLAU_OK) rc = download(c, h, how);
     else cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read
     return rc;
 }
@@ -757,7 +758,7 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
     const int *tx = dnxs, *ty = dnys;
     mlau_sim *c = get_ctx(2, nx, ny, 1, xoff, yoff, 0, dx, dy, 1.0, gamma);
     int rc = c ? mlau_sim_set_bc_2d(c, tx, ty) : MLAU_ERR_NOMEM;
-    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, Move::Kernel);
+    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, Move::Copies);
     if (rc == MLAU_OK) {
         if (op == MRX_RESISTIVE) rc = diff2d_resistive(c, coef, dt);
         else if (op == MRX_VISCOUS) rc = diff2d_viscous(c, coef, dt);
@@ -766,7 +767,7 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
     if (rc == MLAU_OK || rc == MLAU_ERR_CONVERGE) {
         double *out[8];
         for (int v = 0; v < 8; v++) out[v] = back[v] ? h[v] : nullptr;
-        const int rd = download(c, out, Move::Kernel);
+        const int rd = download(c, out, Move::Copies);
         if (rd != MLAU_OK) rc = rd;
     } else if (c) {
         cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read
