@@ -26,6 +26,17 @@
 namespace mlau {
 namespace {
 
+__device__ __forceinline__ double as_double(double x) { return x; }
+__device__ __forceinline__ double as_double(ed x) { return x.v; }
+
+// The explicit operators on small grids wait for their launches and
+// instructions, not for the FP64 pipe: below 4th order, where there is little for
+// the integer forms to take off it, the built-in double is the faster up to some
+// 20000 cells.  The same bits either way.  A call at 2nd order, double against ed:
+// viscous 8 x 8 cells 62 and 68 us, 64 x 56 73 and 78, 192 x 112 87 and 81;
+// resistive 64 x 56 83 and 87, 192 x 112 93 and 90.
+inline bool small_explicit(const Sim *s) { return lin_odr(s->odr) <= 2 && s->g.n <= 20480; }
+
 __device__ __forceinline__ long long at2(const Dims &d, int i, int j)
 {
     return (long long)d.nx * j + i;
@@ -39,6 +50,7 @@ struct Res {
 };
 
 // E = eta0 * J over [2, nx-1) x [2, ny-1) (:772-801)
+template <class T>
 __global__ void __launch_bounds__(TPB) k_res_e(Res r, Dims d, Box b, int odr, double eta0,
                                                double idx, double idy)
 {
@@ -46,17 +58,18 @@ __global__ void __launch_bounds__(TPB) k_res_e(Res r, Dims d, Box b, int odr, do
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long s = at2(d, i, j), sy = d.nx;
     const double *bx = r.bx, *by = r.by, *bz = r.bz;
-    const ed jx = +fdiff<ed>(odr, bz[s - 2 * sy], bz[s - sy], bz[s], bz[s + sy]) * idy;
-    const ed jy = -fdiff<ed>(odr, bz[s - 2], bz[s - 1], bz[s], bz[s + 1]) * idx;
-    const ed jz = +fdiff<ed>(odr, by[s - 2], by[s - 1], by[s], by[s + 1]) * idx
-                      - fdiff<ed>(odr, bx[s - 2 * sy], bx[s - sy], bx[s], bx[s + sy]) * idy;
-    r.ex[s] = (ed(eta0) * jx).v;
-    r.ey[s] = (ed(eta0) * jy).v;
-    r.ez[s] = (ed(eta0) * jz).v;
+    const T jx = +fdiff<T>(odr, bz[s - 2 * sy], bz[s - sy], bz[s], bz[s + sy]) * idy;
+    const T jy = -fdiff<T>(odr, bz[s - 2], bz[s - 1], bz[s], bz[s + 1]) * idx;
+    const T jz = +fdiff<T>(odr, by[s - 2], by[s - 1], by[s], by[s + 1]) * idx
+                      - fdiff<T>(odr, bx[s - 2 * sy], bx[s - sy], bx[s], bx[s + sy]) * idy;
+    r.ex[s] = as_double(T(eta0) * jx);
+    r.ey[s] = as_double(T(eta0) * jy);
+    r.ez[s] = as_double(T(eta0) * jz);
 }
 
 // Energy fluxes: along X over [2, nx-1) x [2, ny-2), along Y over
 // [2, nx-2) x [2, ny-1) (:802-852)
+template <class T>
 __global__ void __launch_bounds__(TPB) k_res_flux(Res r, Dims d, Box b, int odr)
 {
     int i, j, k;
@@ -64,27 +77,28 @@ __global__ void __launch_bounds__(TPB) k_res_flux(Res r, Dims d, Box b, int odr)
     const long long s = at2(d, i, j), sy = d.nx;
     const double *bx = r.bx, *by = r.by, *bz = r.bz, *ez = r.ez;
     if (j < d.ny - 2) {
-        const ed ep = r.ey[s];
-        const ed bp = face2cen<ed>(odr, bz[s - 2], bz[s - 1], bz[s], bz[s + 1]);
-        const ed em = thalf(ed(ez[s]) + ez[s + sy]);
-        const ed bm = thalf(face2cen<ed>(odr, by[s - 2], by[s - 1], by[s], by[s + 1])
-                                 + face2cen<ed>(odr, by[s + sy - 2], by[s + sy - 1], by[s + sy],
+        const T ep = r.ey[s];
+        const T bp = face2cen<T>(odr, bz[s - 2], bz[s - 1], bz[s], bz[s + 1]);
+        const T em = thalf(T(ez[s]) + ez[s + sy]);
+        const T bm = thalf(face2cen<T>(odr, by[s - 2], by[s - 1], by[s], by[s + 1])
+                                 + face2cen<T>(odr, by[s + sy - 2], by[s + sy - 1], by[s + sy],
                                             by[s + sy + 1]));
-        r.fx[s] = (ep * bp - em * bm).v;
+        r.fx[s] = as_double(ep * bp - em * bm);
     }
     if (i < d.nx - 2) {
-        const ed ep = thalf(ed(ez[s]) + ez[s + 1]);
-        const ed bp = thalf(face2cen<ed>(odr, bx[s - 2 * sy], bx[s - sy], bx[s], bx[s + sy])
-                                 + face2cen<ed>(odr, bx[s + 1 - 2 * sy], bx[s + 1 - sy], bx[s + 1],
+        const T ep = thalf(T(ez[s]) + ez[s + 1]);
+        const T bp = thalf(face2cen<T>(odr, bx[s - 2 * sy], bx[s - sy], bx[s], bx[s + sy])
+                                 + face2cen<T>(odr, bx[s + 1 - 2 * sy], bx[s + 1 - sy], bx[s + 1],
                                             bx[s + 1 + sy]));
-        const ed em = r.ex[s];
-        const ed bm = face2cen<ed>(odr, bz[s - 2 * sy], bz[s - sy], bz[s], bz[s + sy]);
-        r.fy[s] = (ep * bp - em * bm).v;
+        const T em = r.ex[s];
+        const T bm = face2cen<T>(odr, bz[s - 2 * sy], bz[s - sy], bz[s], bz[s + sy]);
+        r.fy[s] = as_double(ep * bp - em * bm);
     }
 }
 
 // CT Bx over [xoff, nx-xoff] x [yoff, ny-yoff), By over [xoff, nx-xoff) x
 // [yoff, ny-yoff], Bz and energy over the interior (:854-921)
+template <class T>
 __global__ void __launch_bounds__(TPB)
 k_res_update(Res r, Dims d, Box b, int odr, double ra, double rb, double dtdx, double dtdy)
 {
@@ -94,20 +108,20 @@ k_res_update(Res r, Dims d, Box b, int odr, double ra, double rb, double dtdx, d
     const double *ez = r.ez, *ex = r.ex, *ey = r.ey, *fx = r.fx, *fy = r.fy;
     const bool in_x = i < d.nx - d.ox, in_y = j < d.ny - d.oy;
     if (in_y) {
-        const ed du = fdiff<ed>(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
-        r.bx[s] = (ed(ra) * r.ut[0][s] + ed(rb) * (ed(r.bx[s]) - dtdy * du)).v;
+        const T du = fdiff<T>(odr, ez[s - sy], ez[s], ez[s + sy], ez[s + 2 * sy]);
+        r.bx[s] = as_double(T(ra) * r.ut[0][s] + T(rb) * (T(r.bx[s]) - dtdy * du));
     }
     if (in_x) {
-        const ed du = fdiff<ed>(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
-        r.by[s] = (ed(ra) * r.ut[1][s] + ed(rb) * (ed(r.by[s]) + dtdx * du)).v;
+        const T du = fdiff<T>(odr, ez[s - 1], ez[s], ez[s + 1], ez[s + 2]);
+        r.by[s] = as_double(T(ra) * r.ut[1][s] + T(rb) * (T(r.by[s]) + dtdx * du));
     }
     if (in_x && in_y) {
-        const ed d00 = fdiff<ed>(odr, ey[s - 1], ey[s], ey[s + 1], ey[s + 2]);
-        const ed d01 = fdiff<ed>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
-        const ed d10 = fdiff<ed>(odr, ex[s - sy], ex[s], ex[s + sy], ex[s + 2 * sy]);
-        const ed d11 = fdiff<ed>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
-        r.bz[s] = (ed(ra) * r.ut[2][s] + ed(rb) * (ed(r.bz[s]) - dtdx * d00 + dtdy * d10)).v;
-        r.en[s] = (ed(ra) * r.ut[3][s] + ed(rb) * (ed(r.en[s]) - dtdx * d01 - dtdy * d11)).v;
+        const T d00 = fdiff<T>(odr, ey[s - 1], ey[s], ey[s + 1], ey[s + 2]);
+        const T d01 = fdiff<T>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
+        const T d10 = fdiff<T>(odr, ex[s - sy], ex[s], ex[s + sy], ex[s + 2 * sy]);
+        const T d11 = fdiff<T>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
+        r.bz[s] = as_double(T(ra) * r.ut[2][s] + T(rb) * (T(r.bz[s]) - dtdx * d00 + dtdy * d10));
+        r.en[s] = as_double(T(ra) * r.ut[3][s] + T(rb) * (T(r.en[s]) - dtdx * d01 - dtdy * d11));
     }
 }
 
@@ -120,106 +134,110 @@ struct Visc {
     double *fx[4], *fy[4];
 };
 
+template <class T>
 __global__ void __launch_bounds__(TPB) k_visc_begin(Visc q, long long n)
 {
     const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
-    const ed ir = trcp(ed(q.ro[s]));
-    q.ir[s] = ir.v;
+    const T ir = trcp(T(q.ro[s]));
+    q.ir[s] = as_double(ir);
     for (int c = 0; c < 3; c++) {
-        q.v[c][s] = (ed(q.v[c][s]) * ir).v;
+        q.v[c][s] = as_double(T(q.v[c][s]) * ir);
         q.ut[c][s] = q.v[c][s];
     }
     q.ut[3][s] = q.en[s];
 }
 
+template <class T>
 __global__ void __launch_bounds__(TPB) k_visc_end(Visc q, long long n)
 {
     const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
-    for (int c = 0; c < 3; c++) q.v[c][s] = (ed(q.v[c][s]) * q.ro[s]).v;
+    for (int c = 0; c < 3; c++) q.v[c][s] = as_double(T(q.v[c][s]) * q.ro[s]);
 }
 
 // Fluxes: along X over [2, nx-1) x [1, ny-1), along Y over [1, nx-1) x
 // [2, ny-1) (:999-1089)
+template <class T>
 __global__ void __launch_bounds__(TPB)
 k_visc_flux(Visc q, Dims d, Box b, int odr, double nu0, double idx, double idy)
 {
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long s = at2(d, i, j), sy = d.nx;
-    const ed c2 = 2. / 3., c4 = 4. / 3.;
+    const T c2 = 2. / 3., c4 = 4. / 3.;
     const double *vx = q.v[0], *vy = q.v[1], *vz = q.v[2], *ro = q.ro;
     if (i >= 2) {
-        const ed ro0 = thalf(ed(ro[s]) + ro[s - 1]);
-        const ed rnu = ro0 * nu0;
-        const ed vx0 = face2cen<ed>(odr, vx[s - 2], vx[s - 1], vx[s], vx[s + 1]);
-        const ed vy0 = face2cen<ed>(odr, vy[s - 2], vy[s - 1], vy[s], vy[s + 1]);
-        const ed vz0 = face2cen<ed>(odr, vz[s - 2], vz[s - 1], vz[s], vz[s + 1]);
-        const ed dvxdx = fdiff<ed>(odr, vx[s - 2], vx[s - 1], vx[s], vx[s + 1]) * idx;
-        const ed dvydx = fdiff<ed>(odr, vy[s - 2], vy[s - 1], vy[s], vy[s + 1]) * idx;
-        const ed dvzdx = fdiff<ed>(odr, vz[s - 2], vz[s - 1], vz[s], vz[s + 1]) * idx;
-        ed dv[4];
+        const T ro0 = thalf(T(ro[s]) + ro[s - 1]);
+        const T rnu = ro0 * nu0;
+        const T vx0 = face2cen<T>(odr, vx[s - 2], vx[s - 1], vx[s], vx[s + 1]);
+        const T vy0 = face2cen<T>(odr, vy[s - 2], vy[s - 1], vy[s], vy[s + 1]);
+        const T vz0 = face2cen<T>(odr, vz[s - 2], vz[s - 1], vz[s], vz[s + 1]);
+        const T dvxdx = fdiff<T>(odr, vx[s - 2], vx[s - 1], vx[s], vx[s + 1]) * idx;
+        const T dvydx = fdiff<T>(odr, vy[s - 2], vy[s - 1], vy[s], vy[s + 1]) * idx;
+        const T dvzdx = fdiff<T>(odr, vz[s - 2], vz[s - 1], vz[s], vz[s + 1]) * idx;
+        T dv[4];
 #pragma unroll
-        for (int m = 0; m < 4; m++) dv[m] = thalf(ed(vx[s - 2 + m + sy]) - vx[s - 2 + m - sy]);
-        const ed dvxdy = face2cen<ed>(odr, dv[0], dv[1], dv[2], dv[3]) * idy;
+        for (int m = 0; m < 4; m++) dv[m] = thalf(T(vx[s - 2 + m + sy]) - vx[s - 2 + m - sy]);
+        const T dvxdy = face2cen<T>(odr, dv[0], dv[1], dv[2], dv[3]) * idy;
 #pragma unroll
-        for (int m = 0; m < 4; m++) dv[m] = thalf(ed(vy[s - 2 + m + sy]) - vy[s - 2 + m - sy]);
-        const ed dvydy = face2cen<ed>(odr, dv[0], dv[1], dv[2], dv[3]) * idy;
-        const ed f0 = -rnu * (c4 * dvxdx - c2 * dvydy);
-        const ed f1 = -rnu * (dvydx + dvxdy);
-        const ed f2 = -rnu * (dvzdx);
-        q.fx[0][s] = (f0).v;
-        q.fx[1][s] = (f1).v;
-        q.fx[2][s] = (f2).v;
-        q.fx[3][s] = (f0 * vx0 + f1 * vy0 + f2 * vz0).v;
+        for (int m = 0; m < 4; m++) dv[m] = thalf(T(vy[s - 2 + m + sy]) - vy[s - 2 + m - sy]);
+        const T dvydy = face2cen<T>(odr, dv[0], dv[1], dv[2], dv[3]) * idy;
+        const T f0 = -rnu * (c4 * dvxdx - c2 * dvydy);
+        const T f1 = -rnu * (dvydx + dvxdy);
+        const T f2 = -rnu * (dvzdx);
+        q.fx[0][s] = as_double(f0);
+        q.fx[1][s] = as_double(f1);
+        q.fx[2][s] = as_double(f2);
+        q.fx[3][s] = as_double(f0 * vx0 + f1 * vy0 + f2 * vz0);
     }
     if (j >= 2) {
-        const ed ro0 = thalf(ed(ro[s]) + ro[s - sy]);
-        const ed rnu = ro0 * nu0;
-        const ed vx0 = face2cen<ed>(odr, vx[s - 2 * sy], vx[s - sy], vx[s], vx[s + sy]);
-        const ed vy0 = face2cen<ed>(odr, vy[s - 2 * sy], vy[s - sy], vy[s], vy[s + sy]);
-        const ed vz0 = face2cen<ed>(odr, vz[s - 2 * sy], vz[s - sy], vz[s], vz[s + sy]);
-        const ed dvxdy = fdiff<ed>(odr, vx[s - 2 * sy], vx[s - sy], vx[s], vx[s + sy]) * idy;
-        const ed dvydy = fdiff<ed>(odr, vy[s - 2 * sy], vy[s - sy], vy[s], vy[s + sy]) * idy;
-        const ed dvzdy = fdiff<ed>(odr, vz[s - 2 * sy], vz[s - sy], vz[s], vz[s + sy]) * idy;
-        ed dv[4];
+        const T ro0 = thalf(T(ro[s]) + ro[s - sy]);
+        const T rnu = ro0 * nu0;
+        const T vx0 = face2cen<T>(odr, vx[s - 2 * sy], vx[s - sy], vx[s], vx[s + sy]);
+        const T vy0 = face2cen<T>(odr, vy[s - 2 * sy], vy[s - sy], vy[s], vy[s + sy]);
+        const T vz0 = face2cen<T>(odr, vz[s - 2 * sy], vz[s - sy], vz[s], vz[s + sy]);
+        const T dvxdy = fdiff<T>(odr, vx[s - 2 * sy], vx[s - sy], vx[s], vx[s + sy]) * idy;
+        const T dvydy = fdiff<T>(odr, vy[s - 2 * sy], vy[s - sy], vy[s], vy[s + sy]) * idy;
+        const T dvzdy = fdiff<T>(odr, vz[s - 2 * sy], vz[s - sy], vz[s], vz[s + sy]) * idy;
+        T dv[4];
 #pragma unroll
         for (int m = 0; m < 4; m++)
-            dv[m] = thalf(ed(vx[s + (m - 2) * sy + 1]) - vx[s + (m - 2) * sy - 1]);
-        const ed dvxdx = face2cen<ed>(odr, dv[0], dv[1], dv[2], dv[3]) * idx;
+            dv[m] = thalf(T(vx[s + (m - 2) * sy + 1]) - vx[s + (m - 2) * sy - 1]);
+        const T dvxdx = face2cen<T>(odr, dv[0], dv[1], dv[2], dv[3]) * idx;
 #pragma unroll
         for (int m = 0; m < 4; m++)
-            dv[m] = thalf(ed(vy[s + (m - 2) * sy + 1]) - vy[s + (m - 2) * sy - 1]);
-        const ed dvydx = face2cen<ed>(odr, dv[0], dv[1], dv[2], dv[3]) * idx;
-        const ed g0 = -rnu * (dvxdy + dvydx);
-        const ed g1 = -rnu * (c4 * dvydy - c2 * dvxdx);
-        const ed g2 = -rnu * (dvzdy);
-        q.fy[0][s] = (g0).v;
-        q.fy[1][s] = (g1).v;
-        q.fy[2][s] = (g2).v;
-        q.fy[3][s] = (g0 * vx0 + g1 * vy0 + g2 * vz0).v;
+            dv[m] = thalf(T(vy[s + (m - 2) * sy + 1]) - vy[s + (m - 2) * sy - 1]);
+        const T dvydx = face2cen<T>(odr, dv[0], dv[1], dv[2], dv[3]) * idx;
+        const T g0 = -rnu * (dvxdy + dvydx);
+        const T g1 = -rnu * (c4 * dvydy - c2 * dvxdx);
+        const T g2 = -rnu * (dvzdy);
+        q.fy[0][s] = as_double(g0);
+        q.fy[1][s] = as_double(g1);
+        q.fy[2][s] = as_double(g2);
+        q.fy[3][s] = as_double(g0 * vx0 + g1 * vy0 + g2 * vz0);
     }
 }
 
 // Update of the interior (:1091-1139)
+template <class T>
 __global__ void __launch_bounds__(TPB)
 k_visc_update(Visc q, Dims d, Box b, int odr, double ra, double rb, double dtdx, double dtdy)
 {
     int i, j, k;
     if (!b.decode((long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long s = at2(d, i, j), sy = d.nx;
-    ed du[2][4];
+    T du[2][4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         const double *fx = q.fx[c], *fy = q.fy[c];
-        du[0][c] = fdiff<ed>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
-        du[1][c] = fdiff<ed>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
+        du[0][c] = fdiff<T>(odr, fx[s - 1], fx[s], fx[s + 1], fx[s + 2]);
+        du[1][c] = fdiff<T>(odr, fy[s - sy], fy[s], fy[s + sy], fy[s + 2 * sy]);
     }
 #pragma unroll
     for (int c = 0; c < 3; c++)
-        q.v[c][s] = (ed(ra) * q.ut[c][s] + ed(rb) * (ed(q.v[c][s]) - (dtdx * du[0][c] + dtdy * du[1][c]) * q.ir[s])).v;
-    q.en[s] = (ed(ra) * q.ut[3][s] + ed(rb) * (ed(q.en[s]) - (dtdx * du[0][3] + dtdy * du[1][3]))).v;
+        q.v[c][s] = as_double(T(ra) * q.ut[c][s] + T(rb) * (T(q.v[c][s]) - (dtdx * du[0][c] + dtdy * du[1][c]) * q.ir[s]));
+    q.en[s] = as_double(T(ra) * q.ut[3][s] + T(rb) * (T(q.en[s]) - (dtdx * du[0][3] + dtdy * du[1][3])));
 }
 
 // ---- boundary fill of up to four arrays ----------------------------------------
@@ -553,7 +571,9 @@ int check_2d(Sim *s, const char *what)
 
 }  // namespace
 
-int diff2d_resistive(Sim *s, double eta0, double dt)
+namespace {
+
+template <class T> int resistive(Sim *s, double eta0, double dt)
 {
     int rc = check_2d(s, "resistive diffusion");
     if (rc) return rc;
@@ -574,10 +594,10 @@ int diff2d_resistive(Sim *s, double eta0, double dt)
     for (int rk = 0; rk < s->nrk; rk++) {
         double ra, rb;
         rk_coef(s->nrk, rk, ra, rb);
-        k_res_e<<<blocks_for(e.count(), TPB), TPB, 0, st>>>(r, d, e, s->odr, eta0, idx, idy);
-        k_res_flux<<<blocks_for(e.count(), TPB), TPB, 0, st>>>(r, d, e, s->odr);
-        k_res_update<<<blocks_for(up.count(), TPB), TPB, 0, st>>>(r, d, up, s->odr, ra, rb, dtdx,
-                                                                  dtdy);
+        k_res_e<T><<<blocks_for(e.count(), TPB), TPB, 0, st>>>(r, d, e, s->odr, eta0, idx, idy);
+        k_res_flux<T><<<blocks_for(e.count(), TPB), TPB, 0, st>>>(r, d, e, s->odr);
+        k_res_update<T><<<blocks_for(up.count(), TPB), TPB, 0, st>>>(r, d, up, s->odr, ra, rb, dtdx,
+                                                                     dtdy);
         launch_fill(fb, d, st);
         MLAU_CUDA(cudaGetLastError());
     }
@@ -586,7 +606,16 @@ int diff2d_resistive(Sim *s, double eta0, double dt)
     return MLAU_OK;
 }
 
-int diff2d_viscous(Sim *s, double nu0, double dt)
+}  // namespace
+
+int diff2d_resistive(Sim *s, double eta0, double dt)
+{
+    return small_explicit(s) ? resistive<double>(s, eta0, dt) : resistive<ed>(s, eta0, dt);
+}
+
+namespace {
+
+template <class T> int viscous(Sim *s, double nu0, double dt)
 {
     int rc = check_2d(s, "viscosity");
     if (rc) return rc;
@@ -601,20 +630,27 @@ int diff2d_viscous(Sim *s, double nu0, double dt)
     const Box in{g.ox, g.oy, 0, g.nx - 2 * g.ox, g.ny - 2 * g.oy, 1};
     const Fill fv = make_fill(s, {{f.s[1], 1}, {f.s[2], 2}, {f.s[3], 3}});
     const Fill fe = make_fill(s, {{f.s[4], 4}});
-    k_visc_begin<<<blocks_for(g.n, TPB), TPB, 0, st>>>(q, g.n);
+    k_visc_begin<T><<<blocks_for(g.n, TPB), TPB, 0, st>>>(q, g.n);
     for (int rk = 0; rk < s->nrk; rk++) {
         double ra, rb;
         rk_coef(s->nrk, rk, ra, rb);
-        k_visc_flux<<<blocks_for(fl.count(), TPB), TPB, 0, st>>>(q, d, fl, s->odr, nu0, idx, idy);
-        k_visc_update<<<blocks_for(in.count(), TPB), TPB, 0, st>>>(q, d, in, s->odr, ra, rb, dtdx,
-                                                                   dtdy);
+        k_visc_flux<T><<<blocks_for(fl.count(), TPB), TPB, 0, st>>>(q, d, fl, s->odr, nu0, idx, idy);
+        k_visc_update<T><<<blocks_for(in.count(), TPB), TPB, 0, st>>>(q, d, in, s->odr, ra, rb, dtdx,
+                                                                      dtdy);
         launch_fill(fv, d, st);
         MLAU_CUDA(cudaGetLastError());
     }
     launch_fill(fe, d, st);
-    k_visc_end<<<blocks_for(g.n, TPB), TPB, 0, st>>>(q, g.n);
+    k_visc_end<T><<<blocks_for(g.n, TPB), TPB, 0, st>>>(q, g.n);
     MLAU_CUDA(cudaGetLastError());
     return MLAU_OK;
+}
+
+}  // namespace
+
+int diff2d_viscous(Sim *s, double nu0, double dt)
+{
+    return small_explicit(s) ? viscous<double>(s, nu0, dt) : viscous<ed>(s, nu0, dt);
 }
 
 namespace {
