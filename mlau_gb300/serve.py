@@ -345,7 +345,7 @@ class Server:
     shares: fraction of the budget for each lane's pool ("1d", "2d64",
     "2d32", "3d").  max_inst: slots per batched lane."""
 
-    BYTES_PER_CELL = {"1d": 312, "2d64": 472, "2d32": 352}
+    BYTES_PER_CELL = {"1d": 168, "2d64": 472, "2d32": 352}
 
     def __init__(self, budget_bytes=120e9, shares=None, max_inst=256, steps_per_tick=None,
                  odr_2d=4, odr_1d=2):
