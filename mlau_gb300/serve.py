@@ -204,12 +204,20 @@ class _Lane(threading.Thread):
             self.server._wake.set()
 
 
+def blocks_1d(r, odr, threads=256):
+    """Blocks of the 1D engine's grid that request r keeps busy: one for each
+    tile of `threads` cells, which share the stencil's overlap with their
+    neighbours, and one for an open boundary."""
+    new = threads - (4 if odr in (3, 4) else 2)
+    return -(-r.interior // new) + (r.meta.get("bc") == "open")
+
+
 class _BatchLane(_Lane):
-    def __init__(self, server, name, batch, steps_per_tick, prio=False, tile=None):
+    def __init__(self, server, name, batch, steps_per_tick, prio=False, blocks_of=None):
         super().__init__(server, name)
         self.batch, self.k = batch, steps_per_tick
         self.live: dict[int, Request] = {}
-        self.prio, self.tile = prio, tile
+        self.prio, self.blocks_of = prio, blocks_of
 
     def _admit(self):
         while self.waiting:
@@ -239,8 +247,8 @@ class _BatchLane(_Lane):
             self._drain(block=not self.live)
             self._admit()
             cells = sum(r.interior for r in self.live.values())
-            useful = (sum(-(-r.interior // self.tile) for r in self.live.values())
-                      if self.tile else None)
+            useful = (sum(self.blocks_of(r) for r in self.live.values())
+                      if self.blocks_of else None)
             srv.blocks.set_load(self.lane, cells, useful, self.prio)
             if not self.live:
                 if srv.closing.is_set() and not self.waiting and self.inbox.empty():
@@ -367,9 +375,9 @@ class Server:
         self._wake = threading.Event()
         self._lock = threading.Lock()
         self.done: list[Request] = []
-        # the 1D lane is served first (see _Blocks); a block per 64-cell tile
+        # the 1D lane is served first (see _Blocks), with a block for each of its tiles
         self.lanes = {k: _BatchLane(self, k, b, spt[k], prio=(k == "1d"),
-                                    tile=64 if k == "1d" else None)
+                                    blocks_of=(lambda r: blocks_1d(r, odr_1d)) if k == "1d" else None)
                       for k, b in self.batches.items()}
         self.lanes["3d"] = _Lane3D(self, budget_bytes * shares["3d"])
         self.t0 = None
