@@ -348,7 +348,7 @@ int mlau_batch1d_add(mlau_batch *b, int nx, double dx, double bx, double gamma, 
  * device-memory budget: one 1D step like mhd_fd4c_1d (odr/flux/nrk/bc as in
  * the handle API) on arrays the caller already holds in device-accessible
  * memory, updated in place, with no allocation.  Its scratch is one static
- * device array of 32*(MLAU_NOALLOC_1D_MAX_NX+1) doubles (4.2 MB) that every
+ * device array of 14*MLAU_NOALLOC_1D_MAX_NX doubles (1.8 MB) that every
  * GPU loading the library holds until the process exits; nx above
  * MLAU_NOALLOC_1D_MAX_NX is rejected.  The first call on a device resolves
  * that array's device address (cudaGetSymbolAddress) - make it before any

@@ -22,10 +22,8 @@ int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int eig, int
 namespace {
 
 constexpr int kMaxNx = MLAU_NOALLOC_1D_MAX_NX;
-// the two buffers the stages go through: 14 nx doubles (the array's size is the
-// one the header states)
-constexpr long long kScratch = 32LL * (kMaxNx + 1);
-static_assert(14LL * kMaxNx <= kScratch, "noalloc scratch too small");
+// the two buffers of seven arrays that the stages go through
+constexpr long long kScratch = 14LL * kMaxNx;
 
 // One array per process and device; it lives until the process exits.
 static __device__ __align__(256) double g_noalloc_scratch[kScratch];
