@@ -226,7 +226,8 @@ void *mlau_sim_stream(mlau_sim *sim);
 int mlau_sim_device_ptr(mlau_sim *sim, int v, double **ptr);
 /* Per-kernel CUDA-event timing (off by default).  kind: 0 prim, 1 aux,
  * 2 reconstruction, 3 flux, 4 emf, 5 update, 6 copy, 7 cfl, 8 split sweep,
- * 9 split prep, 10 split update. */
+ * 9 split prep, 10 split update, 11 stage (1D: a whole RK stage is one kernel).
+ * In 2D kinds 2 and 3 are one launch for both directions. */
 int mlau_sim_set_timing(mlau_sim *sim, int on);
 int mlau_sim_timing(mlau_sim *sim, int kind, long *count, double *total_ms);
 /* Device bytes held by the simulation. */

@@ -28,7 +28,7 @@ OUT_F64, OUT_F32_RANK = 0, 1
 BC1D = {"open": 0, "periodic": 1}
 VARS = ("ro", "mx", "my", "mz", "en", "bx", "by", "bz")
 KERNEL_KINDS = ("prim", "aux", "rec", "flux", "emf", "update", "copy", "cfl",
-                "split_sweep", "split_prep", "split_update")
+                "split_sweep", "split_prep", "split_update", "stage")
 
 
 class MlauError(RuntimeError):

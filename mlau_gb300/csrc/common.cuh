@@ -59,7 +59,7 @@ struct Bc3 {
 // Kernel-kind identifiers for the optional per-kernel event timing.
 enum KernelKind {
     KK_PRIM = 0, KK_AUX, KK_REC, KK_FLUX, KK_EMF, KK_UPDATE, KK_COPY, KK_CFL,
-    KK_SPLIT_SWEEP, KK_SPLIT_PREP, KK_SPLIT_UPDATE, KK_COUNT
+    KK_SPLIT_SWEEP, KK_SPLIT_PREP, KK_SPLIT_UPDATE, KK_STAGE, KK_COUNT
 };
 
 // Records a CUDA event pair around each launch when enabled.

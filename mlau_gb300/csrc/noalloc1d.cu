@@ -16,7 +16,7 @@
 
 namespace mlau {
 int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int eig, int flux, int nrk, int bc,
-                    double bx, double dt, double dx, double gamma, cudaStream_t st);
+                    double bx, double dt, double dx, double gamma, cudaStream_t st, KernelTimer *timer);
 }
 
 namespace {
@@ -90,5 +90,5 @@ extern "C" int mlau_fd4c_1d_noalloc(double *ro, double *mx, double *my, double *
     for (int v = 0; v < 7; v++) { f.ul[v] = p; p += nx; }
     for (int v = 0; v < 7; v++) { f.ur[v] = p; p += nx; }
     return plain1d_enqueue(f, nx, xoff, odr, EIG_FULL, flux, nrk, bc, bx, dt, dx, gamma,
-                           (cudaStream_t)stream);
+                           (cudaStream_t)stream, nullptr);
 }

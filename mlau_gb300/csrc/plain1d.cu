@@ -76,9 +76,9 @@ int plain1d_alloc(Sim *s)
 }
 
 // Enqueue one 1D step on `st`: the state f.s, with f.ul and f.ur (7 arrays of nx
-// each) as the buffers between the stages.
+// each) as the buffers between the stages; timer: records each launch, or null.
 int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int eig, int flux, int nrk, int bc,
-                    double bx, double dt, double dx, double gamma, cudaStream_t st)
+                    double bx, double dt, double dx, double gamma, cudaStream_t st, KernelTimer *timer)
 {
     static const int slot[7] = {0, 1, 2, 3, 6, 7, 4};
     const void *kern = odr == 4 ? stage_kernel1<true>(flux) : stage_kernel1<false>(flux);
@@ -103,8 +103,11 @@ int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int eig, int
         for (int k = 0; k < 7; k++)
             a.d_[slot[k]] = back ? f.s[slot[k]] : (rk & 1 ? f.ur[k] : f.ul[k]);
         void *args[] = {&a, &ntiles};
-        MLAU_CUDA(cudaLaunchKernel(kern, dim3(ntiles + (a.open && a.first ? 1 : 0)), dim3(T1D), args, 0,
-                                   st));
+        {
+            TimedLaunch tl(timer, KK_STAGE);
+            MLAU_CUDA(cudaLaunchKernel(kern, dim3(ntiles + (a.open && a.first ? 1 : 0)), dim3(T1D), args,
+                                       0, st));
+        }
         for (int k = 0; k < 7; k++) a.s_[slot[k]] = a.d_[slot[k]];
     }
     if (nrk == 1)
@@ -117,9 +120,8 @@ int plain1d_enqueue(const PlainFields &f, int nx, int off, int odr, int eig, int
 int plain1d_step(Sim *s, double dt)
 {
     const Geometry &g = s->g;
-    TimedLaunch tl(&s->timer, KK_FLUX);
     return plain1d_enqueue(s->f, g.nx, g.ox, s->odr, s->eig, s->flux, s->nrk, s->bc1d, s->bx1d, dt, g.dx,
-                           s->gamma, s->stream);
+                           s->gamma, s->stream, &s->timer);
 }
 
 }  // namespace mlau
