@@ -278,7 +278,9 @@ __device__ void pp_bc(const BArgs &A, int nt, const BTile *tl)
     });
 }
 
-__global__ void __launch_bounds__(256) kb_step_plain(BArgs A)
+// 240 registers a thread leave room for a warp of the copy kernel (hostcopy.cu) in
+// each SM sub-partition.
+__global__ void __maxnreg__(240) kb_step_plain(BArgs A)
 {
     const int nt = A.sync->ntiles;
     const BTile *tl = A.sync->tiles;

@@ -24,8 +24,6 @@
 // queued on its stream (51 kB arrays behind 39 ms of steps: 33 us by copies), and
 // a download into arrays not used before, as Sim.download makes them, for the
 // pages (2 MB each: 0.2 to 1.6 ms by copies, 3.3 to 5.5 by the kernel).
-#include <algorithm>
-
 #include "hostcopy.h"
 
 namespace mlau {
@@ -38,18 +36,34 @@ struct Fields8 {
 
 constexpr long long kKernelBytes = 256 << 10;  // the largest array the kernel moves
 
-// Array blockIdx.y, by pairs where both sides are aligned for it.
-__global__ void __launch_bounds__(256) k_copy8(const __grid_constant__ Fields8 a, long long n)
+// Array blockIdx.y, 2 NCOPY NTC doubles of it to a block; by pairs where both sides
+// are aligned for it, loads first.  Blocks of one warp with 32 registers a thread:
+// the engines' step kernels fill the GPU for milliseconds and leave room for one
+// such block in each SM sub-partition (kb_step_split 80 registers x 6 warps of 512 x
+// 32, kb_step_plain 240 x 2, kb_step_1d half of them), so that a move starts beside
+// them.  With blocks of 256 threads it waited for the end of a step: 16 kB arrays
+// beside a batch with 2.4 ms steps 2.4 ms, in blocks of a warp 31 to the device and
+// 34 us back; alone no difference.
+constexpr int NTC = 32, NCOPY = 4;
+__global__ void __maxnreg__(32) k_copy8(const __grid_constant__ Fields8 a, long long n)
 {
     const double *s = a.src[blockIdx.y];
     double *d = a.dst[blockIdx.y];
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
     if ((((unsigned long long)s | (unsigned long long)d) & 15) == 0) {
-        for (long long i = t; i < n / 2; i += nt)
-            reinterpret_cast<double2 *>(d)[i] = reinterpret_cast<const double2 *>(s)[i];
-        if (t == 0 && (n & 1)) d[n - 1] = s[n - 1];
+        const double2 *s2 = reinterpret_cast<const double2 *>(s);
+        double2 *d2 = reinterpret_cast<double2 *>(d), v[NCOPY];
+        const long long i = (long long)blockIdx.x * NTC * NCOPY + threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < NCOPY; u++)
+            if (i + u * NTC < n / 2) v[u] = s2[i + u * NTC];
+#pragma unroll
+        for (int u = 0; u < NCOPY; u++)
+            if (i + u * NTC < n / 2) d2[i + u * NTC] = v[u];
+        if (i == 0 && (n & 1)) d[n - 1] = s[n - 1];
     } else {
-        for (long long i = t; i < n; i += nt) d[i] = s[i];
+        const long long i = (long long)blockIdx.x * NTC * NCOPY * 2 + threadIdx.x;
+        for (int u = 0; u < 2 * NCOPY; u++)
+            if (i + u * NTC < n) d[i + u * NTC] = s[i + u * NTC];
     }
 }
 
@@ -112,10 +126,10 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
     if (kernel) {
         if (m == 0) return MLAU_OK;
         for (int v = 0; v < m; v++) touch(to_host ? a.dst[v] : a.src[v], n, to_host);
-        const unsigned nb = (unsigned)std::min(152LL, (n / 2 + 255) / 256 + 1);
+        const unsigned nb = blocks_for(n, 2 * NCOPY * NTC);
         // the launch's own status: an error that an earlier call left behind is not this one's
         void *args[] = {&a, &n};
-        MLAU_CUDA(cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(256), args, 0, st));
+        MLAU_CUDA(cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(NTC), args, 0, st));
         if (to_host) MLAU_CUDA(cudaStreamSynchronize(st));
         return MLAU_OK;
     }
