@@ -212,7 +212,7 @@ static int download(mlau_sim *s, double *const *h, Move how)
     return s->sp ? split3d_check(s) : MLAU_OK;
 }
 
-int mlau_sim_download(mlau_sim *s, double *const *h) { return download(s, h, Move::Copies); }
+int mlau_sim_download(mlau_sim *s, double *const *h) { return download(s, h, Move::Kernel); }
 
 // A captured step graph holds the scheme parameters of its capture.
 static void drop_graph(mlau_sim *s)

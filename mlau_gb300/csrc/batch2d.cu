@@ -255,7 +255,7 @@ int move_fields(mlau_batch *b, const BInst &I, double *const *host, bool to_host
 {
     double *dev[8];
     for (int v = 0; v < 8; v++) dev[v] = b->a.s[v] ? b->a.s[v] + I.base : nullptr;
-    const int rc = copy_fields(dev, host, 8, (long long)I.nx * I.ny, to_host, Move::Copies, b->stream);
+    const int rc = copy_fields(dev, host, 8, (long long)I.nx * I.ny, to_host, Move::Kernel, b->stream);
     if (rc != MLAU_OK) return rc;
     MLAU_CUDA(cudaStreamSynchronize(b->stream));
     return MLAU_OK;

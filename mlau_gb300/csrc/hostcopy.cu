@@ -16,14 +16,14 @@
 // arrays of 0.7 / 2 MB 12 / 11 ms by copies, 22 / 28 by the kernel; 192 KB 15.8
 // and 15.7).
 //
-// Only the drivers' calls on host arrays ask for the kernel: they wait for their
-// result and need the SMs for the step in between.  The handles' and engines' own
-// uploads and downloads are copies, which need no SM: the kernel had them wait for
-// a step of whatever else ran on the GPU (16 kB to 0.7 MB beside a batch with 2.4 ms
-// steps: 38 to 140 us by copies, 2400 by the kernel), an upload for all that was
-// queued on its stream (51 kB arrays behind 39 ms of steps: 33 us by copies), and
-// a download into arrays not used before, as Sim.download makes them, for the
-// pages (2 MB each: 0.2 to 1.6 ms by copies, 3.3 to 5.5 by the kernel).
+// Who asks for the kernel: the 1D and 2D drivers' calls on host arrays, the engines'
+// uploads and downloads and the handles' downloads, all of which return when the
+// arrays have been moved.  Not the handles' uploads, which return while what is
+// queued before them runs (51 kB arrays behind 39 ms of steps: 33 us; the kernel
+// would have to be waited for), nor 3D drivers' calls and the MRX operators':
+// beside another engine's steps each launch may wait for one of them, and two more
+// cost ns_viscous_2d on 112 x 112 cells 13 ms against 6.6 by copies, a 24 x 20 x 16
+// step 44 against 20 (1D 4.9 against 9.7 by ten copies, a 2D step 25 and 27).
 #include "hostcopy.h"
 
 namespace mlau {

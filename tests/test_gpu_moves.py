@@ -32,11 +32,12 @@ def test_a_small_upload_does_not_wait_for_queued_steps(gpu_lib):
     assert t1 - t0 < 0.25 * (t2 - t0), (t1 - t0, t2 - t0)
 
 
-def test_moves_do_not_wait_for_another_engines_step(gpu_lib):
-    """Beside an engine whose step holds every SM for some 2 ms, another's
-    arrays move in the copy engines' time (0.1 ms)."""
+@pytest.mark.parametrize("precision", [0, 1])
+def test_moves_do_not_wait_for_another_engines_step(gpu_lib, precision):
+    """Beside an engine whose step holds every SM for some 2 ms (FP32-split) or
+    30 ms (FP64), another's arrays move in some 0.1 ms."""
     M = gpu_lib
-    heavy = M.Batch.open(8 * 520 * 520, 8)
+    heavy = M.Batch.open(8 * 520 * 520, 8, precision=precision)
     for k in range(8):
         st, m = ics.turbulence_2d(n=512, seed=k, vrms=0.3)
         heavy.add(st, m["dx"], m["dy"], m["gamma"], "mlau", 0.3, 1e9)
