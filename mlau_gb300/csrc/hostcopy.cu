@@ -7,14 +7,13 @@
 // host's page tables (Grace and Blackwell share them over NVLink-C2C) a kernel
 // reads and writes the arrays where they are.  Eight arrays there / back, copies
 // against the kernel: 2056 doubles each 23 / 66 against 11 / 10 us, 26624 79 / 74
-// against 18 / 19.  Arrays above 256 KB are copied, as are device or managed
-// arrays and where the GPU cannot reach host memory: the bytes count there, and
-// the kernel gains less or loses (pinned arrays to the host: 213 KB 30 against
-// 23 us, 0.7 MB 51 against 56, 2 MB 108 against 145; ordinary ones 3.8 MB 233
-// against 266), and where another engine's steps hold the SMs, which copies do
-// without, a driver's call waits for them (beside 2.4 ms steps, a 2D call with
-// arrays of 0.7 / 2 MB 12 / 11 ms by copies, 22 / 28 by the kernel; 192 KB 15.8
-// and 15.7).
+// against 18 / 19.  The line lies where the bytes count and the kernel loses: to the
+// device 4 MB (0.7 MB an array 73 against 129 us, 2 MB 98 against 174, 3.8 MB 168
+// against 252, pinned 164 against 197), to the host 256 KB (pinned arrays 213 KB 23
+// against 30 us, 0.7 MB 56 against 51, 2 MB 145 against 108; ordinary ones gain up
+// to 2 MB, but new ones, as Sim.download makes them, wait for their pages: 64^3 3.3
+// against 0.2 to 1 ms).  Larger arrays are copied, as are device or managed arrays
+// and where the GPU cannot reach host memory.
 //
 // Who asks for the kernel: the 1D and 2D drivers' calls on host arrays, the engines'
 // uploads and downloads and the handles' downloads, all of which return when the
@@ -34,14 +33,15 @@ struct Fields8 {
     double *dst[8];
 };
 
-constexpr long long kKernelBytes = 256 << 10;  // the largest array the kernel moves
+// the largest array the kernel moves to the device, to the host
+constexpr long long kKernelUp = 4 << 20, kKernelDown = 256 << 10;
 
 // Array blockIdx.y, 2 NCOPY NTC doubles of it to a block; by pairs where both sides
 // are aligned for it, loads first.  Blocks of one warp with 32 registers a thread:
 // the engines' step kernels fill the GPU for milliseconds and leave room for one
-// such block in each SM sub-partition (kb_step_split 80 registers x 6 warps of 512 x
-// 32, kb_step_plain 240 x 2, kb_step_1d half of them), so that a move starts beside
-// them.  With blocks of 256 threads it waited for the end of a step: 16 kB arrays
+// such block in each SM sub-partition (of its 512 registers a lane kb_step_split
+// takes 6 x 80, kb_step_plain 2 x 240, kb_step_1d 2 x 128), so that a move starts
+// beside them.  With blocks of 256 threads it waited for the end of a step: 16 kB arrays
 // beside a batch with 2.4 ms steps 2.4 ms, in blocks of a warp 31 to the device and
 // 34 us back; alone no difference.
 constexpr int NTC = 32, NCOPY = 4;
@@ -94,7 +94,7 @@ bool host_array(const void *p)
 // pageable memory: the GPU's first access to a bad page would be a fault that takes
 // the context with it.  Before a write the pages are also made present (the GPU
 // would wait for each; the bytes stay as they are).  4 KB is the smallest page;
-// the largest array here takes 65 accesses.
+// the largest array here takes 1024 accesses.
 void touch(const double *p, long long n, bool write)
 {
     volatile char *b = (volatile char *)p;
@@ -113,7 +113,8 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
 {
     Fields8 a{};
     int m = 0;
-    bool kernel = how == Move::Kernel && n > 0 && (long long)sizeof(double) * n <= kKernelBytes && nv <= 8 && reaches_host_memory();
+    bool kernel = how == Move::Kernel && n > 0 && nv <= 8 &&
+                  (long long)sizeof(double) * n <= (to_host ? kKernelDown : kKernelUp) && reaches_host_memory();
     for (int v = 0; v < nv && kernel; v++) {
         if (!dev[v] || !host[v]) continue;
         kernel = host_array(host[v]);

@@ -46,7 +46,7 @@ cudaError_t cudaLaunchKernel(const void *, dim3 grid, dim3, void **args, size_t,
 }
 }
 
-static double g_dev[8 << 16];
+static double g_dev[8 << 17];
 
 static int move(double *host, long long n, bool to_host)
 {
@@ -102,11 +102,11 @@ extern "C" int bad_array_check(int pages, long long n, int shift, int hole, int 
     return *launched ? 2 : 1;
 }
 
-// moves of n doubles there and back: 1 by the kernel, 2 by copies
-extern "C" int moved_by(long long n)
+// a move of n doubles: 1 by the kernel, 2 by a copy
+extern "C" int moved_by(long long n, int to_host)
 {
     setup();
-    static double host[8 << 16];
-    if (move(host, n, false) || move(host, n, true)) return 0;
-    return *launched == 2 && copies == 0 ? 1 : *launched == 0 && copies == 2 ? 2 : 0;
+    static double host[8 << 17];
+    if (move(host, n, to_host != 0)) return 0;
+    return *launched == 1 && copies == 0 ? 1 : *launched == 0 && copies == 1 ? 2 : 0;
 }

@@ -79,9 +79,9 @@ def _array(a, shift, pinned):
 
 @pytest.mark.parametrize("pinned", [False, True, "mixed"])
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("shape", [(4, 4), (13, 9), (120, 248), (121, 247), (292, 293), (712, 712)])
+@pytest.mark.parametrize("shape", [(4, 4), (13, 9), (120, 248), (121, 247), (292, 293), (504, 1016), (505, 1017)])
 def test_driver_calls_equal_the_handle(gpu_lib, shape, shift, pinned):
-    """Arrays up to the size at which the moves change (256 KB), above it, at 16 bytes
+    """Arrays up to the sizes at which the moves change (256 KB, 4 MB) and above, at 16 bytes
     and 8 beyond, ordinary and pinned: the same bits as upload, step, download."""
     M = gpu_lib
     st, m = ics.turbulence_2d(n=shape[1], ny=shape[0], seed=3, vrms=0.4)

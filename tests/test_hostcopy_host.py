@@ -42,7 +42,7 @@ def test_a_bad_array_fails_on_the_host(fake, back, to_host):
 
 
 def test_large_arrays_are_copied(fake):
-    """Above 256 KB the kernel is slower than copies beside another engine's
-    steps and for pinned downloads."""
-    for n, by in ((1, 1), (4096, 1), (32768, 1), (32769, 2), (90000, 2), (400000, 2)):
-        assert fake.moved_by(C.c_longlong(n)) == by, n
+    """To the device above 4 MB, to the host above 256 KB."""
+    for to_host, limit in ((0, 1 << 19), (1, 1 << 15)):
+        for n, by in ((1, 1), (4096, 1), (limit, 1), (limit + 1, 2), (1 << 20, 2)):
+            assert fake.moved_by(C.c_longlong(n), to_host) == by, (n, to_host)
