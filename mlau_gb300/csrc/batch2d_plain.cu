@@ -278,9 +278,13 @@ __device__ void pp_bc(const BArgs &A, int nt, const BTile *tl)
     });
 }
 
-// 240 registers a thread leave room for a warp of the copy kernel (hostcopy.cu) in
-// each SM sub-partition.
-__global__ void __maxnreg__(240) kb_step_plain(BArgs A)
+// At 216 registers a thread an SM sub-partition keeps 80 a lane free for a warp of
+// other streams' kernels - host array moves, the MRX operators, primitives, updates -
+// which otherwise wait for the end of a step (at the 250 the compiler takes by itself
+// ns_viscous_2d on 112 x 112 cells beside 36 ms steps takes 300 ms, at 240 150, here
+// 0.26).  No spills at any of these; 8 instances of 512^2, WCNS4 and mixed solvers, a
+// step 37.7 ms at 250 and here.
+__global__ void __maxnreg__(216) kb_step_plain(BArgs A)
 {
     const int nt = A.sync->ntiles;
     const BTile *tl = A.sync->tiles;

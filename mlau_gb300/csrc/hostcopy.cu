@@ -40,7 +40,7 @@ constexpr long long kKernelUp = 4 << 20, kKernelDown = 256 << 10;
 // are aligned for it, loads first.  Blocks of one warp with 32 registers a thread:
 // the engines' step kernels fill the GPU for milliseconds and leave room for one
 // such block in each SM sub-partition (of its 512 registers a lane kb_step_split
-// takes 6 x 80, kb_step_plain 2 x 240, kb_step_1d 2 x 128), so that a move starts
+// takes 6 x 80, kb_step_plain 2 x 216, kb_step_1d 2 x 128), so that a move starts
 // beside them.  With blocks of 256 threads it waited for the end of a step: 16 kB arrays
 // beside a batch with 2.4 ms steps 2.4 ms, in blocks of a warp 31 to the device and
 // 34 us back; alone no difference.
