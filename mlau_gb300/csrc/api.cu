@@ -595,10 +595,9 @@ int run_dropin(mlau_sim *c, double *const *h, double dt)
 {
     // FP32-split: the host link's copies overlap the step where the data allow
     if (c->sp && !c->walls3d) return split3d_step_host(c, dt, h);
-    const Move how = c->g.dim < 3 ? Move::Kernel : Move::Copies;
-    int rc = upload(c, (const double *const *)h, how);
+    int rc = upload(c, (const double *const *)h, Move::Kernel);
     if (rc == MLAU_OK) rc = mlau_sim_step(c, dt, 1);
-    if (rc == MLAU_OK) rc = download(c, h, how);
+    if (rc == MLAU_OK) rc = download(c, h, c->g.dim < 3 ? Move::Kernel : Move::Copies);
     else cudaStreamSynchronize(c->stream);  // the caller's arrays may still be read
     return rc;
 }
@@ -758,7 +757,7 @@ static int dropin_mrx(const char *who, double *const *h, const bool *back, doubl
     const int *tx = dnxs, *ty = dnys;
     mlau_sim *c = get_ctx(2, nx, ny, 1, xoff, yoff, 0, dx, dy, 1.0, gamma);
     int rc = c ? mlau_sim_set_bc_2d(c, tx, ty) : MLAU_ERR_NOMEM;
-    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, Move::Copies);
+    if (rc == MLAU_OK) rc = upload(c, (const double *const *)h, Move::Kernel);
     if (rc == MLAU_OK) {
         if (op == MRX_RESISTIVE) rc = diff2d_resistive(c, coef, dt);
         else if (op == MRX_VISCOUS) rc = diff2d_viscous(c, coef, dt);

@@ -15,14 +15,14 @@
 // against 0.2 to 1 ms).  Larger arrays are copied, as are device or managed arrays
 // and where the GPU cannot reach host memory.
 //
-// Who asks for the kernel: the 1D and 2D drivers' calls on host arrays, the engines'
-// uploads and downloads and the handles' downloads, all of which return when the
-// arrays have been moved.  Not the handles' uploads, which return while what is
-// queued before them runs (51 kB arrays behind 39 ms of steps: 33 us; the kernel
-// would have to be waited for), nor 3D drivers' calls and the MRX operators':
-// beside another engine's steps each launch may wait for one of them, and two more
-// cost ns_viscous_2d on 112 x 112 cells 13 ms against 6.6 by copies, a 24 x 20 x 16
-// step 44 against 20 (1D 4.9 against 9.7 by ten copies, a 2D step 25 and 27).
+// Who asks for the kernel: the drivers' calls on host arrays, the engines' uploads
+// and downloads and the handles' downloads, all of which return when the arrays have
+// been moved.  Not the handles' uploads, which return while what is queued before
+// them runs (51 kB arrays behind 39 ms of steps: 33 us; the kernel would have to be
+// waited for), nor the downloads of 3D drivers' calls and the MRX operators': beside
+// another engine's steps it queues behind their many launches and those behind the
+// steps (moves both ways by the kernel, a 24 x 20 x 16 step 44 ms beside 2.4 ms
+// steps, by copies back 19.3, by copies both ways 19.6; alone 545, 610, 680 us).
 #include "hostcopy.h"
 
 namespace mlau {
