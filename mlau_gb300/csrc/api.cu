@@ -327,7 +327,7 @@ static int step_once(mlau_sim *s, double dt)
 }
 
 // Long runs at one dt replay a captured graph of kGraphSteps steps: one
-// launch per kGraphSteps steps instead of 4-10 per stage, which is what bounds
+// launch per kGraphSteps steps instead of 1 (1D) to 12 per stage, which is what bounds
 // small problems.  The graph is rebuilt when dt changes; per-kernel timing
 // runs uncaptured.
 constexpr int kGraphSteps = 16;

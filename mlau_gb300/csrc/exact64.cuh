@@ -14,10 +14,10 @@
 // seed, one Newton step whose residual is formed exactly modulo 2^64, and a
 // correction from the next exact residual give the quotient to well below a
 // unit; the correctly rounded result follows unless that lies within the
-// correction's error of a midpoint between two doubles (about one operand in
-// 2^15), where the pipe's own operation decides.  Division instead makes two
-// quotient digits (32 and 29 bits) and settles the last unit by its exact
-// remainder.  Operands whose magnitude is outside 2^-255 .. 2^256, zeros,
+// correction's error of a midpoint between two doubles (about one reciprocal in
+// 2^15, one root in 2^13), where the pipe's own operation decides.  Division
+// instead makes two quotient digits (32 and 29 bits) and settles the last unit by
+// its exact remainder.  Operands whose magnitude is outside 2^-255 .. 2^256, zeros,
 // infinities and NaN also take the pipe's operation.  The seeds may be off by
 // 2 units in the last place (CUDA states at most 1 for rcp.approx, 2^-22.9 for
 // rsqrt.approx); tests/test_exact64.py tries them perturbed.

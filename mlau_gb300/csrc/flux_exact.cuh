@@ -7,8 +7,8 @@
 // it; the other products, the quotients and roots run as integer sequences
 // (exact64.cuh), comparisons look at the values' bits, products by powers of
 // two move exponents, and weights that are 0 or 1 become selections (which can
-// change the sign of a zero, no value).  A quotient or root whose rounding is
-// undecided (one in 2^15) is settled by the pipe on the spot: collected instead,
+// change the sign of a zero, no value).  A reciprocal or root whose rounding is
+// undecided (one in 2^15, 2^13) is settled by the pipe on the spot: collected instead,
 // one lane in a warp of some 600 evaluations sent the whole face through
 // riemann<double>, and every small launch waited for such a warp (200 x 120
 // cells, fluxes of a step 139 -> 83 us; 128^3 8.9 -> 7.7 ms).  `bad` collects

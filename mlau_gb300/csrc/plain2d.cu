@@ -233,7 +233,7 @@ k_flux2_ed(PlainFields f, const __grid_constant__ Sweeps2 S, Dims d, double gamm
 // less than what the GPU holds at a time, so that it spreads evenly (200 x 120
 // cells, a step of LHLLD + MUSCL: 268 us with blocks of 32, 273 of 64, 289 of 128
 // and 256; 300 x 300: no difference beyond 2 %).
-constexpr long long kSmall2 = 97280;  // threads: 5 reconstruction blocks of 128 on each SM
+constexpr long long kSmall2 = 97280;  // threads: 5 reconstruction blocks of 128 on each of 152 SMs
 
 template <int NR> void launch_rec2(Sim *s, const Sweeps2 &S, const Dims &d)
 {

@@ -843,6 +843,8 @@ ks_update(PlainFields f, SplitPtrs g, Dims d, int odr_rt, RkFF rk, RkF64 rd, flo
 #pragma unroll
     for (int v = 0; v < 5; v++) {
         float div;
+        // the energy's products join in another order than the others' for no reason but
+        // that the compiler once chose so: the bits stay
         if constexpr (ODR == 4)
             div = __fmaf_rn(dtdz, fdiff4(fz[v]),
                             v < 4 ? __fmaf_rn(dtdx, fdiff4(fx[v]), __fmul_rn(dtdy, fdiff4(fy[v])))
