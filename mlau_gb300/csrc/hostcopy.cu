@@ -124,22 +124,31 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
         a.src[m] = to_host ? dev[v] : host[v];
         a.dst[m++] = to_host ? host[v] : dev[v];
     }
+    cudaError_t e = cudaSuccess;
     if (kernel) {
         if (m == 0) return MLAU_OK;
         for (int v = 0; v < m; v++) touch(to_host ? a.dst[v] : a.src[v], n, to_host);
         const unsigned nb = blocks_for(n, 2 * NCOPY * NTC);
         // the launch's own status: an error that an earlier call left behind is not this one's
         void *args[] = {&a, &n};
-        MLAU_CUDA(cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(NTC), args, 0, st));
-        if (to_host) MLAU_CUDA(cudaStreamSynchronize(st));
-        return MLAU_OK;
+        e = cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(NTC), args, 0, st);
+    } else {
+        for (int v = 0; v < nv && e == cudaSuccess; v++) {
+            if (!dev[v] || !host[v]) continue;
+            e = to_host ? cudaMemcpyAsync(host[v], dev[v], sizeof(double) * n, cudaMemcpyDeviceToHost, st)
+                        : cudaMemcpyAsync(dev[v], host[v], sizeof(double) * n, cudaMemcpyHostToDevice, st);
+        }
     }
-    for (int v = 0; v < nv; v++) {
-        if (!dev[v] || !host[v]) continue;
-        MLAU_CUDA(to_host ? cudaMemcpyAsync(host[v], dev[v], sizeof(double) * n, cudaMemcpyDeviceToHost, st)
-                          : cudaMemcpyAsync(dev[v], host[v], sizeof(double) * n, cudaMemcpyHostToDevice, st));
+    // waited for on failure too: what is queued may read the caller's arrays (an
+    // upload by the kernel) or write them
+    if (to_host) {
+        const cudaError_t w = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = w;
     }
-    if (to_host) MLAU_CUDA(cudaStreamSynchronize(st));
+    if (e != cudaSuccess) {
+        set_error("host arrays %s the device: %s", to_host ? "from" : "to", cudaGetErrorString(e));
+        return MLAU_ERR_CUDA;
+    }
     return MLAU_OK;
 }
 

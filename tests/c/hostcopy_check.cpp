@@ -12,7 +12,8 @@
 #include "hostcopy.cu"
 
 static int *launched;  // shared with the children
-static int copies;
+static int copies, syncs;
+static cudaError_t copy_fails = cudaSuccess;
 static cudaError_t pending = cudaSuccess;
 
 namespace mlau {
@@ -29,10 +30,11 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *)
 }
 cudaError_t cudaGetLastError() { const cudaError_t e = pending; pending = cudaSuccess; return e; }
 const char *cudaGetErrorString(cudaError_t) { return ""; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { syncs++; return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t)
 {
     copies++;
+    if (copy_fails != cudaSuccess) return copy_fails;
     memcpy(d, s, n);
     return cudaSuccess;
 }
@@ -61,7 +63,7 @@ static void setup()
     if (!launched)
         launched = (int *)mmap(nullptr, 4096, PROT_READ | PROT_WRITE, MAP_SHARED | MAP_ANONYMOUS, -1, 0);
     *launched = 0;
-    copies = 0;
+    copies = syncs = 0;
 }
 
 // 0: moved by the kernel although an error of another call was pending
@@ -109,4 +111,15 @@ extern "C" int moved_by(long long n, int to_host)
     static double host[8 << 17];
     if (move(host, n, to_host != 0)) return 0;
     return *launched == 1 && copies == 0 ? 1 : *launched == 0 && copies == 1 ? 2 : 0;
+}
+
+// A download whose copy is refused: an error, after the stream has been waited for.
+extern "C" int failed_download_check()
+{
+    setup();
+    static double host[40000];
+    copy_fails = cudaErrorInvalidValue;
+    const int rc = move(host, 40000, true);
+    copy_fails = cudaSuccess;
+    return rc == 0 || copies != 1 || syncs != 1;
 }

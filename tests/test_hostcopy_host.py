@@ -46,3 +46,8 @@ def test_large_arrays_are_copied(fake):
     for to_host, limit in ((0, 1 << 19), (1, 1 << 15)):
         for n, by in ((1, 1), (4096, 1), (limit, 1), (limit + 1, 2), (1 << 20, 2)):
             assert fake.moved_by(C.c_longlong(n), to_host) == by, (n, to_host)
+
+
+def test_a_failed_download_waits_for_the_stream(fake):
+    """The upload of the same call may still read the caller's arrays."""
+    assert fake.failed_download_check() == 0
