@@ -125,14 +125,13 @@ int copy_fields(double *const *dev, double *const *host, int nv, long long n, bo
         a.dst[m++] = to_host ? host[v] : dev[v];
     }
     cudaError_t e = cudaSuccess;
-    if (kernel) {
-        if (m == 0) return MLAU_OK;
+    if (kernel && m > 0) {
         for (int v = 0; v < m; v++) touch(to_host ? a.dst[v] : a.src[v], n, to_host);
         const unsigned nb = blocks_for(n, 2 * NCOPY * NTC);
         // the launch's own status: an error that an earlier call left behind is not this one's
         void *args[] = {&a, &n};
         e = cudaLaunchKernel((const void *)k_copy8, dim3(nb, m), dim3(NTC), args, 0, st);
-    } else {
+    } else if (!kernel) {
         for (int v = 0; v < nv && e == cudaSuccess; v++) {
             if (!dev[v] || !host[v]) continue;
             e = to_host ? cudaMemcpyAsync(host[v], dev[v], sizeof(double) * n, cudaMemcpyDeviceToHost, st)

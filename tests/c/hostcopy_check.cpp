@@ -123,3 +123,12 @@ extern "C" int failed_download_check()
     copy_fails = cudaSuccess;
     return rc == 0 || copies != 1 || syncs != 1;
 }
+
+// A download of no arrays still waits for the stream.
+extern "C" int empty_download_check()
+{
+    setup();
+    double *dev[8] = {}, *h[8] = {};
+    const int rc = mlau::copy_fields(dev, h, 8, 100, true, mlau::Move::Kernel, nullptr);
+    return rc != 0 || *launched || copies || syncs != 1;
+}

@@ -51,3 +51,7 @@ def test_large_arrays_are_copied(fake):
 def test_a_failed_download_waits_for_the_stream(fake):
     """The upload of the same call may still read the caller's arrays."""
     assert fake.failed_download_check() == 0
+
+
+def test_a_download_of_nothing_waits_for_the_stream(fake):
+    assert fake.empty_download_check() == 0
